@@ -28,18 +28,17 @@ __global__ void k_intersect(DevScene sc, const float* __restrict__ rays, long lo
     if (brute == 0) {
       h = trace_closest(sc, o, d, tmin, tmax);
     } else if (brute == 2) {
-      // the resumable traversal of the wavefront closest-hit kernel (trace_step)
-      struct Stk {
-        int a[kStack];
-        __device__ void push(int i, int v) { a[i] = v; }
-        __device__ int pop(int i) const { return a[i]; }
-      } stk;
-      TraceState s;
-      trace_begin(s, o, d, tmin, tmax, -INFINITY, sc.root);
-      if (sc.ntri > 0)
-        while (!trace_step(sc, s, stk)) {
-        }
-      h = s.h;
+      // the traversal as the wavefront closest-hit kernel drives it, one ray per thread
+      LocalMem mem;
+      Trav s;
+      mem.rp = ray_pre(o, d);
+      mem.bary(0.f, 0.f);
+      trav_begin(s, o, d, tmax, -INFINITY, sc.ntri > 0 ? sc.root : kNoNode);
+      while (s.node != kNoNode) {
+        if (s.node < 0) trav_leaf(sc.leaf, s, tmin, mem);
+        else trav_node(sc.nodes, s, tmin, mem, sc.err);
+      }
+      h.tri = s.tri; h.b1 = mem.b1; h.b2 = mem.b2; h.t = s.t;
     } else {
       h.tri = -1; h.t = tmax; h.b1 = h.b2 = 0.f;
       const RayPre rp = ray_pre(o, d);

@@ -249,109 +249,146 @@ __global__ void __launch_bounds__(256) k_shade(WF w, const DevScene* __restrict_
 
 // ------------------------------------------------------------------ trace kernel
 // Closest hit of every queued ray of a depth (light-sample rays r < nL stop at the first
-// hit short of the light). Persistent warps with dynamic ray fetch: a lane whose ray
-// has finished takes the next unclaimed ray of the queue after every 8 traversal steps,
-// so a warp keeps its lanes busy instead of waiting for its longest ray (the rays of a
-// warp differ in traversal length by an order of magnitude). The fetch counter is
-// w.cnt[2D+2], reset by k_shade.
-constexpr int kTraceSteps = 8;
+// hit short of the light). Persistent warps with dynamic ray fetch: the lanes whose rays
+// have finished take the next unclaimed rays of the queue together once there are kRefill
+// of them, so a warp keeps its lanes busy instead of waiting for its longest ray (the rays
+// of a warp differ in traversal length by an order of magnitude) and the ray set-up runs on
+// at least half a warp. The fetch counter is w.cnt[2D+2], reset by k_shade.
+//
+// Bound by instruction issue and divergence, not by memory: on 512^2 x 8 spp rays of the
+// icosphere scene the SMs issue 64 % of the cycles with 14 of 32 lanes active (11 before lanes
+// waited for one another at leaves, trav_step), L1 33 % and L2 6 % of their peaks. Traversal
+// of the 512^2 x 32 spp icosphere step: 14.0 ms before, 12.2 ms now (2^20-path tiles).
+constexpr int kRefill = 16;
 // Lights of at most this many triangles in all let k_trace answer MIS BSDF-sample rays
 // with a light test and a bounded occlusion query.
 constexpr int kMisLightTris = 16;
-__global__ void __launch_bounds__(128) k_trace(WF w, const DevScene* __restrict__ scenes,
-                                                   const DevView* __restrict__ views, int d,
-                                                   unsigned long long* __restrict__ ray_count) {
-  const int nk = w.cnt[2 * d + 1];
+// Per-lane memory of k_trace: the first kShort stack entries, the ray as the triangle test
+// takes it and the hit's barycentrics live in shared memory (one column per lane, so a
+// warp's accesses hit 32 banks), which keeps them out of the registers of the node visits;
+// deeper stack entries are in local memory.
+constexpr int kShort = 16;
+// Resident blocks asked for: 64 registers, no spills. 6 and 7 blocks take 1-3 % longer, 9 and
+// more spill (+16 % and up).
+constexpr int kTraceBlocks = 8;
+struct TraceShared {
+  int stack[kShort][128];
+  float ray[8][128];  // origin, shear constants, barycentrics
+};
+struct TraceMem {
+  TraceShared* sh;
+  int lane;
+  int axes;  // kx | ky << 2 | kz << 4
+  int deep[kStack - kShort];
+  PSDR_D void set_ray(const RayPre& r) {
+    sh->ray[0][lane] = r.o.x; sh->ray[1][lane] = r.o.y; sh->ray[2][lane] = r.o.z;
+    sh->ray[3][lane] = r.Sx; sh->ray[4][lane] = r.Sy; sh->ray[5][lane] = r.Sz;
+    axes = r.kx | r.ky << 2 | r.kz << 4;
+    bary(0.f, 0.f);
+  }
+  PSDR_D RayPre ray() const {
+    RayPre r;
+    r.o = f3(sh->ray[0][lane], sh->ray[1][lane], sh->ray[2][lane]);
+    r.Sx = sh->ray[3][lane]; r.Sy = sh->ray[4][lane]; r.Sz = sh->ray[5][lane];
+    r.kx = axes & 3; r.ky = (axes >> 2) & 3; r.kz = axes >> 4;
+    return r;
+  }
+  PSDR_D void bary(float u, float v) { sh->ray[6][lane] = u; sh->ray[7][lane] = v; }
+  PSDR_D float b1() const { return sh->ray[6][lane]; }
+  PSDR_D float b2() const { return sh->ray[7][lane]; }
+  PSDR_D void put(int i, int v) { if (i < kShort) sh->stack[i][lane] = v; else deep[i - kShort] = v; }
+  PSDR_D void push3(int sp, int n, int c1, int c2, int c3) {
+    if (sp + 3 <= kShort) {
+      // a slot above the new top may be overwritten: three stores, no branch
+      sh->stack[sp + 2][lane] = c1;
+      sh->stack[sp + (n > 2 ? 1 : 0)][lane] = n > 2 ? c2 : (n > 1 ? c2 : c1);
+      sh->stack[sp + (n > 2 ? 0 : 1)][lane] = n > 2 ? c3 : c1;
+    } else {
+      if (n > 2) put(sp, c3);
+      if (n > 1) put(sp + n - 2, c2);
+      if (n > 0) put(sp + n - 1, c1);
+    }
+  }
+  PSDR_D int pop(int i) const { return i < kShort ? sh->stack[i][lane] : deep[i - kShort]; }
+};
+__global__ void __launch_bounds__(128, kTraceBlocks) k_trace(WF w, const DevScene* __restrict__ scenes,
+                                                             const DevView* __restrict__ views, int d,
+                                                             unsigned long long* __restrict__ ray_count) {
+  const unsigned nk = (unsigned)w.cnt[2 * d + 1];
   const int Rd = (d == w.D - 1) ? w.R - 1 : w.R;
-  const long long total = (long long)nk * Rd;
+  const unsigned total = nk * (unsigned)Rd;
   if (ray_count && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(ray_count, (unsigned long long)total);
-  int* fetch = w.cnt + 2 * w.D + 2;
-  // traversal stack: the first kShort entries of each lane in shared memory (one column per
-  // lane, so a warp's pushes and pops hit 32 banks), the deeper ones in local memory
-  constexpr int kShort = 16;
-  __shared__ int sst[kShort][128];
-  struct Stk {
-    int (*sh)[128];
-    int lane;
-    int deep[kStack - kShort];
-    __device__ __forceinline__ void push(int i, int v) { if (i < kShort) sh[i][lane] = v; else deep[i - kShort] = v; }
-    __device__ __forceinline__ int pop(int i) const { return i < kShort ? sh[i][lane] : deep[i - kShort]; }
-  } stack;
-  stack.sh = sst;
-  stack.lane = threadIdx.x;
-  TraceState s;
-  const DevScene* sc = nullptr;
+  unsigned* fetch = reinterpret_cast<unsigned*>(w.cnt + 2 * w.D + 2);
+  __shared__ TraceShared sh;
+  TraceMem mem;
+  mem.sh = &sh;
+  mem.lane = threadIdx.x;
+  Trav s;
+  s.node = kNoNode;
+  const DevScene* sc = scenes;
   size_t slot = 0;
-  bool live = false, done = false;
+  bool open = false;  // the lane's ray has been traversed and its hit is not written yet
+  unsigned next = 0;  // last index this warp claimed: beyond `total` the queue is empty
+  const float4* nodes = nullptr;
+  const float4* leaf = nullptr;
   while (true) {
-    const unsigned want = __ballot_sync(0xffffffffu, !live && !done);
-    if (want) {
-      const int lane = threadIdx.x & 31, leader = __ffs(want) - 1;
-      int base = 0;
-      if (lane == leader) base = atomicAdd(fetch, __popc(want));
+    if (open && s.node == kNoNode) {
+      w.hit[slot] = make_float4(__int_as_float(s.tri), mem.b1(), mem.b2(), s.t);
+      open = false;
+    }
+    const unsigned idle = __ballot_sync(0xffffffffu, !open);
+    if (next < total && (__popc(idle) >= kRefill)) {
+      const int lane = threadIdx.x & 31, leader = __ffs(idle) - 1;
+      unsigned base = 0;
+      if (lane == leader) base = atomicAdd(fetch, (unsigned)__popc(idle));
       base = __shfl_sync(0xffffffffu, base, leader);
-      if (!live && !done) {
-        const long long idx = (long long)base + __popc(want & lanemask_lt());
-        if (idx < total) {
-          const int r = (int)(idx / nk);
-          const int k = (int)(idx - (long long)r * nk);
-          slot = (size_t)r * w.cap + k;
-          sc = &scenes[views[w.view[w.qs[k]]].scene];
-          const float4 o = w.ro[slot], dd = w.rd[slot];
-          const float t_occ = r < w.nL ? (o.w - 4e-3f) / 1.0001f - 4e-3f : -INFINITY;
-          trace_begin(s, xyz(o), xyz(dd), kTmin, o.w, t_occ, sc->root);
-          live = sc->ntri > 0;
-          if (live && r >= w.nL && r < w.nL + w.nB && sc->nlight > 0) {
-            // MIS BSDF-sample ray: only a light hit contributes (the shade, accumulate and
-            // adjoint kernels skip any other hit). The closest light triangle along the ray
-            // (the traversal's test and tie rule) bounds an occlusion query: a nearer hit is
-            // reported as a miss, and with no light along the ray nothing is traversed.
-            int nlt = 0;
-            for (int l = 0; l < sc->nlight; ++l) nlt += sc->lights[l].ntri;
-            if (nlt <= kMisLightTris) {
-              float tl = o.w;
-              int best = -1;
-              for (int l = 0; l < sc->nlight; ++l) {
-                const DevLight& Lt = sc->lights[l];
-                for (int t = Lt.tri0; t < Lt.tri0 + Lt.ntri; ++t) {
-                  const float4* q = sc->tri + 6 * (size_t)t;
-                  float tt, b1, b2;
-                  if (tri_test(s.rp, xyz(__ldg(q)), xyz(__ldg(q + 1)), xyz(__ldg(q + 2)), kTmin, tl, tt, b1, b2) &&
-                      (tt < tl || best < 0 || t < best)) {
-                    tl = tt;
-                    best = t;
-                  }
+      next = base + __popc(idle);
+      const unsigned idx = base + __popc(idle & lanemask_lt());
+      if (!open && idx < total) {
+        const unsigned r = idx / nk;
+        const unsigned k = idx - r * nk;
+        slot = (size_t)r * w.cap + k;
+        sc = scenes + (w.one_scene >= 0 ? w.one_scene : views[w.view[w.qs[k]]].scene);
+        const float4 o = w.ro[slot], dd = w.rd[slot];
+        const float t_occ = (int)r < w.nL ? (o.w - 4e-3f) / 1.0001f - 4e-3f : -INFINITY;
+        const RayPre rp = ray_pre(xyz(o), xyz(dd));
+        mem.set_ray(rp);
+        trav_begin(s, xyz(o), xyz(dd), o.w, t_occ, sc->ntri > 0 ? sc->root : kNoNode);
+        nodes = sc->nodes;
+        leaf = sc->leaf;
+        open = true;
+        if ((int)r >= w.nL && (int)r < w.nL + w.nB && sc->nlight > 0) {
+          // MIS BSDF-sample ray: only a light hit contributes (the shade, accumulate and
+          // adjoint kernels skip any other hit). The closest light triangle along the ray
+          // (the traversal's test and tie rule) bounds an occlusion query: a nearer hit is
+          // reported as a miss, and with no light along the ray nothing is traversed.
+          int nlt = 0;
+          for (int l = 0; l < sc->nlight; ++l) nlt += sc->lights[l].ntri;
+          if (nlt <= kMisLightTris) {
+            float tl = o.w;
+            int best = -1;
+            for (int l = 0; l < sc->nlight; ++l) {
+              const DevLight& Lt = sc->lights[l];
+              for (int t = Lt.tri0; t < Lt.tri0 + Lt.ntri; ++t) {
+                const float4* q = sc->tri + 6 * (size_t)t;
+                float tt, b1, b2;
+                if (tri_test(rp, xyz(__ldg(q)), xyz(__ldg(q + 1)), xyz(__ldg(q + 2)), kTmin, tl, tt, b1, b2) &&
+                    (tt < tl || best < 0 || t < best)) {
+                  tl = tt;
+                  best = t;
                 }
               }
-              if (best < 0) {
-                live = false;
-                w.hit[slot] = make_float4(__int_as_float(-1), 0.f, 0.f, o.w);
-              } else {
-                s.h.t = tl;
-                s.t_occ = tl;
-              }
             }
+            s.t = tl;
+            s.t_occ = tl;
+            if (best < 0) s.node = kNoNode;
           }
-          if (!live && sc->ntri <= 0) w.hit[slot] = make_float4(__int_as_float(-1), 0.f, 0.f, o.w);
-        } else {
-          done = true;
         }
       }
-    }
-    if (!__any_sync(0xffffffffu, live)) {
-      if (__all_sync(0xffffffffu, done)) break;
       continue;
     }
-    if (live) {
-#pragma unroll 1
-      for (int it = 0; it < kTraceSteps; ++it) {
-        if (trace_step(*sc, s, stack)) {
-          w.hit[slot] = make_float4(__int_as_float(s.h.tri), s.h.b1, s.h.b2, s.h.t);
-          live = false;
-          break;
-        }
-      }
-    }
+    if (idle == 0xffffffffu) break;
+    trav_step(0xffffffffu, nodes, leaf, s, kTmin, mem, sc->err);
   }
 }
 
@@ -2061,7 +2098,7 @@ __global__ void __launch_bounds__(128) k_crease_pairs(const DevScene* __restrict
     int node = sc.root;
     while (true) {
       if (node >= 0) {
-        const float4* nd = sc.nodes + 7 * (size_t)node;
+        const float4* nd = sc.nodes + kNodeF4 * (size_t)node;
         const float4 lx = __ldg(nd), hx = __ldg(nd + 1), ly = __ldg(nd + 2), hy = __ldg(nd + 3);
         const float4 lz = __ldg(nd + 4), hz = __ldg(nd + 5);
         const int4 e = __ldg(reinterpret_cast<const int4*>(nd + 6));
@@ -2070,7 +2107,7 @@ __global__ void __launch_bounds__(128) k_crease_pairs(const DevScene* __restrict
         const float clz[4] = {lz.x, lz.y, lz.z, lz.w}, chz[4] = {hz.x, hz.y, hz.z, hz.w};
         const int ch[4] = {e.x, e.y, e.z, e.w};
         for (int c = 0; c < 4; ++c) {
-          if (ch[c] == 0x7fffffff) continue;
+          if (ch[c] == kNoNode) continue;
           if (clx[c] > hi.x || chx[c] < lo.x || cly[c] > hi.y || chy[c] < lo.y || clz[c] > hi.z || chz[c] < lo.z)
             continue;
           if (sp < 64) stack[sp++] = ch[c];
@@ -3290,6 +3327,13 @@ void Profiler::replayed(std::vector<EvPair>* graph_ev, long long n_trace) {
 #define PSDR_LAUNCHED(n) (profiler().launches += (n))
 void count_launches(int n) { profiler().launches += n; }
 
+// The scene of every view of a job, or -1 when its views have several.
+static int job_scene(const std::vector<DevView>& views) {
+  for (const DevView& v : views)
+    if (v.scene != views[0].scene) return -1;
+  return views.empty() ? -1 : views[0].scene;
+}
+
 static int any_ortho(const std::vector<DevView>& views) {
   for (const DevView& v : views)
     if (v.ortho) return 1;
@@ -3438,6 +3482,7 @@ void set_wf(WF& w, const psdr_config& cfg, int nviews, int nB_override, int ligh
   w.R = w.nL + w.nB + 1;
   w.light_vis = light_vis;
   w.nviews = nviews;
+  w.one_scene = -1;
   // seed s offsets every sample stream by s * 2654435761 (mod 2^32, the width of the
   // stream index): jobs of different seeds draw from disjoint stream ranges
   w.seed = cfg.seed * 2654435761ull;
@@ -3453,6 +3498,7 @@ void forward_tile(const DevScene* scenes_dev, const std::vector<DevView>& views,
   set_wf(w, cfg, (int)views.size(), -1, cfg.enable_light_visable);
   w.bsdf = ws->bsdf;
   w.ortho = any_ortho(views);
+  w.one_scene = job_scene(views);
   if (keep) {
     w.rec = keep->rec + (size_t)t.begin * w.rec_stride;
     w.view = keep->view + t.begin;
@@ -3755,6 +3801,7 @@ void backward_unit(const DevScene* scenes_dev, const std::vector<DevView>& views
     set_wf(w, cfg, (int)views.size(), -1, cfg.enable_light_visable);
     w.bsdf = ws->bsdf;
     w.ortho = any_ortho(views);
+    w.one_scene = job_scene(views);
     const Tile& t = u.tile;
     if (keep) {
       w.rec = keep->rec + (size_t)t.begin * w.rec_stride;
@@ -3786,12 +3833,14 @@ void backward_unit(const DevScene* scenes_dev, const std::vector<DevView>& views
   set_wf(w, cfg, (int)views.size(), 1, 0);
   w.bsdf = ws->bsdf;
   w.ortho = any_ortho(views);
+  w.one_scene = job_scene(views);
   // paths of the unbiased boundary samples carry the interior estimator's radiance
   WF wi = ws->wf;
   wi.cap = ws->cap;
   set_wf(wi, cfg, (int)views.size(), -1, cfg.enable_light_visable);
   wi.bsdf = ws->bsdf;
   wi.ortho = any_ortho(views);
+  wi.one_scene = w.one_scene;
   EdgeBuf eb{ws->eb_a.as<float4>(), ws->eb_n.as<float4>(), ws->eb_hb.as<float4>(), ws->eb_La.as<float4>(), nullptr};
   const int v = u.view;
   const DevView& V = views[v];
@@ -4089,6 +4138,7 @@ extern "C" PSDR_API psdr_status psdr_render_fwd_noalloc(psdr_scene* scene, const
     set_wf(w, *cfg, 1, -1, cfg->enable_light_visable);
     w.bsdf = scene->has_bsdf || scene->env_light >= 0 ? 1 : 0;
     w.ortho = cam->type == PSDR_CAM_ORTHOGRAPHIC ? 1 : 0;
+    w.one_scene = 0;
     // the view record goes into the scratch too (the previous call's view is overwritten)
     DevView V;
     make_view(*cam, cfg->spp_interior, V);

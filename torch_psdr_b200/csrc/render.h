@@ -50,6 +50,7 @@ struct WF {
   int rec_stride;
   int bsdf;      // host side: launch the extended kernel instances (DiffuseBsdfMaterial, environment light)
   int ortho;     // host side: an orthographic view is in the job (camera kernel instance)
+  int one_scene; // the scene of every view of the job, or -1 when the views have several
   int trace_bps; // host side: blocks of 128 rays per SM of the closest-hit kernel (queue depth)
 };
 

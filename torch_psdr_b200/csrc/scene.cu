@@ -471,7 +471,7 @@ __global__ void k_layout4(int n, int leaf_size, const int* __restrict__ slots4, 
   for (int k = 0; k < 4; ++k) {
     if (k >= ns) {
       for (int q = 0; q < 3; ++q) { lo[q][k] = INFINITY; hi[q][k] = -INFINITY; }
-      enc[k] = 0x7fffffff;
+      enc[k] = kNoNode;
       continue;
     }
     const int c = slot[k];
@@ -482,7 +482,7 @@ __global__ void k_layout4(int n, int leaf_size, const int* __restrict__ slots4, 
     }
     enc[k] = is_leaf(c) ? leaf_code(c) : idx4[c];
   }
-  float4* o = nodes4 + 7 * (size_t)idx4[i];
+  float4* o = nodes4 + kNodeF4 * (size_t)idx4[i];
   o[0] = make_float4(lo[0][0], lo[0][1], lo[0][2], lo[0][3]);
   o[1] = make_float4(hi[0][0], hi[0][1], hi[0][2], hi[0][3]);
   o[2] = make_float4(lo[1][0], lo[1][1], lo[1][2], lo[1][3]);
@@ -672,7 +672,7 @@ void psdr_scene_alloc(psdr_scene* s) {
   s->edge_f.alloc(sizeof(int2) * nh, st);
   s->edge_pmf.alloc(sizeof(float) * nh, st);
   s->edge_cmf.alloc(sizeof(float) * nh, st);
-  s->nodes.alloc(sizeof(float4) * 7 * n, st);
+  s->nodes.alloc(sizeof(float4) * kNodeF4 * n, st);
   s->leaf.alloc(sizeof(float4) * 3 * n, st);
   s->err.alloc(sizeof(int), st);
   s->keys.alloc(sizeof(uint64_t) * nh, st);
