@@ -340,13 +340,13 @@ def run_b200(args):
     integ = dr.PathIntegrator(estimator=args.estimator, batch_lanes=args.batch_lanes,
                               batch_records=args.batch_records, tile_paths=args.tile_paths, **CFG)
 
-    leaf = {"size": 1}
+    leaf = {"size": 2}  # the library's default
 
     def build_scene(verts, texture):
         sc = dr.Scene([cam], [dr.Mesh(verts, uvs, faces, uvi, dr.DiffuseMaterial(texture)),
                               dr.Mesh(gV, None, gF, None, dr.DiffuseMaterial(gT))],
                       [dr.AreaLight(lV, lF, lE)])
-        if leaf["size"] != 1:
+        if leaf["size"] != 2:
             L.check(lib.psdr_scene_set_leaf_size(sc.handle, leaf["size"],
                                                  ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)), "leaf")
         return sc
