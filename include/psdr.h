@@ -104,7 +104,8 @@ typedef struct {
 } psdr_camera_desc;
 
 /* PathIntegrator::Config (path_integrator.h:8-21; torch_psdr.py:478-536) plus the
- * B200 extensions: estimator, tile_paths (wavefront tile, 0 = 2^20 paths; see
+ * B200 extensions: estimator, tile_paths (wavefront tile, 0 = 2^20 to 2^22 paths by job and
+ * free memory; see
  * psdr_autotune), leaf_size
  * (BVH leaf collapse, 0 = default), terms, spp_pixel_boundary and seed (0 = the
  * reference's sample streams; seed s offsets every stream index by s * 2654435761

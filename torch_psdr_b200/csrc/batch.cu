@@ -169,7 +169,7 @@ PSDR_API psdr_status psdr_batch_create(psdr_scene* const* scenes, int32_t n_scen
     }
     assign_offsets(b->views);
     set_scene_ntri(b->views, scenes);
-    b->cap = choose_cap(*cfg, b->views, true);
+    b->cap = choose_cap(*cfg, b->views, true, cfg->batch_lanes > 0 ? cfg->batch_lanes : 4, nullptr);
     const int Rmax = cfg->mis_light_samples + std::max(cfg->mis_bsdf_samples, 1) + 1;
     if (b->backward && cfg->batch_records >= 0) {
       long long paths = 0;

@@ -3406,12 +3406,61 @@ static void run_tile(WF& w, const DevScene* scenes, const DevView* views, const 
   depth_loop(w, scenes, views, mode, st);
 }
 
-int choose_cap(const psdr_config& cfg, const std::vector<DevView>& views, bool backward) {
+// Device bytes of a workspace per path of tile capacity (psdr_workspace::ensure).
+static size_t path_bytes(const psdr_config& cfg, bool records) {
+  const size_t R = (size_t)cfg.mis_light_samples + std::max(cfg.mis_bsdf_samples, 1) + 1, D = cfg.max_bounce;
+  return 2 * 8 + 2 * 4 + 4 * 16 + 3 * 4 + 4 * 16 * R + 4 * 16 + 2 * 4 + 20 +
+         (records ? 16 * (1 + D * R + 2 * D) : 0);
+}
+
+// Paths of a wavefront tile when the caller leaves it to the library: 2^22, halved until the
+// workspace is at most kTileBytes and an eighth of the free device memory (down to 2^20, the
+// smallest). Every launch over a tile ends with its warps draining their last rays (50 to
+// 120 node visits for the longest against 14 on average), about 60 us in which the lanes
+// empty out; larger tiles pay for it less often. 1.31 M triangles, 1024^2 x 16 spp, depth 5:
+// traversal 18.2 ms with 2^20-path tiles, 14.7 with 2^21, 13.0 with 2^22.
+// A workspace that already holds such a tile keeps it without asking for the free memory.
+constexpr long long kTileMax = 1 << 22, kTileMin = 1 << 20;
+constexpr size_t kTileBytes = size_t(4) << 30;
+static long long auto_tile(const psdr_config& cfg, long long need, bool records, const psdr_workspace* ws) {
+  if (need <= kTileMin) return kTileMin;
+  const size_t pb = path_bytes(cfg, records);
+  long long t = kTileMax;
+  while (t > kTileMin && (size_t)t * pb > kTileBytes) t >>= 1;
+  if (t == kTileMin || (ws && ws->cap >= std::min(t, need) && (!records || ws->rec.p))) return t;
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+    cudaGetLastError();
+    return kTileMin;
+  }
+  while (t > kTileMin && (size_t)t * pb > free_b / 8) t >>= 1;
+  return t;
+}
+
+// lanes: concurrent tiles of a batch; its automatic tile is small enough for each lane to
+// get one (but no smaller than 2^20).
+int choose_cap(const psdr_config& cfg, const std::vector<DevView>& views, bool backward, int lanes,
+               const psdr_workspace* ws) {
   int maxspp = 1;
-  long long total = 0;
-  for (auto& v : views) { maxspp = std::max(maxspp, v.spp); total += (long long)v.H * v.W * v.spp; }
-  long long cap = cfg.tile_paths > 0 ? cfg.tile_paths : (1 << 20);
+  long long total = 0, need = 0;
+  for (auto& v : views) {
+    maxspp = std::max(maxspp, v.spp);
+    total += (long long)v.H * v.W * v.spp;
+    if (!backward) continue;
+    // the largest boundary term of the view (backward_unit)
+    const long long px = (long long)v.H * v.W;
+    need = std::max({need, px * cfg.spp_primary_edge, px * cfg.spp_secondary_edge});
+    if (cfg.estimator == PSDR_EST_UNBIASED)
+      need = std::max({need, border_segments(v) * cfg.spp_pixel_boundary,
+                       2ll * kCreaseSamplesPerSpp * cfg.spp_primary_edge, px * v.spp});
+  }
+  need = std::max(need, total);
+  long long cap = cfg.tile_paths > 0 ? cfg.tile_paths : auto_tile(cfg, need, backward, ws);
   if (backward) {
+    if (cfg.tile_paths == 0) {
+      if (lanes > 1) cap = std::min(cap, std::max(kTileMin, (total + lanes - 1) / lanes));
+      cap = std::min(cap, need);
+    }
     long long cells = std::max<long long>(cfg.primary_edge_hypercube_resolution,
                                           (long long)cfg.secondary_edge_hypercube_resolution[0] *
                                               cfg.secondary_edge_hypercube_resolution[1] *
@@ -3523,7 +3572,7 @@ void forward_launch(const DevScene* scenes_dev, const std::vector<DevView>& view
 void render_forward_impl(const DevScene* scenes_dev, std::vector<DevView>& views, const psdr_config& cfg,
                          psdr_workspace* ws, cudaStream_t st, float* samples_out) {
   assign_offsets(views);
-  const int cap = choose_cap(cfg, views, false);
+  const int cap = choose_cap(cfg, views, false, 1, ws);
   const int R = cfg.mis_light_samples + cfg.mis_bsdf_samples + 1;
   ws->ensure(cap, R, cfg.max_bounce, (int)views.size(), 0, st);
   upload_views(ws, views, st);
@@ -3691,7 +3740,7 @@ void backward_launch(const DevScene* scenes_dev, const std::vector<DevView>& vie
 void render_backward_impl(const DevScene* scenes_dev, std::vector<DevView>& views, const psdr_config& cfg,
                           psdr_workspace* ws, const SceneGradInfo& gi, cudaStream_t st) {
   assign_offsets(views);
-  const int cap = choose_cap(cfg, views, true);
+  const int cap = choose_cap(cfg, views, true, 1, ws);
   const int Rmax = cfg.mis_light_samples + std::max(cfg.mis_bsdf_samples, 1) + 1;
   ws->ensure(cap, Rmax, cfg.max_bounce, (int)views.size(), 1, st);
   ensure_border(ws, cfg, views, st);

@@ -138,7 +138,8 @@ void render_backward_impl(const DevScene* scenes_dev, std::vector<DevView>& view
                           psdr_workspace* ws, const SceneGradInfo& gi, cudaStream_t st);
 void grad_out(const GradAcc* acc, float* out, long long n, int accumulate, cudaStream_t st);
 void assign_offsets(std::vector<DevView>& views);
-int choose_cap(const psdr_config& cfg, const std::vector<DevView>& views, bool backward);
+int choose_cap(const psdr_config& cfg, const std::vector<DevView>& views, bool backward, int lanes,
+               const psdr_workspace* ws);
 void upload_views(psdr_workspace* ws, const std::vector<DevView>& views, cudaStream_t st);
 void forward_launch(const DevScene* scenes_dev, const std::vector<DevView>& views, const psdr_config& cfg, int cap,
                     psdr_workspace* ws, cudaStream_t st, float* samples_out);
