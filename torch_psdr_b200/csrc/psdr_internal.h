@@ -56,16 +56,27 @@ struct DBuf {
 int num_sms();
 void count_launches(int n);  // profiler launch counter (psdr_profile_read)
 
-// Scan / sort primitives (sort.cu).
-void exclusive_scan_int(const int* in, int* out, int n, int* tmp_blocks, cudaStream_t st);
+// Scan / sort primitives (sort.cu). Temporary sizes: scan_tmp_ints(n) ints, scan_tmp_doubles(n)
+// doubles.
 size_t scan_tmp_ints(int n);
-void inclusive_scan_double(const double* in, double* out, int n, double* tmp_blocks, cudaStream_t st);
 size_t scan_tmp_doubles(int n);
+void inclusive_scan_double(const double* in, double* out, int n, double* tmp_blocks, cudaStream_t st);
+// Prefix sums of (double)in[i], zero from *n_dev on.
+void inclusive_scan_widen(const float* in, const int* n_dev, double* out, int n, double* tmp_blocks, cudaStream_t st);
 struct SortTmp {
   DBuf keys2, vals2, hist;
 };
+// Sorted pairs: in the caller's arrays or in the temporary ones, whichever the last pass wrote.
+struct SortedKeys {
+  uint64_t* k64 = nullptr;  // 64-bit keys, or
+  uint32_t* k32 = nullptr;  // 32-bit keys
+  uint32_t* vals = nullptr;
+};
 // Stable LSD radix sort of (key, value) pairs over the low `bits` bits of the keys.
-void radix_sort_pairs(uint64_t* keys, uint32_t* vals, int n, int bits, SortTmp& tmp, cudaStream_t st);
+SortedKeys radix_sort_pairs(uint64_t* keys, uint32_t* vals, int n, int bits, SortTmp& tmp, cudaStream_t st);
+SortedKeys radix_sort_pairs(uint32_t* keys, uint32_t* vals, int n, int bits, SortTmp& tmp, cudaStream_t st);
+// out[i] = number of runs of equal keys that start before entry i.
+void exclusive_scan_runs(const SortedKeys& k, int* out, int n, int* tmp_blocks, cudaStream_t st);
 
 }  // namespace psdr
 
@@ -86,12 +97,12 @@ struct psdr_scene {
   psdr::DBuf verts, tri, tri_v, objs, lights_buf, light_pmf, light_cmf, ltri_pmf, ltri_cmf;
   psdr::DBuf n_edges, edge, edge_v, edge_f, edge_pmf, edge_cmf;
   psdr::DBuf nodes, leaf, err;
-  // tree topology of the last full build, kept for psdr_scene_refit: binary child links,
-  // leaf triangle order, 4-wide node flags and indices (the build's scratch is reused)
-  psdr::DBuf bvh_child, bvh_order, bvh_f4;
-  psdr::DBuf bvh_slots;  // per 4-wide node (by binary node id): its four children, -1 for none
+  // tree of the last full build, kept for psdr_scene_refit: leaf triangle order, the leaf
+  // ranges of the binary nodes (range), the children of every 4-wide node (binary ids, -1 for
+  // none) and the number of 4-wide nodes (bvh_counters[0])
+  psdr::DBuf bvh_order, range, bvh_slots, bvh_counters;
   // build scratch
-  psdr::DBuf keys, vals, aux_i, aux_i2, aux_d, aux_d2, aabb, parent, range, flags, cbox;
+  psdr::DBuf keys, vals, aux_i, aux_i2, aux_d, aux_d2, aabb, box_levels, flags, cbox;
   psdr::SortTmp sort_tmp;
   // fp64 gradient accumulators (allocated on first backward)
   psdr::DBuf g_verts, g_tex, g_emit;
