@@ -78,6 +78,15 @@ SortedKeys radix_sort_pairs(uint32_t* keys, uint32_t* vals, int n, int bits, Sor
 // out[i] = number of runs of equal keys that start before entry i.
 void exclusive_scan_runs(const SortedKeys& k, int* out, int n, int* tmp_blocks, cudaStream_t st);
 
+// The caller's buffers of one object, for the geometry build (k_records).
+struct DevSrc {
+  const float* verts;
+  const int* faces;
+  const float* uvs;  // null: the default uvs
+  const int* uvi;
+  int vert_off, tri_off;
+};
+
 }  // namespace psdr
 
 struct psdr_scene {
@@ -93,8 +102,9 @@ struct psdr_scene {
   std::vector<int> obj_vert_off, obj_tri_off, obj_nvert, obj_ntri;
   std::vector<psdr::DevObj> h_objs;
   std::vector<psdr::DevLight> h_lights;
+  std::vector<psdr::DevSrc> h_srcs;
   // device storage
-  psdr::DBuf verts, tri, tri_v, objs, lights_buf, light_pmf, light_cmf, ltri_pmf, ltri_cmf;
+  psdr::DBuf verts, tri, tri_v, objs, srcs, lights_buf, light_pmf, light_cmf, ltri_pmf, ltri_cmf;
   psdr::DBuf n_edges, edge, edge_v, edge_f, edge_pmf, edge_cmf;
   psdr::DBuf nodes, leaf, err;
   // tree of the last full build, kept for psdr_scene_refit: leaf triangle order, the leaf

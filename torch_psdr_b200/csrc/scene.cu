@@ -20,22 +20,46 @@ namespace psdr {
 
 namespace {
 
-// mesh.cc:27-67 triangle attributes (normal, uv tangent, Heron area).
-__global__ void k_tri_records(int nF, const int* __restrict__ faces, int vbase, int tri_off, int obj,
-                              const float* __restrict__ verts, const float* __restrict__ uvs,
-                              const int* __restrict__ uvi, float4* __restrict__ out, int4* __restrict__ out_v) {
-  int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= nF) return;
-  const int i0 = faces[3 * f] + vbase, i1 = faces[3 * f + 1] + vbase, i2 = faces[3 * f + 2] + vbase;
-  const float3 p0 = f3(verts[3 * i0], verts[3 * i0 + 1], verts[3 * i0 + 2]);
-  const float3 p1 = f3(verts[3 * i1], verts[3 * i1 + 1], verts[3 * i1 + 2]);
-  const float3 p2 = f3(verts[3 * i2], verts[3 * i2 + 1], verts[3 * i2 + 2]);
+// Last entry of the table whose offset is at most i.
+template <class F>
+__device__ __forceinline__ int table_find(int n, int i, F off) {
+  int lo = 0, hi = n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (off(mid) <= i) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
+
+// The flattened vertices and the triangle records (mesh.cc:27-67: normal, uv tangent, Heron
+// area) of every object in one launch; a copy and a launch per object took longer than the
+// work of small meshes (17 objects: 34 launches, 110 us).
+__global__ void k_records(int nobj, const DevSrc* __restrict__ src, int nvert, int ntri, float* __restrict__ verts,
+                          float4* __restrict__ out, int4* __restrict__ out_v) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < nvert) {
+    const DevSrc& s = src[table_find(nobj, i, [&](int o) { return src[o].vert_off; })];
+    const float* v = s.verts + 3 * (size_t)(i - s.vert_off);
+    verts[3 * (size_t)i] = v[0];
+    verts[3 * (size_t)i + 1] = v[1];
+    verts[3 * (size_t)i + 2] = v[2];
+  }
+  if (i >= ntri) return;
+  const int obj = table_find(nobj, i, [&](int o) { return src[o].tri_off; });
+  const DevSrc& s = src[obj];
+  const int f = i - s.tri_off;
+  const int j0 = s.faces[3 * f], j1 = s.faces[3 * f + 1], j2 = s.faces[3 * f + 2];
+  const float* V = s.verts;
+  const float3 p0 = f3(V[3 * j0], V[3 * j0 + 1], V[3 * j0 + 2]);
+  const float3 p1 = f3(V[3 * j1], V[3 * j1 + 1], V[3 * j1 + 2]);
+  const float3 p2 = f3(V[3 * j2], V[3 * j2 + 1], V[3 * j2 + 2]);
   float uv[6] = {0.f, 0.f, 0.f, 1.f, 1.f, 0.f};
-  if (uvs && uvi) {
+  if (s.uvs) {
     for (int c = 0; c < 3; ++c) {
-      const int u = uvi[3 * f + c];
-      uv[2 * c] = uvs[2 * u];
-      uv[2 * c + 1] = uvs[2 * u + 1];
+      const int u = s.uvi[3 * f + c];
+      uv[2 * c] = s.uvs[2 * u];
+      uv[2 * c + 1] = s.uvs[2 * u + 1];
     }
   }
   const float3 a = p2 - p1, b = p0 - p2, c = p1 - p0;
@@ -45,17 +69,17 @@ __global__ void k_tri_records(int nF, const int* __restrict__ faces, int vbase, 
   const float3 tw = c * du2y + b * du1y;
   const float3 t = tw / sqrtf(sqnorm(tw));
   const float la = norm(a), lb = norm(b), lc = norm(c);
-  const float s = (la + lb + lc) / 2.0f;
-  const float q = s * (s - la) * (s - lb) * (s - lc);
+  const float hp = (la + lb + lc) / 2.0f;
+  const float q = hp * (hp - la) * (hp - lb) * (hp - lc);
   const float area = q > 0.f ? sqrtf(q) : 0.f;
-  float4* r = out + 6 * (size_t)(tri_off + f);
+  float4* r = out + 6 * (size_t)i;
   r[0] = make_float4(p0.x, p0.y, p0.z, area);
   r[1] = make_float4(p1.x, p1.y, p1.z, __int_as_float(obj));
   r[2] = make_float4(p2.x, p2.y, p2.z, uv[0]);
   r[3] = make_float4(n.x, n.y, n.z, uv[1]);
   r[4] = make_float4(t.x, t.y, t.z, uv[2]);
   r[5] = make_float4(uv[3], uv[4], uv[5], 0.f);
-  out_v[tri_off + f] = make_int4(i0, i1, i2, obj);
+  out_v[i] = make_int4(j0 + s.vert_off, j1 + s.vert_off, j2 + s.vert_off, obj);
 }
 
 // emitter.cc:4-14 + sampler.h:86-96: per-light area, power and triangle CDF.
@@ -651,28 +675,9 @@ int num_sms() {
 // Vertices, triangle records, light tables and the edge list (everything but the BVH).
 // Returns the number of triangles outside the environment light's box.
 static int build_records_and_edges(psdr_scene* s, cudaStream_t st) {
-  // vertices
-  for (int o = 0; o < s->nobj; ++o) {
-    const float* src = o < (int)s->meshes.size() ? s->meshes[o].vertices : s->lights[o - s->meshes.size()].vertices;
-    PSDR_CUDA(cudaMemcpyAsync(s->verts.as<float>() + 3 * (size_t)s->obj_vert_off[o], src,
-                              sizeof(float) * 3 * (size_t)s->obj_nvert[o], cudaMemcpyDeviceToDevice, st));
-  }
-  for (int o = 0; o < s->nobj; ++o) {
-    const bool is_mesh = o < (int)s->meshes.size();
-    const int* faces = is_mesh ? s->meshes[o].faces : s->lights[o - s->meshes.size()].faces;
-    const float* uvs = is_mesh ? s->meshes[o].uvs : nullptr;
-    const int* uvi = is_mesh ? s->meshes[o].uv_indices : nullptr;
-    if (is_mesh && (!uvs || !uvi)) { uvs = nullptr; uvi = nullptr; }
-    // the EnvLight box carries the cube-map uvs
-    if (!is_mesh && o - (int)s->meshes.size() == s->env_light && s->lights[s->env_light].type == PSDR_LIGHT_ENV) {
-      uvs = s->env_uv.as<float>();
-      uvi = s->env_uvi.as<int>();
-    }
-    const int nF = s->obj_ntri[o];
-    if (nF == 0) continue;
-    k_tri_records<<<nblk(nF), 256, 0, st>>>(nF, faces, s->obj_vert_off[o], s->obj_tri_off[o], o, s->verts.as<float>(),
-                                            uvs, uvi, s->tri.as<float4>(), s->tri_v.as<int4>());
-  }
+  k_records<<<nblk(std::max(s->nvert, s->ntri)), 256, 0, st>>>(s->nobj, s->srcs.as<DevSrc>(), s->nvert, s->ntri,
+                                                                s->verts.as<float>(), s->tri.as<float4>(),
+                                                                s->tri_v.as<int4>());
   PSDR_CUDA(cudaGetLastError());
   // lights (the table was uploaded at creation; area, power and CDFs are recomputed)
   if (s->nlight > 0) {
@@ -713,7 +718,7 @@ static int build_records_and_edges(psdr_scene* s, cudaStream_t st) {
                                      s->edge_cmf.as<float>());
   PSDR_CUDA(cudaGetLastError());
   // records, lights, half-edges, run scan (3), edges, length CDF (4)
-  count_launches(s->nobj + (s->nlight > 0) + 9);
+  count_launches(1 + (s->nlight > 0) + 9);
   return n_edge_tri;
 }
 
@@ -811,6 +816,7 @@ void psdr_scene_alloc(psdr_scene* s) {
   s->tri.alloc(sizeof(float4) * 6 * n, st);
   s->tri_v.alloc(sizeof(int4) * n, st);
   s->objs.alloc(sizeof(DevObj) * std::max(1, s->nobj), st);
+  s->srcs.alloc(sizeof(DevSrc) * std::max(1, s->nobj), st);
   s->lights_buf.alloc(sizeof(DevLight) * std::max(1, s->nlight), st);
   s->light_pmf.alloc(sizeof(float) * std::max(1, s->nlight), st);
   s->light_cmf.alloc(sizeof(float) * std::max(1, s->nlight), st);
@@ -868,6 +874,26 @@ void psdr_scene::upload_tables() {
   using namespace psdr;
   PSDR_CUDA(cudaMemcpyAsync(objs.p, h_objs.data(), sizeof(DevObj) * std::max<size_t>(1, h_objs.size()),
                             cudaMemcpyHostToDevice, stream));
+  h_srcs.clear();
+  for (int o = 0; o < nobj; ++o) {
+    const bool is_mesh = o < (int)meshes.size();
+    const int l = o - (int)meshes.size();
+    DevSrc d{};
+    d.verts = is_mesh ? meshes[o].vertices : lights[l].vertices;
+    d.faces = is_mesh ? meshes[o].faces : lights[l].faces;
+    if (is_mesh && meshes[o].uvs && meshes[o].uv_indices) {
+      d.uvs = meshes[o].uvs;
+      d.uvi = meshes[o].uv_indices;
+    } else if (!is_mesh && l == env_light && lights[l].type == PSDR_LIGHT_ENV) {
+      // the EnvLight box carries the cube-map uvs
+      d.uvs = env_uv.as<float>();
+      d.uvi = env_uvi.as<int>();
+    }
+    d.vert_off = obj_vert_off[o];
+    d.tri_off = obj_tri_off[o];
+    h_srcs.push_back(d);
+  }
+  PSDR_CUDA(cudaMemcpyAsync(srcs.p, h_srcs.data(), sizeof(DevSrc) * h_srcs.size(), cudaMemcpyHostToDevice, stream));
   if (nlight > 0)
     PSDR_CUDA(cudaMemcpyAsync(lights_buf.p, h_lights.data(), sizeof(DevLight) * nlight, cudaMemcpyHostToDevice,
                               stream));
