@@ -113,14 +113,6 @@ SceneGradInfo grad_info(const psdr_scene* s) {
   SceneGradInfo gi;
   gi.bsdf = s->has_bsdf || s->env_light >= 0 ? 1 : 0;
   gi.jump = s->has_bsdf ? 1 : 0;
-  const int nm = (int)s->meshes.size();
-  if (s->nlight == 1) {
-    gi.emit_hot = 1;
-    if (s->obj_nvert[nm] <= kMaxLightVerts) {
-      gi.hot_lv0 = s->obj_vert_off[nm];
-      gi.hot_nlv = s->obj_nvert[nm];
-    }
-  }
   return gi;
 }
 

@@ -151,8 +151,11 @@ struct DevLight {
 //  [0] lo.x of children 0..3 [1] hi.x [2] lo.y [3] hi.y [4] lo.z [5] hi.z [6] links (int) [7] -
 // link >= 0: internal node; link < 0: leaf ~((first << 3) | (count-1)); 0x7fffffff: empty.
 // Leaf triangles, 3 x float4 (48 B) in BVH order: p0.xyz + id(bits), p1.xyz, p2.xyz.
+constexpr int kMaxLightVerts = 8;  // light vertices whose gradients the adjoint sums per lane
+
 struct DevScene {
   int ntri, nvert, nobj, nlight;
+  int light_v0, light_nv;  // vertices of the only light (0: several lights, or more than kMaxLightVerts)
   const float4* tri;
   const int4* tri_v;       // global vertex ids (x,y,z) + object (w)
   const float* verts;      // (nvert, 3)

@@ -9,7 +9,6 @@ namespace psdr {
 
 constexpr int kMaxDepth = 16;
 constexpr int kMaxRays = 18;          // rays per path per depth: light + bsdf + indirect
-constexpr int kMaxLightVerts = 8;     // light vertices accumulated in registers by the adjoint
 
 // One camera view of a job. Matrices are row-major 4x4 (camera.h:108-124).
 struct DevView {
@@ -130,7 +129,6 @@ void make_view(const psdr_camera_desc& c, int spp, DevView& v);
 void render_forward_impl(const DevScene* scenes_dev, std::vector<DevView>& views, const psdr_config& cfg,
                          psdr_workspace* ws, cudaStream_t st, float* samples_out);
 struct SceneGradInfo {
-  int hot_lv0 = 0, hot_nlv = 0, emit_hot = 0;
   int bsdf = 0;  // a DiffuseBsdfMaterial mesh or an environment light (extended adjoint kernel)
   int jump = 0;  // a DiffuseBsdfMaterial mesh: the unbiased default terms include its BRDF jumps
 };

@@ -851,6 +851,10 @@ void psdr_scene_alloc(psdr_scene* s) {
   PSDR_CUDA(cudaMemsetAsync(s->err.p, 0, sizeof(int), st));
   DevScene& d = s->dev;
   d.ntri = s->ntri; d.nvert = s->nvert; d.nobj = s->nobj; d.nlight = s->nlight;
+  const int nm = (int)s->meshes.size();
+  const bool hot = s->nlight == 1 && s->obj_nvert[nm] <= kMaxLightVerts;
+  d.light_v0 = hot ? s->obj_vert_off[nm] : 0;
+  d.light_nv = hot ? s->obj_nvert[nm] : 0;
   d.tri = s->tri.as<float4>(); d.tri_v = s->tri_v.as<int4>(); d.verts = s->verts.as<float>();
   d.objs = s->objs.as<DevObj>(); d.lights = s->lights_buf.as<DevLight>();
   d.light_pmf = s->light_pmf.as<float>(); d.light_cmf = s->light_cmf.as<float>();
