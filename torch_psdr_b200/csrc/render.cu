@@ -1175,7 +1175,7 @@ PSDR_D bool primary_point(const WF& w, const DevScene* __restrict__ scenes, cons
 constexpr int kVertCap = 64;     // at most 31 waiting + 32 new
 constexpr int kVertFields = 22;
 constexpr int kHitFields = 11;
-constexpr int kAdjWarps = 4;
+constexpr int kAdjWarps = 8;
 __host__ __device__ constexpr int adj_hit_cap(int nB) { return 32 + 32 * (nB > 0 ? nB : 1); }
 __host__ __device__ constexpr int adj_warp_words(int nB) { return kVertFields * kVertCap + kHitFields * adj_hit_cap(nB); }
 
@@ -1184,10 +1184,12 @@ __host__ __device__ constexpr int adj_warp_words(int nB) { return kVertFields * 
 // (about one in twenty), go to the warp's lists and are worked on 32 at a time. Walking
 // each path to its end instead (one thread per path over all depths) ran every depth's code
 // for the few paths still alive, and the BSDF-sample code for two lanes of a warp on average:
-// 5.3 ms per 512^2 x 32 spp x depth 3 step against 2.7 ms now. The kernel is bound by
-// instruction fetch and issue; its records are read once.
+// 5.8 ms per 512^2 x 32 spp x depth 3 step against 2.9 ms with lists; 2.3 ms with the warps of a
+// block starting together. Bound by instruction fetch (7.2 of 18.3 cycles per issued
+// instruction before that, 25 % occupancy at 128 registers) and by the latency of its record
+// loads; DRAM 7 % busy.
 template <bool UNB>
-__global__ void __launch_bounds__(32 * kAdjWarps, 4) k_adjoint(WF w, const DevScene* __restrict__ scenes,
+__global__ void __launch_bounds__(32 * kAdjWarps, 2) k_adjoint(WF w, const DevScene* __restrict__ scenes,
                                                                const DevView* __restrict__ views, Tile tile) {
   extern __shared__ float adj_lists[];
   const int lane = threadIdx.x & 31;
@@ -1206,7 +1208,10 @@ __global__ void __launch_bounds__(32 * kAdjWarps, 4) k_adjoint(WF w, const DevSc
   const int stride = gridDim.x * blockDim.x;
   int s0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31);  // first path of the warp's next 32
   while (true) {
+    // The block's warps start each batch together: the kernel is bound by instruction fetch, and
+    // warps that run the same code at the same time share it.
     const bool more = s0 < tile.n;
+    if (!__syncthreads_or(more || nv > 0 || nh > 0)) break;
     if (nh >= 32 || (nh > 0 && nv == 0 && !more)) {
       // ---- BSDF samples that hit a light
       const int take = min(32, nh);
@@ -1236,7 +1241,7 @@ __global__ void __launch_bounds__(32 * kAdjWarps, 4) k_adjoint(WF w, const DevSc
       continue;
     }
     const bool fresh = nv < 32 && more;
-    if (!fresh && nv == 0) break;
+    if (!fresh && nv == 0) continue;
     bool act = false, has0 = false;  // act: a vertex to work on; has0: a fresh path with something to scatter
     int s = 0, d = 0, tri = -1;
     float4 hx = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -4051,9 +4056,13 @@ std::vector<std::vector<Tile>> schedule_tiles(const std::vector<Tile>& tiles, in
 // paths), as many as are resident.
 template <bool UNB>
 static void launch_adjoint(const WF& w, const DevScene* scenes, const DevView* vd, const Tile& t, cudaStream_t st) {
-  const int bytes = (int)sizeof(float) * kAdjWarps * adj_warp_words(w.nB);
-  PSDR_CUDA(cudaFuncSetAttribute(k_adjoint<UNB>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  k_adjoint<UNB><<<grid_for(t.n, 32 * kAdjWarps, 4), 32 * kAdjWarps, bytes, st>>>(w, scenes, vd, t);
+  // fewer warps where many BSDF samples make the lists long (nB > 13)
+  int warps = kAdjWarps;
+  constexpr int kMost = 200 << 10;  // shared memory of a block
+  while (warps > 1 && (int)sizeof(float) * warps * adj_warp_words(w.nB) > kMost) warps >>= 1;
+  const int bytes = (int)sizeof(float) * warps * adj_warp_words(w.nB);
+  PSDR_CUDA(cudaFuncSetAttribute(k_adjoint<UNB>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
+  k_adjoint<UNB><<<grid_for(t.n, 32 * warps, 2), 32 * warps, bytes, st>>>(w, scenes, vd, t);
 }
 
 // Device work of one backward unit on workspace ws (views at vd); no allocation, no
