@@ -2774,10 +2774,9 @@ __global__ void __launch_bounds__(256) k_jump_final(WF w, const DevScene* __rest
 // albedos of the diffuse bounces between x_d and the camera-visible vertex.
 // BSDF: the DiffuseBsdfMaterial instance (direction-dependent f at the receiver and
 // along the bounce chain); the other instance is the DiffuseMaterial one.
-// The draws of shadow-boundary sample i: hypercube cell and position (PRE: the cell's
-// sampler stream, persisted in w.rs / w.ri from the second preprocess round on), edge point x_b,
-// light point y; returns the silhouette test (the edge's faces see y on opposite sides).
-// PRE leaves the sampler state after the draws in `rng`; the caller persists it.
+// The draws of shadow-boundary sample i: hypercube cell and position (PRE: the three draws of
+// preprocess round `round` in the cell's sampler stream; each round takes three), edge point
+// x_b, light point y; returns the silhouette test (the edge's faces see y on opposite sides).
 struct DirDraw {
   Rng rng;
   float hpdf, sx, pdf_e;
@@ -2791,8 +2790,8 @@ PSDR_D bool direct_draw(const WF& w, const DevScene& sc, const HCube& hc, int ro
   float s3[3];
   o.hpdf = 1.f;
   if (PRE) {
-    if (round == 0) o.rng = make_rng((unsigned long long)i);
-    else { o.rng.state = w.rs[i]; o.rng.inc = w.ri[i]; }
+    o.rng = make_rng((unsigned long long)i);
+    for (int k = 0; k < 3 * round; ++k) o.rng.next(true);
     const int r12 = hc.res[1] * hc.res[2];
     const int c0 = (int)(i / r12);
     const int rem = (int)(i - (long long)c0 * r12);
@@ -2839,51 +2838,59 @@ PSDR_D bool direct_draw(const WF& w, const DevScene& sc, const HCube& hc, int ro
   return dot(o.nl, o.dir) * dot(o.nr, o.dir) < 0.f && norm(o.nl - o.nr) > kEps;
 }
 
+// The queue of the samples that pass the silhouette test: the ray origins' array (unused by these
+// samples), which holds four entries per path of the tile.
+PSDR_D int* direct_queue(const WF& w) { return reinterpret_cast<int*>(w.ro); }
+constexpr int kDirectPerPath = 4;
+
+// Index k of a preprocess launch: cell k % cells of round round0 + k / cells.
+PSDR_D long long direct_index(bool pre, const HCube& hc, int round0, long long k, int& round) {
+  if (!pre) return k;
+  const int cells = hc.res[0] * hc.res[1] * hc.res[2];
+  const long long r = k / cells;
+  round = round0 + (int)r;
+  return k - r * cells;
+}
+
 // First stage of the shadow-boundary samples [begin, begin + n): the draws and the
-// silhouette test only; the samples that pass are queued (w.q0, count in w.cnt[0]) for
+// silhouette test only; the samples that pass are queued (direct_queue, count in w.cnt[0]) for
 // k_direct, whose warps then start with every lane on a sample that traces (most samples
-// fail the test, and a lane that fails would idle while its warp traces). PRE persists the
-// sampler state of the cells that fail; k_direct does it for the others.
+// fail the test, and a lane that fails would idle while its warp traces).
 template <bool PRE, bool UNB>
 __global__ void __launch_bounds__(256) k_direct_pick(WF w, const DevScene* __restrict__ scenes,
                                                      const DevView* __restrict__ views, int v, long long begin,
-                                                     int n, HCube hc, int round) {
+                                                     int n, HCube hc, int round0) {
   const DevScene& sc = scenes[views[v].scene];
   const int stride = gridDim.x * blockDim.x;
   const int n32 = (n + 31) & ~31;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n32; k += stride) {
     bool ok = false;
     if (k < n) {
-      const long long i = begin + k;
+      int round = 0;
+      const long long i = direct_index(PRE, hc, round0, begin + k, round);
       DirDraw o;
       ok = direct_draw<PRE, UNB>(w, sc, hc, round, i, o);
-      if (PRE && !ok) {
-        w.rs[i] = o.rng.state;
-        w.ri[i] = o.rng.inc;
-      }
     }
     const int q = warp_append(&w.cnt[0], ok);
-    if (ok) w.q0[q] = k;
+    if (ok) direct_queue(w)[q] = k;
   }
 }
 
 template <bool PRE, bool UNB, bool BSDF>
 __global__ void __launch_bounds__(128) k_direct(WF w, const DevScene* __restrict__ scenes,
                                                 const DevView* __restrict__ views, int v, long long begin, HCube hc,
-                                                int round, float* mass, int spp) {
+                                                int round0, float* mass, int spp) {
   const DevView& V = views[v];
   const DevScene& sc = scenes[V.scene];
   const int nq = w.cnt[0];
   const int stride = gridDim.x * blockDim.x;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += stride) {
-    const long long i = begin + w.q0[q];
+    const long long k = begin + direct_queue(w)[q];  // PRE: also the sample's entry in `mass`
+    int round = 0;
+    const long long i = direct_index(PRE, hc, round0, k, round);
     DirDraw o;
     if (!direct_draw<PRE, UNB>(w, sc, hc, round, i, o)) continue;
     Rng& rng = o.rng;
-    if (PRE) {
-      w.rs[i] = rng.state;
-      w.ri[i] = rng.inc;
-    }
     const float hpdf = o.hpdf, sx = o.sx, pdf_e = o.pdf_e;
     const int e = o.e;
     const float3 p0 = o.p0, p1 = o.p1, out = o.out, xb = o.xb, dir = o.dir;
@@ -2968,7 +2975,7 @@ __global__ void __launch_bounds__(128) k_direct(WF w, const DevScene* __restrict
       }
       if (PRE) {
         const float m = msum * norm(nsv);
-        if (isfinite(m)) mass[i] = mass[i] + m;
+        if (isfinite(m)) mass[k] = m;
         continue;
       }
       const float3 a = nsv * (wsum / (hpdf * (float)hc.ncells * (float)spp));
@@ -3031,7 +3038,7 @@ __global__ void __launch_bounds__(128) k_direct(WF w, const DevScene* __restrict
       val.x = val.x < kEps ? kEps : val.x;
       val.y = val.y < kEps ? kEps : val.y;
       val.z = val.z < kEps ? kEps : val.z;
-      mass[i] = mass[i] + norm(val);
+      mass[k] = norm(val);
     } else {
       const float3 nep = cross(nd, ep);
       const float3 z = mul(mul(mul(f3(0.f, 0.f, 0.f), nep * dG) * Jb / pdf_xw, Ts), Td);
@@ -3084,6 +3091,9 @@ constexpr int kIndirectSampleDiv = 4, kIndirectCellDiv = 4;
 // are heavy-tailed, and with four samples per cell its standard deviation on the 512²
 // icosphere workload drops by a third (about 2.5x less variance) for ~1 ms.
 constexpr int kDirectGuideRounds = 4;
+// Preprocess rounds of the shadow-boundary guide that run in one launch (a launch of 360k cells
+// traces few enough samples to be bound by its longest chain of rays).
+constexpr int kGuideRounds = 8;
 
 // Direction of lune coordinates (u2, u3) in [0, 1)^2 at an edge with unit direction ev and
 // unit face normals nl, nr (both perpendicular to ev); alpha gets the wedge angle.
@@ -3272,6 +3282,13 @@ __global__ void __launch_bounds__(128) k_indirect_final(WF w, const DevScene* __
 }
 
 // ------------------------------------------------------------------ small utilities
+__global__ void k_mass_rounds(const float* __restrict__ rm, int cells, int rounds, float* __restrict__ mass) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= cells) return;
+  float m = mass[i];
+  for (int r = 0; r < rounds; ++r) m = m + rm[(size_t)r * cells + i];
+  mass[i] = m;
+}
 __global__ void k_mass_cdf(const float* __restrict__ mass, int n, double* __restrict__ w) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) w[i] = (double)mass[i];
@@ -3557,19 +3574,20 @@ static int any_ortho(const std::vector<DevView>& views) {
   return 0;
 }
 
-// Shadow-boundary samples [0, n) in chunks of the tile capacity: the pick stage queues the
+// Shadow-boundary samples [0, n) in chunks of four tile capacities: the pick stage queues the
 // samples that pass the silhouette test, then the k_direct instance for the job's
-// materials (w.bsdf) traces them.
+// materials (w.bsdf) traces them. PRE: n = cells x rounds, from round0 on.
 template <bool PRE, bool UNB>
 static void launch_direct(const WF& w, cudaStream_t st, const DevScene* scenes, const DevView* vd, int v,
-                          long long n, const HCube& hc, int round, float* mass, int spp) {
-  for (long long b = 0; b < n; b += w.cap) {
-    const int nb = (int)std::min<long long>(w.cap, n - b);
+                          long long n, const HCube& hc, int round0, float* mass, int spp) {
+  const long long chunk = std::min<long long>((long long)kDirectPerPath * w.cap, 1 << 30);
+  for (long long b = 0; b < n; b += chunk) {
+    const int nb = (int)std::min<long long>(chunk, n - b);
     PSDR_CUDA(cudaMemsetAsync(w.cnt, 0, sizeof(int), st));
-    k_direct_pick<PRE, UNB><<<grid_for(nb, 256, 8), 256, 0, st>>>(w, scenes, vd, v, b, nb, hc, round);
+    k_direct_pick<PRE, UNB><<<grid_for(nb, 256, 8), 256, 0, st>>>(w, scenes, vd, v, b, nb, hc, round0);
     const int g = grid_for(nb, 128, 16);
-    if (w.bsdf) k_direct<PRE, UNB, true><<<g, 128, 0, st>>>(w, scenes, vd, v, b, hc, round, mass, spp);
-    else k_direct<PRE, UNB, false><<<g, 128, 0, st>>>(w, scenes, vd, v, b, hc, round, mass, spp);
+    if (w.bsdf) k_direct<PRE, UNB, true><<<g, 128, 0, st>>>(w, scenes, vd, v, b, hc, round0, mass, spp);
+    else k_direct<PRE, UNB, false><<<g, 128, 0, st>>>(w, scenes, vd, v, b, hc, round0, mass, spp);
     PSDR_LAUNCHED(2);
   }
   PSDR_CUDA(cudaGetLastError());
@@ -3908,7 +3926,11 @@ long long border_segments(const DevView& V) {
 }
 
 void ensure_border(psdr_workspace* ws, const psdr_config& cfg, const std::vector<DevView>& views, cudaStream_t st) {
-  if (cfg.estimator != PSDR_EST_UNBIASED) return;
+  const bool unb = cfg.estimator == PSDR_EST_UNBIASED;
+  const int* r3 = cfg.secondary_edge_hypercube_resolution;
+  const int rounds = std::min(kGuideRounds, cfg.secondary_edge_preprocess_rounds * (unb ? kDirectGuideRounds : 1));
+  ws->mass_rounds.alloc(sizeof(float) * (size_t)r3[0] * r3[1] * r3[2] * rounds, st);
+  if (!unb) return;
   long long s = kCreaseCap, nt = 1;
   for (const DevView& v : views) {
     s = std::max(s, border_segments(v));
@@ -4150,9 +4172,16 @@ void backward_unit(const DevScene* scenes_dev, const std::vector<DevView>& views
       for (int k = 0; k < 3; ++k) { pre.res[k] = r3[k]; pre.unit[k] = 1.0f / (float)r3[k]; }
       const int rounds = cfg.secondary_edge_preprocess_rounds * (unb ? kDirectGuideRounds : 1);
       PSDR_LAUNCHED(1);
-      for (int r = 0; r < rounds; ++r) {
-        if (unb) launch_direct<true, true>(w, st, scenes_dev, vd, v, cells, pre, r, ws->mass.as<float>(), 1);
-        else launch_direct<true, false>(w, st, scenes_dev, vd, v, cells, pre, r, ws->mass.as<float>(), 1);
+      // the rounds' samples draw from known places of their cells' streams: up to kGuideRounds of
+      // them run in one launch, and their masses are added up in order
+      float* rm = ws->mass_rounds.as<float>();
+      for (int r = 0; r < rounds; r += kGuideRounds) {
+        const int nr = std::min(kGuideRounds, rounds - r);
+        PSDR_CUDA(cudaMemsetAsync(rm, 0, sizeof(float) * (size_t)cells * nr, st));
+        if (unb) launch_direct<true, true>(w, st, scenes_dev, vd, v, (long long)cells * nr, pre, r, rm, 1);
+        else launch_direct<true, false>(w, st, scenes_dev, vd, v, (long long)cells * nr, pre, r, rm, 1);
+        k_mass_rounds<<<(cells + 255) / 256, 256, 0, st>>>(rm, cells, nr, ws->mass.as<float>());
+        PSDR_LAUNCHED(1);
       }
       const HCube hc = build_hcube(ws, cells, r3, 3, unb, st);
       const long long N = (long long)V.H * V.W * cfg.spp_secondary_edge;

@@ -90,7 +90,7 @@ struct psdr_ws_impl;
 struct psdr_workspace {
   int cap = 0, R = 0, D = 0, nviews_cap = 0;
   psdr::DBuf rs, ri, view, pix, T, L, cur, org, q0, q1, qs, cnt, ro, rd, ra, hit, rec;
-  psdr::DBuf views, eb_a, eb_n, eb_hb, eb_La, eb_rng, mass, mass_d, mass_pre, hc_pmf, hc_cmf, scan_tmp, ncells;
+  psdr::DBuf views, eb_a, eb_n, eb_hb, eb_La, eb_rng, mass, mass_rounds, mass_d, mass_pre, hc_pmf, hc_cmf, scan_tmp, ncells;
   psdr::DBuf campos_acc, lens_acc;
   psdr::DBuf crease;  // interpenetration segments (unbiased estimator): kCreaseCap records + count
   long long mass_cap = 0;
