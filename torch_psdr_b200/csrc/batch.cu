@@ -185,6 +185,7 @@ PSDR_API psdr_status psdr_batch_create(psdr_scene* const* scenes, int32_t n_scen
         b->keep_view.alloc(4 * (size_t)paths, st);
         b->keep_pix.alloc(4 * (size_t)paths, st);
         b->keep.rec = b->keep_rec.as<float4>();
+        b->keep.plane = (size_t)paths;
         b->keep.view = b->keep_view.as<int>();
         b->keep.pix = b->keep_pix.as<int>();
       }

@@ -97,6 +97,15 @@ PSDR_D int find_view_pix(const DevView* __restrict__ views, int nv, long long g)
   return lo;
 }
 
+// Replay record k of path s: 0 its primary hit; 1 + d R + r the hit of ray r of depth d;
+// 1 + D R + 2 d and the next the depth's contribution C and throughput factor beta. Records lie
+// field by field, so that a warp's neighbouring paths read and write whole lines (path by
+// path, 264 B apart, each access of a depth-3 path moved a 32-byte sector for 16 bytes).
+PSDR_D float4& rec_at(const WF& w, int s, int k) { return w.rec[(size_t)k * w.rec_plane + s]; }
+PSDR_D float4& rec_hit(const WF& w, int s, int d, int r) { return rec_at(w, s, 1 + d * w.R + r); }
+PSDR_D float4& rec_c(const WF& w, int s, int d) { return rec_at(w, s, 1 + w.D * w.R + 2 * d); }
+PSDR_D float4& rec_beta(const WF& w, int s, int d) { return rec_at(w, s, 2 + w.D * w.R + 2 * d); }
+
 PSDR_D float4 hit4(const HitRec& h) { return make_float4(__int_as_float(h.tri), h.b1, h.b2, h.t); }
 
 // Out of line: the adjoint kernels scatter vertex and texel gradients from many call
@@ -154,12 +163,7 @@ __global__ void __launch_bounds__(256, MODE != MODE_FWD ? 4 : 1) k_camera(WF w, 
       w.T[s] = make_float4(1.f, 1.f, 1.f, 0.f);
       w.L[s] = make_float4(0.f, 0.f, 0.f, 0.f);
       w.cur[s] = hit4(h);
-      if (MODE != MODE_FWD) {
-        float4* rec = w.rec + (size_t)s * w.rec_stride;
-        rec[0] = hit4(h);
-        float4* cb = rec + 1 + (size_t)w.D * w.R;
-        for (int q = 0; q < 2 * w.D; ++q) cb[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-      }
+      if (MODE != MODE_FWD) rec_at(w, s, 0) = hit4(h);
       alive = h.tri >= 0;
     }
     const int k = warp_append(&w.cnt[0], alive);
@@ -466,6 +470,7 @@ __global__ void __launch_bounds__(256) k_accum(WF w, const DevScene* __restrict_
         C += mul(light_emit<BSDF>(Lt, q), f) * (G / pdf_b * wgt);
       }
       float4 hn = make_float4(__int_as_float(-1), 0.f, 0.f, 0.f);
+      bool more = false;  // the next depth shades the path
       if (!last) {
         const size_t slot = (w.nL + w.nB) * cs + k;
         hn = w.hit[slot];
@@ -481,16 +486,22 @@ __global__ void __launch_bounds__(256) k_accum(WF w, const DevScene* __restrict_
           w.cur[s] = hn;
           w.org[s] = make_float4(x.p.x, x.p.y, x.p.z, 0.f);
           cont = true;
+          more = !nx.is_light;
         }
       }
       if (MODE != MODE_FWD) {
-        float4* rec = w.rec + (size_t)s * w.rec_stride;
-        float4* rh = rec + 1 + (size_t)d * w.R;
         const int Rd = last ? w.R - 1 : w.R;
-        for (int r = 0; r < Rd; ++r) rh[r] = w.hit[r * cs + k];
-        float4* cb = rec + 1 + (size_t)w.D * w.R + 2 * d;
-        cb[0] = make_float4(C.x, C.y, C.z, 0.f);
-        cb[1] = make_float4(beta.x, beta.y, beta.z, 0.f);
+        for (int r = 0; r < Rd; ++r) rec_hit(w, s, d, r) = w.hit[r * cs + k];
+        rec_c(w, s, d) = make_float4(C.x, C.y, C.z, 0.f);
+        rec_beta(w, s, d) = make_float4(beta.x, beta.y, beta.z, 0.f);
+        // a path that is not shaded again: nothing comes from the depths it does not reach (the
+        // records of paths that miss the scene, or see a light, are never read past the first)
+        if (!more) {
+          for (int q = d + 1; q < w.D; ++q) {
+            rec_c(w, s, q) = make_float4(0.f, 0.f, 0.f, 0.f);
+            rec_beta(w, s, q) = make_float4(0.f, 0.f, 0.f, 0.f);
+          }
+        }
       }
       if (MODE != MODE_REPLAY) {
         const float3 T = xyz(w.T[s]);
@@ -519,7 +530,7 @@ __global__ void k_film(WF w, const DevView* __restrict__ views, Tile tile, int n
     for (int k = 0; k < V.spp; ++k) {
       const long long s = s0 + k;
       float3 L = xyz(w.L[s]);
-      if (!finite3(L) || __float_as_int(w.cur[s].x) == -2) L = f3(0.f, 0.f, 0.f);
+      if (!finite3(L)) L = f3(0.f, 0.f, 0.f);
       if (samples_out) {
         samples_out[3 * (lp * V.spp + k)] = L.x;
         samples_out[3 * (lp * V.spp + k) + 1] = L.y;
@@ -1074,9 +1085,9 @@ PSDR_D void scatter_tex_warp(const DevTex* tx, int off, float3 a, bool active) {
 // its sampler stream, and every depth's reverse-mode adjoint is applied
 // (PSDR_EST_REFERENCE: pdfs and MIS weights are constants, jacobi = area/detach(area),
 // barycentrics are not differentiated), scattering into fp64 accumulators.
-PSDR_D float3 suffix_radiance(const float4* __restrict__ cb, int from, int D) {
+PSDR_D float3 suffix_radiance(const WF& w, int s, int from) {
   float3 S = f3(0.f, 0.f, 0.f);
-  for (int k = D - 1; k >= from; --k) S = xyz(cb[2 * k]) + mul(xyz(cb[2 * k + 1]), S);
+  for (int k = w.D - 1; k >= from; --k) S = xyz(rec_c(w, s, k)) + mul(xyz(rec_beta(w, s, k)), S);
   return S;
 }
 
@@ -1150,7 +1161,7 @@ PSDR_D bool primary_point(const WF& w, const DevScene* __restrict__ scenes, cons
   const DevView& V = views[w.view[s]];
   Vp = &V;
   scp = &scenes[V.scene];
-  h0 = w.rec[(size_t)s * w.rec_stride];
+  h0 = rec_at(w, s, 0);
   const int tri0 = __float_as_int(h0.x);
   if (tri0 < 0 || !V.dimage) return false;
   const float* gp = V.dimage + 3 * (size_t)w.pix[s];
@@ -1224,16 +1235,15 @@ __global__ void __launch_bounds__(32 * kAdjWarps, 2) k_adjoint(WF w, const DevSc
         const float3 org = f3(hget(4, e), hget(5, e), hget(6, e)), adjC = f3(hget(7, e), hget(8, e), hget(9, e));
         const DevScene& sc = scenes[__float_as_int(hget(10, e))];
         hot_bind(hot, &sc);
-        const float4* rec = w.rec + (size_t)s * w.rec_stride;
-        const float4 hx = d == 0 ? rec[0] : rec[1 + (size_t)(d - 1) * w.R + w.nL + w.nB];
+        const float4 hx = d == 0 ? rec_at(w, s, 0) : rec_hit(w, s, d - 1, w.nL + w.nB);
         const int tri = __float_as_int(hx.x);
         const Surf x = make_surf(sc, tri, hx.y, hx.z, org);
         const DevObj& ob = sc.objs[x.obj];
         const int off = texel_offset(ob.color, x.u, x.v);
         SurfAdj ax = zero_adj();
         float3 atx = f3(0.f, 0.f, 0.f);
-        bsdf_sample_adj<UNB, false>(w, sc, x, tex_rgb(ob.color, off) * kInvPi, rx, ry, rec[1 + (size_t)d * w.R + w.nL + j],
-                                    adjC, ax, hot, atx, nullptr, nullptr);
+        bsdf_sample_adj<UNB, false>(w, sc, x, tex_rgb(ob.color, off) * kInvPi, rx, ry,
+                                    rec_hit(w, s, d, w.nL + j), adjC, ax, hot, atx, nullptr, nullptr);
         scatter_tex(ob.color, off, atx, false);
         scatter_mesh(sc, tri, hx.y, hx.z, x.front, ax);
       }
@@ -1270,7 +1280,7 @@ __global__ void __launch_bounds__(32 * kAdjWarps, 2) k_adjoint(WF w, const DevSc
             add_emit(*scp, hot, x.light, g);
           }
         } else {
-          const float3 L = suffix_radiance(w.rec + (size_t)s * w.rec_stride + 1 + (size_t)w.D * w.R, 0, w.D);
+          const float3 L = suffix_radiance(w, s, 0);
           if (finite3(L)) {
             act = has0 = true;
             rng = make_rng((unsigned long long)(tile.begin + s - V.sample_off) + w.seed);
@@ -1302,14 +1312,12 @@ __global__ void __launch_bounds__(32 * kAdjWarps, 2) k_adjoint(WF w, const DevSc
         hot_bind(hot, scp);
         const float* gp = V.dimage + 3 * (size_t)w.pix[s];
         g = f3(gp[0], gp[1], gp[2]) / (float)V.spp;
-        hx = w.rec[(size_t)s * w.rec_stride + 1 + (size_t)(d - 1) * w.R + w.nL + w.nB];
+        hx = rec_hit(w, s, d - 1, w.nL + w.nB);
         tri = __float_as_int(hx.x);
         x = make_surf(*scp, tri, hx.y, hx.z, org);
       }
       __syncwarp();
     }
-    const float4* hits = w.rec + (size_t)s * w.rec_stride + 1 + (size_t)d * w.R;
-    const float4* cb = w.rec + (size_t)s * w.rec_stride + 1 + (size_t)w.D * w.R;
     const DevTex* tx = nullptr;
     int toff = 0;
     float3 atx = f3(0.f, 0.f, 0.f), bsdf = atx;
@@ -1320,7 +1328,7 @@ __global__ void __launch_bounds__(32 * kAdjWarps, 2) k_adjoint(WF w, const DevSc
       bsdf = tex_rgb(*tx, toff) * kInvPi;
       for (int i = 0; i < w.nL; ++i) {
         const float rx = rng.next_float(), ry = rng.next_float();
-        light_sample_adj<false>(w, *scp, x, bsdf, rx, ry, hits[i], adjC, ax, hot, atx, nullptr, nullptr);
+        light_sample_adj<false>(w, *scp, x, bsdf, rx, ry, rec_hit(w, s, d, i), adjC, ax, hot, atx, nullptr, nullptr);
       }
     }
     for (int j = 0; j < w.nB; ++j) {
@@ -1329,7 +1337,7 @@ __global__ void __launch_bounds__(32 * kAdjWarps, 2) k_adjoint(WF w, const DevSc
       if (act) {
         rx = rng.next_float();
         ry = rng.next_float();
-        const int t = __float_as_int(hits[w.nL + j].x);
+        const int t = __float_as_int(rec_hit(w, s, d, w.nL + j).x);
         hit = t >= 0 && scp->objs[__ldg(scp->tri_v + t).w].light >= 0;
       }
       const unsigned m = __ballot_sync(0xffffffffu, hit);
@@ -1350,9 +1358,9 @@ __global__ void __launch_bounds__(32 * kAdjWarps, 2) k_adjoint(WF w, const DevSc
     Surf nx;
     if (act && d < w.D - 1) {
       const float rx = rng.next_float(), ry = rng.next_float();
-      const float3 adjB = mul(adjC, suffix_radiance(cb, d + 1, w.D));
-      go = continuation_adj<UNB, false>(*scp, x, bsdf, rx, ry, hits[w.nL + w.nB], adjB, ax, carry, nx, atx, nullptr,
-                                        nullptr) &&
+      const float3 adjB = mul(adjC, suffix_radiance(w, s, d + 1));
+      go = continuation_adj<UNB, false>(*scp, x, bsdf, rx, ry, rec_hit(w, s, d, w.nL + w.nB), adjB, ax, carry, nx, atx,
+                                        nullptr, nullptr) &&
            !nx.is_light;  // a path that ends on a light has nothing downstream
     }
     if (fresh) {
@@ -1365,7 +1373,7 @@ __global__ void __launch_bounds__(32 * kAdjWarps, 2) k_adjoint(WF w, const DevSc
     const unsigned m = __ballot_sync(0xffffffffu, go);
     if (go) {
       const int e = nv + __popc(m & lanemask_lt());
-      const float3 Tn = mul(T, xyz(cb[2 * d + 1]));
+      const float3 Tn = mul(T, xyz(rec_beta(w, s, d)));
       vput(0, e, __int_as_float(s));
       vput(1, e, __int_as_float(d + 1));
       vput(2, e, x.p.x); vput(3, e, x.p.y); vput(4, e, x.p.z);
@@ -1411,8 +1419,6 @@ __global__ void __launch_bounds__(128, 2) k_adjoint_ext(WF w, const DevScene* __
       const DevView& V = *Vp;
       const DevScene& sc = *scp;
       hot_bind(hot, scp);
-      const float4* hits = w.rec + (size_t)s * w.rec_stride + 1;
-      const float4* cb = hits + (size_t)w.D * w.R;
       if (x0.is_light) {
         // camera ray on a light: L = emit at depth 0 when lights are visible
         if (w.light_vis) {
@@ -1431,7 +1437,7 @@ __global__ void __launch_bounds__(128, 2) k_adjoint_ext(WF w, const DevScene* __
           }
         }
       } else {
-        const float3 L = suffix_radiance(cb, 0, w.D);
+        const float3 L = suffix_radiance(w, s, 0);
         if (finite3(L)) {
           has0 = true;
           Rng rng = make_rng((unsigned long long)(tile.begin + s - V.sample_off) + w.seed);
@@ -1451,8 +1457,7 @@ __global__ void __launch_bounds__(128, 2) k_adjoint_ext(WF w, const DevScene* __
           bool frontq = true;
           for (int d = 0; d < w.D; ++d) {
             const float3 adjC = mul(g, T);
-            const float3 adjB = mul(adjC, suffix_radiance(cb, d + 1, w.D));
-            const float4* rec = hits + (size_t)d * w.R;
+            const float3 adjB = mul(adjC, suffix_radiance(w, s, d + 1));
             const DevObj& ob = sc.objs[xc.obj];
             const MatPt mp = mat_point(ob, xc);
             MatAdj ma = zero_mat_adj();
@@ -1461,15 +1466,17 @@ __global__ void __launch_bounds__(128, 2) k_adjoint_ext(WF w, const DevScene* __
             float3 none;
             for (int i = 0; i < w.nL; ++i) {
               const float rx = rng.next_float(), ry = rng.next_float();
-              light_sample_adj<true>(w, sc, xc, mp.color * kInvPi, rx, ry, rec[i], adjC, ax, hot, none, &mp, &ma);
+              light_sample_adj<true>(w, sc, xc, mp.color * kInvPi, rx, ry, rec_hit(w, s, d, i), adjC, ax, hot, none, &mp,
+                                     &ma);
             }
             for (int j = 0; j < w.nB; ++j) {
               const float rx = rng.next_float(), ry = rng.next_float();
-              bsdf_sample_adj<UNB, true>(w, sc, xc, mp.color * kInvPi, rx, ry, rec[w.nL + j], adjC, ax, hot, none, &mp, &ma);
+              bsdf_sample_adj<UNB, true>(w, sc, xc, mp.color * kInvPi, rx, ry, rec_hit(w, s, d, w.nL + j), adjC, ax, hot, none,
+                                         &mp, &ma);
             }
             const float rx = rng.next_float(), ry = rng.next_float();
-            const bool next = d < w.D - 1 && continuation_adj<UNB, true>(sc, xc, mp.color * kInvPi, rx, ry, rec[w.nL + w.nB],
-                                                                         adjB, ax, nextc, nx, none, &mp, &ma);
+            const bool next = d < w.D - 1 && continuation_adj<UNB, true>(sc, xc, mp.color * kInvPi, rx, ry,
+                                                                         rec_hit(w, s, d, w.nL + w.nB), adjB, ax, nextc, nx, none, &mp, &ma);
             const float3 aorg = mat_finalize(ob, xc, mp, ma, ax);
             if (d == 0) cam.add(&V, aorg);
             else if (d == 1) ax0.p += aorg;
@@ -1490,8 +1497,8 @@ __global__ void __launch_bounds__(128, 2) k_adjoint_ext(WF w, const DevScene* __
               frontq = xc.front;
             }
             if (!next) break;
-            T = mul(T, xyz(cb[2 * d + 1]));
-            hc = rec[w.nL + w.nB];
+            T = mul(T, xyz(rec_beta(w, s, d)));
+            hc = rec_hit(w, s, d, w.nL + w.nB);
             tric = __float_as_int(hc.x);
             xc = nx;
             if (xc.is_light) break;  // the path ends on a light: nothing downstream
@@ -2060,8 +2067,7 @@ __global__ void __launch_bounds__(256) k_lens_interior(WF w, const DevScene* __r
     if (s >= tile.n) continue;
     const DevView& V = views[w.view[s]];
     if (!V.grad_lens || !V.dimage) continue;
-    const float4* rec = w.rec + (size_t)s * w.rec_stride;
-    const float4 h0 = rec[0];
+    const float4 h0 = rec_at(w, s, 0);
     const int tri0 = __float_as_int(h0.x);
     if (tri0 < 0) continue;
     const DevScene& sc = scenes[V.scene];
@@ -2071,7 +2077,7 @@ __global__ void __launch_bounds__(256) k_lens_interior(WF w, const DevScene* __r
       if (!w.light_vis) continue;
       L = light_emit<BSDF>(sc.lights[x0.light], x0);
     } else {
-      L = suffix_radiance(rec + 1 + (size_t)w.D * w.R, 0, w.D);
+      L = suffix_radiance(w, s, 0);
     }
     if (!finite3(L)) continue;
     const int pix = w.pix[s];
@@ -3750,6 +3756,7 @@ void psdr_workspace::ensure(int c, int r, int d, int nv, int rec_needed, cudaStr
   wf.q0 = q0.as<int>(); wf.q1 = q1.as<int>(); wf.qs = qs.as<int>(); wf.cnt = cnt.as<int>();
   wf.ro = ro.as<float4>(); wf.rd = rd.as<float4>(); wf.ra = ra.as<float4>(); wf.hit = hit.as<float4>();
   wf.rec = rec.as<float4>();
+  wf.rec_plane = cap;
 }
 
 namespace psdr {
@@ -3770,7 +3777,6 @@ void set_wf(WF& w, const psdr_config& cfg, int nviews, int nB_override, int ligh
   // seed s offsets every sample stream by s * 2654435761 (mod 2^32, the width of the
   // stream index): jobs of different seeds draw from disjoint stream ranges
   w.seed = cfg.seed * 2654435761ull;
-  w.rec_stride = 1 + w.D * w.R + 2 * w.D;  // primary hit, hits per depth, (C, beta) per depth
   w.trace_bps = cfg.trace_queue > 0 ? cfg.trace_queue : 8;
 }
 
@@ -3784,7 +3790,8 @@ void forward_tile(const DevScene* scenes_dev, const std::vector<DevView>& views,
   w.ortho = any_ortho(views);
   w.one_scene = job_scene(views);
   if (keep) {
-    w.rec = keep->rec + (size_t)t.begin * w.rec_stride;
+    w.rec = keep->rec + t.begin;
+    w.rec_plane = keep->plane;
     w.view = keep->view + t.begin;
     w.pix = keep->pix + t.begin;
   }
@@ -4105,7 +4112,8 @@ void backward_unit(const DevScene* scenes_dev, const std::vector<DevView>& views
     w.one_scene = job_scene(views);
     const Tile& t = u.tile;
     if (keep) {
-      w.rec = keep->rec + (size_t)t.begin * w.rec_stride;
+      w.rec = keep->rec + t.begin;
+      w.rec_plane = keep->plane;
       w.view = keep->view + t.begin;
       w.pix = keep->pix + t.begin;
     } else {

@@ -46,7 +46,7 @@ struct WF {
   float4* ra;    // aux: NEE target point + pdf / bsdf cos(theta)
   float4* hit;   // tri(bits), b1, b2, t
   float4* rec;   // replay records: 1 + D*R per path
-  int rec_stride;
+  size_t rec_plane;  // paths between consecutive records of a path (rec_at)
   int bsdf;      // host side: launch the extended kernel instances (DiffuseBsdfMaterial, environment light)
   int ortho;     // host side: an orthographic view is in the job (camera kernel instance)
   int one_scene; // the scene of every view of the job, or -1 when the views have several
@@ -75,10 +75,11 @@ struct EdgeBuf {
 enum Mode { MODE_FWD = 0, MODE_REPLAY = 1, MODE_KEEP = 2 };
 
 // Replay records of every interior path of a job kept from its forward (psdr_batch): path
-// s of the job's sample space has its record at rec + s * rec_stride and its view and
+// s of the job's sample space has its record k at rec + k * plane + s and its view and
 // pixel at view[s], pix[s].
 struct KeptRecords {
   float4* rec = nullptr;
+  size_t plane = 0;  // paths of the job
   int* view = nullptr;
   int* pix = nullptr;
 };
