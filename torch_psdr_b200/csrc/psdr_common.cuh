@@ -31,8 +31,6 @@ PSDR_HD float sqnorm(float3 a) { return dot(a, a); }
 PSDR_HD float norm(float3 a) { return sqrtf(sqnorm(a)); }
 PSDR_HD float3 normalize(float3 a) { return a * (1.0f / sqrtf(sqnorm(a))); }
 PSDR_HD float3 xyz(float4 a) { return f3(a.x, a.y, a.z); }
-PSDR_HD float sel3(float3 v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : v.z); }
-PSDR_HD float comp(float3 v, int k) { return sel3(v, k); }
 PSDR_HD bool finite3(float3 v) { return isfinite(sqnorm(v)); }
 
 constexpr float kPi = 3.14159265358979323846f;
@@ -205,24 +203,28 @@ PSDR_D int discrete_sample(const float* __restrict__ pmf, const float* __restric
 // ------------------------------------------------------------------ watertight test
 // Woop, Benthin & Wald (JCGT 2013). Every arithmetic step is an explicitly rounded
 // IEEE operation so the device result is bit-identical to the float oracle.
+//
+// The test works in coordinates permuted so that the ray's largest direction component comes
+// last. The published test also swaps the other two for a negative component, to keep the
+// winding; that only negates U, V, W and det together, exactly, so it is left out: t and the
+// barycentrics are the same bits.
 struct RayPre {
   float3 o;
-  int kx, ky, kz;
+  int kz;            // the axis that comes last; the order is (kz + 1, kz + 2, kz) mod 3
   float Sx, Sy, Sz;
 };
+PSDR_D float3 rotate_axes(float3 v, int kz) {
+  return kz == 0 ? f3(v.y, v.z, v.x) : (kz == 1 ? f3(v.z, v.x, v.y) : v);
+}
 PSDR_D RayPre ray_pre(float3 o, float3 d) {
   RayPre r;
   r.o = o;
   float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
-  int kz = (ax > ay) ? (ax > az ? 0 : 2) : (ay > az ? 1 : 2);
-  int kx = kz + 1 == 3 ? 0 : kz + 1;
-  int ky = kx + 1 == 3 ? 0 : kx + 1;
-  float dz = sel3(d, kz);
-  if (dz < 0.0f) { int t = kx; kx = ky; ky = t; }
-  r.kx = kx; r.ky = ky; r.kz = kz;
-  r.Sx = __fdiv_rn(sel3(d, kx), dz);
-  r.Sy = __fdiv_rn(sel3(d, ky), dz);
-  r.Sz = __fdiv_rn(1.0f, dz);
+  r.kz = (ax > ay) ? (ax > az ? 0 : 2) : (ay > az ? 1 : 2);
+  const float3 q = rotate_axes(d, r.kz);
+  r.Sx = __fdiv_rn(q.x, q.z);
+  r.Sy = __fdiv_rn(q.y, q.z);
+  r.Sz = __fdiv_rn(1.0f, q.z);
   return r;
 }
 PSDR_D bool tri_test(const RayPre& r, float3 p0, float3 p1, float3 p2, float tmin, float tmax, float& t,
@@ -230,10 +232,11 @@ PSDR_D bool tri_test(const RayPre& r, float3 p0, float3 p1, float3 p2, float tmi
   float3 A = f3(__fsub_rn(p0.x, r.o.x), __fsub_rn(p0.y, r.o.y), __fsub_rn(p0.z, r.o.z));
   float3 B = f3(__fsub_rn(p1.x, r.o.x), __fsub_rn(p1.y, r.o.y), __fsub_rn(p1.z, r.o.z));
   float3 C = f3(__fsub_rn(p2.x, r.o.x), __fsub_rn(p2.y, r.o.y), __fsub_rn(p2.z, r.o.z));
-  float Akz = sel3(A, r.kz), Bkz = sel3(B, r.kz), Ckz = sel3(C, r.kz);
-  float Ax = __fsub_rn(sel3(A, r.kx), __fmul_rn(r.Sx, Akz)), Ay = __fsub_rn(sel3(A, r.ky), __fmul_rn(r.Sy, Akz));
-  float Bx = __fsub_rn(sel3(B, r.kx), __fmul_rn(r.Sx, Bkz)), By = __fsub_rn(sel3(B, r.ky), __fmul_rn(r.Sy, Bkz));
-  float Cx = __fsub_rn(sel3(C, r.kx), __fmul_rn(r.Sx, Ckz)), Cy = __fsub_rn(sel3(C, r.ky), __fmul_rn(r.Sy, Ckz));
+  A = rotate_axes(A, r.kz); B = rotate_axes(B, r.kz); C = rotate_axes(C, r.kz);
+  float Akz = A.z, Bkz = B.z, Ckz = C.z;
+  float Ax = __fsub_rn(A.x, __fmul_rn(r.Sx, Akz)), Ay = __fsub_rn(A.y, __fmul_rn(r.Sy, Akz));
+  float Bx = __fsub_rn(B.x, __fmul_rn(r.Sx, Bkz)), By = __fsub_rn(B.y, __fmul_rn(r.Sy, Bkz));
+  float Cx = __fsub_rn(C.x, __fmul_rn(r.Sx, Ckz)), Cy = __fsub_rn(C.y, __fmul_rn(r.Sy, Ckz));
   float U = __fsub_rn(__fmul_rn(Cx, By), __fmul_rn(Cy, Bx));
   float V = __fsub_rn(__fmul_rn(Ax, Cy), __fmul_rn(Ay, Cx));
   float W = __fsub_rn(__fmul_rn(Bx, Ay), __fmul_rn(By, Ax));
@@ -288,7 +291,9 @@ struct HitRec {
   float b1, b2, t;
 };
 
-PSDR_D float safe_inv(float d) { return 1.0f / (fabsf(d) > 1e-30f ? d : copysignf(1e-30f, d)); }
+// Reciprocal direction component for the box tests alone: the fast division's 2 ulp are a fifth of
+// the slack those have.
+PSDR_D float safe_inv(float d) { return __fdividef(1.0f, fabsf(d) > 1e-30f ? d : copysignf(1e-30f, d)); }
 
 // Closest hit in (tmin, tmax], ties broken by the smaller triangle id. Node boxes are
 // expanded at build time and the cull bound is relaxed by 1e-5 relative so that no

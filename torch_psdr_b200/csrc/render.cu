@@ -282,19 +282,19 @@ struct TraceShared {
 struct TraceMem {
   TraceShared* sh;
   int lane;
-  int axes;  // kx | ky << 2 | kz << 4
+  int kz;
   int deep[kStack - kShort];
   PSDR_D void set_ray(const RayPre& r) {
     sh->ray[0][lane] = r.o.x; sh->ray[1][lane] = r.o.y; sh->ray[2][lane] = r.o.z;
     sh->ray[3][lane] = r.Sx; sh->ray[4][lane] = r.Sy; sh->ray[5][lane] = r.Sz;
-    axes = r.kx | r.ky << 2 | r.kz << 4;
+    kz = r.kz;
     bary(0.f, 0.f);
   }
   PSDR_D RayPre ray() const {
     RayPre r;
     r.o = f3(sh->ray[0][lane], sh->ray[1][lane], sh->ray[2][lane]);
     r.Sx = sh->ray[3][lane]; r.Sy = sh->ray[4][lane]; r.Sz = sh->ray[5][lane];
-    r.kx = axes & 3; r.ky = (axes >> 2) & 3; r.kz = axes >> 4;
+    r.kz = kz;
     return r;
   }
   PSDR_D void bary(float u, float v) { sh->ray[6][lane] = u; sh->ray[7][lane] = v; }
