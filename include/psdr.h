@@ -226,6 +226,12 @@ PSDR_API psdr_status psdr_scene_info(psdr_scene* scene, int64_t* info6);
  * p0, p1, out_direction, n_left, n_right, length) into DEVICE buffers of capacity cap. */
 PSDR_API psdr_status psdr_scene_edges(psdr_scene* scene, int32_t* v01, float* geo, int64_t cap, int64_t* n_out, void* stream);
 
+/* Smallest and largest entry of n device buffers of int32 (buffers[i] holds counts[i] entries)
+ * to the host array out (2 n; an empty buffer gives INT32_MAX, INT32_MIN): the check of
+ * several index buffers with one kernel and one host read. Synchronises `stream`. */
+PSDR_API psdr_status psdr_index_bounds(const int32_t* const* buffers, const int64_t* counts, int32_t n, int32_t* out,
+                                       void* stream);
+
 /* Closest hit for n rays (device, 8 floats per ray: ox oy oz tmin dx dy dz tmax).
  * Outputs the global triangle id (-1 on miss), OptiX-convention barycentrics
  * (weights of p1, p2) and t. brute_force 1 tests every triangle (the KAT path); 2 runs

@@ -85,3 +85,20 @@ def test_kept_tree_renders_as_a_new_one(cuda):
         scene.update(refit=True)
         fresh, _ = to_torch_scene(spec)
         assert torch.equal(integ.renderC(scene)[0], integ.renderC(fresh)[0])
+
+
+def test_index_bounds(cuda):
+    """psdr_index_bounds over more buffers than one launch takes, empty ones and both ends of
+    the 32-bit range among them."""
+    rng = np.random.default_rng(0)
+    bufs = [rng.integers(-2 ** 31, 2 ** 31, size=n, dtype=np.int64).astype(np.int32)
+            for n in (1, 31, 257, 0, 100000) + (3,) * 35]
+    bufs.append(np.array([2 ** 31 - 1, -2 ** 31, 0], np.int32))
+    dev = [torch.tensor(b, device="cuda") for b in bufs]
+    n = len(bufs)
+    out = (C.c_int32 * (2 * n))()
+    L.check(L.load().psdr_index_bounds((C.c_void_p * n)(*[t.data_ptr() for t in dev]),
+                                       (C.c_int64 * n)(*[b.size for b in bufs]), n, out, _stream()), "bounds")
+    for i, b in enumerate(bufs):
+        want = (b.min(), b.max()) if b.size else (2 ** 31 - 1, -2 ** 31)
+        assert (out[2 * i], out[2 * i + 1]) == want, i

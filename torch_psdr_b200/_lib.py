@@ -87,6 +87,7 @@ SIGNATURES = {
     "psdr_scene_set_leaf_size": ([P, C.c_int32, P], C.c_int),
     "psdr_scene_info": ([P, C.POINTER(C.c_int64)], C.c_int),
     "psdr_scene_edges": ([P, P, P, C.c_int64, C.POINTER(C.c_int64), P], C.c_int),
+    "psdr_index_bounds": ([C.POINTER(P), C.POINTER(C.c_int64), C.c_int32, C.POINTER(C.c_int32), P], C.c_int),
     "psdr_intersect": ([P, P, C.c_int64, P, P, P, C.c_int32, P], C.c_int),
     "psdr_camera_lens_jacobian": ([P, C.POINTER(C.c_double), C.POINTER(C.c_double)], C.c_int),
     "psdr_workspace_create": ([C.POINTER(P)], C.c_int),

@@ -13,6 +13,7 @@ import json
 import os
 from typing import List, Optional, Union
 
+import numpy as np
 import torch
 from torch import Tensor
 
@@ -25,7 +26,7 @@ def _dev_tensor(t: Tensor, dtype) -> Tensor:
         t = torch.as_tensor(t)
     if not t.is_cuda:
         raise ValueError("torch_psdr_b200 renders on the GPU: tensors must be CUDA tensors")
-    return t.detach().to(dtype).contiguous().clone()
+    return t.detach().to(dtype=dtype, copy=True, memory_format=torch.contiguous_format)
 
 
 def check_indices(idx: Tensor, n: int, what: str) -> None:
@@ -40,13 +41,37 @@ def check_indices(idx: Tensor, n: int, what: str) -> None:
         raise ValueError(f"{what} must lie in [0, {n}): found values in [{lo}, {hi}]")
 
 
+def _check_index_buffers(jobs) -> None:
+    """check_indices for the (int32 CUDA tensor, bound, name) triples of one object, with one
+    kernel and one host read for all of them."""
+    jobs = [j for j in jobs if j[0].numel()]
+    n = len(jobs)
+    if n == 0:
+        return
+    ptrs = (C.c_void_p * n)(*[t.data_ptr() for t, _, _ in jobs])
+    counts = (C.c_int64 * n)(*[t.numel() for t, _, _ in jobs])
+    out = (C.c_int32 * (2 * n))()
+    L.check(L.load().psdr_index_bounds(ptrs, counts, n, out, _stream()), "psdr_index_bounds")
+    for i, (_, bound, what) in enumerate(jobs):
+        if out[2 * i] < 0 or out[2 * i + 1] >= bound:
+            raise ValueError(f"{what} must lie in [0, {bound}): found values in [{out[2 * i]}, {out[2 * i + 1]}]")
+
+
 def _stream():
     return C.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
-def _host3(t: Tensor):
-    v = t.detach().reshape(-1).float().cpu().tolist()
-    return (C.c_float * 3)(*v[:3])
+def _host_lists(tensors) -> list:
+    """The tensors' values as lists of floats, with one host read when they are float32 tensors
+    on one GPU (each read waits for the stream)."""
+    flat = [t.detach().reshape(-1) for t in tensors]
+    if len(flat) > 1 and all(f.is_cuda and f.dtype == torch.float32 and f.device == flat[0].device for f in flat):
+        values, out = torch.cat(flat).tolist(), []
+        for f in flat:
+            out.append(values[:f.numel()])
+            values = values[f.numel():]
+        return out
+    return [f.float().cpu().tolist() for f in flat]
 
 
 class VarContex:
@@ -71,6 +96,23 @@ class VarContex:
 class BaseCamera(VarContex):
     """Base class of PerspectiveCamera and OrthographicCamera (torch_psdr.py:106-110)."""
 
+    def _desc(self):
+        return _camera_descs([self])[0]
+
+
+def _camera_descs(cams):
+    """Descriptors of the cameras (their parameters are read from the GPU in one go)."""
+    values = iter(_host_lists([t for c in cams for t in (c.look_from, c.look_at, c.up, c.vfov)]))
+    out = (L.CameraDesc * len(cams))()
+    for d, c in zip(out, cams):
+        d.type = L.CAM_ORTHOGRAPHIC if isinstance(c, OrthographicCamera) else L.CAM_PERSPECTIVE
+        d.look_from = (C.c_float * 3)(*next(values))
+        d.look_at = (C.c_float * 3)(*next(values))
+        d.up = (C.c_float * 3)(*next(values))
+        d.fov = next(values)[0]
+        d.height, d.width = c.height, c.width
+    return out
+
 
 class PerspectiveCamera(BaseCamera):
     def __init__(self, look_from: Tensor, look_at: Tensor, up: Tensor, vfov: Tensor, height: int, width: int):
@@ -91,16 +133,6 @@ class PerspectiveCamera(BaseCamera):
             self.append_variable(t)
         self.height = int(height)
         self.width = int(width)
-
-    def _desc(self):
-        d = L.CameraDesc()
-        d.type = L.CAM_PERSPECTIVE
-        d.look_from = _host3(self.look_from)
-        d.look_at = _host3(self.look_at)
-        d.up = _host3(self.up)
-        d.fov = float(self.vfov.detach().reshape(-1)[0].item())
-        d.height, d.width = self.height, self.width
-        return d
 
 
 Camera = PerspectiveCamera  # example/optimize_texture.py:76 uses dr.Camera
@@ -123,16 +155,6 @@ class OrthographicCamera(BaseCamera):
             self.append_variable(t)
         self.height = int(height)
         self.width = int(width)
-
-    def _desc(self):
-        d = L.CameraDesc()
-        d.type = L.CAM_ORTHOGRAPHIC
-        d.look_from = _host3(self.look_from)
-        d.look_at = _host3(self.look_at)
-        d.up = _host3(self.up)
-        d.fov = float(self.view_width.detach().reshape(-1)[0].item())
-        d.height, d.width = self.height, self.width
-        return d
 
 
 class Texture(VarContex):
@@ -239,12 +261,11 @@ class Mesh(VarContex):
         self.vertices = vertices
         self.v = _dev_tensor(vertices, torch.float32)
         self.f = _dev_tensor(face_indices, torch.int32)
-        check_indices(self.f, self.v.shape[0], "face_indices")
         no_uvs = uvs is None or uv_indices is None
         self.uv = None if no_uvs else _dev_tensor(uvs, torch.float32)
         self.uvi = None if no_uvs else _dev_tensor(uv_indices, torch.int32)
-        if self.uvi is not None:
-            check_indices(self.uvi, self.uv.shape[0], "uv_indices")
+        _check_index_buffers([(self.f, self.v.shape[0], "face_indices")] +
+                             ([] if no_uvs else [(self.uvi, self.uv.shape[0], "uv_indices")]))
         self.material = material
         self.append_variable(vertices)
         self.merge_variables(material.get_variables())
@@ -289,15 +310,15 @@ class AreaLight(Light):
         self.vertices, self.emit = vertices, emit
         self.v = _dev_tensor(vertices, torch.float32)
         self.f = _dev_tensor(face_indices, torch.int32)
-        check_indices(self.f, self.v.shape[0], "face_indices")
+        _check_index_buffers([(self.f, self.v.shape[0], "face_indices")])
         self.append_variable(vertices)
         self.append_variable(emit)
 
-    def _desc(self):
+    def _desc(self, emit=None):
         d = L.AreaLightDesc()
         d.vertices, d.num_vertices = self.v.data_ptr(), int(self.v.shape[0])
         d.faces, d.num_faces = self.f.data_ptr(), int(self.f.shape[0])
-        d.emit = _host3(self.emit)
+        d.emit = (C.c_float * 3)(*(emit if emit is not None else _host_lists([self.emit])[0]))
         return d
 
 
@@ -313,7 +334,7 @@ class EnvLight(Light):
         self.vertices = self.v = self.emit = None
         self.params, self.params_data = cube_map.tensor, cube_map.data
 
-    def _desc(self, box):
+    def _desc(self, _, box):
         d = L.AreaLightDesc()
         d.type = L.LIGHT_ENV
         d.cube_map = self.cube_map._desc()
@@ -334,10 +355,10 @@ class SH9Light(Light):
         self.params = sh9_coeff
         self.params_data = torch.zeros((9, 3), dtype=torch.float32, device="cuda")
 
-    def _desc(self, box):
+    def _desc(self, sh9, box):
         d = L.AreaLightDesc()
         d.type = L.LIGHT_SH9
-        d.sh9 = (C.c_float * 27)(*self.sh9_coeff.detach().reshape(-1).cpu().tolist())
+        d.sh9 = (C.c_float * 27)(*sh9)
         d.box_min, d.box_max = (C.c_float * 3)(*map(float, box[0])), (C.c_float * 3)(*map(float, box[1]))
         return d
 
@@ -358,14 +379,24 @@ class Scene(VarContex):
         env = [lt for lt in lights if _is_env(lt)]
         assert len(env) <= 1, "only support no more than one env_light"
         self.lights = [lt for lt in lights if not _is_env(lt)] + env
+        # light radiances and coefficients, and for an environment light the camera positions and
+        # the meshes' boxes (minima and maxima taken on the GPU), in one host read
+        par = [lt.sh9_coeff if isinstance(lt, SH9Light) else lt.emit for lt in self.lights
+               if not isinstance(lt, EnvLight)]
+        ext = []
+        if env:
+            ext = [c.look_from for c in self.cameras] + [e for m in self.meshes for e in (m.v.amin(0), m.v.amax(0))]
+        values = _host_lists(par + ext)
         box = None
         if env:
-            box = synth.env_box([c.look_from.detach().cpu().numpy() for c in self.cameras],
-                                [m.v.detach().cpu().numpy() for m in self.meshes])
+            pts = np.array(values[len(par):], np.float32)
+            box = synth.env_box(pts[:len(self.cameras)], [pts[len(self.cameras):]])
+        values = iter(values[:len(par)])
         lib = L.load()
         md = (L.MeshDesc * max(1, len(self.meshes)))(*[m._desc() for m in self.meshes])
-        ld = (L.AreaLightDesc * max(1, len(self.lights)))(*[lt._desc(box) if _is_env(lt) else lt._desc()
-                                                            for lt in self.lights])
+        ld = (L.AreaLightDesc * max(1, len(self.lights)))(*[
+            lt._desc(None, box) if isinstance(lt, EnvLight) else
+            lt._desc(next(values), box) if isinstance(lt, SH9Light) else lt._desc(next(values)) for lt in self.lights])
         desc = L.SceneDesc(md, len(self.meshes), ld, len(self.lights))
         handle = C.c_void_p()
         L.check(lib.psdr_scene_create(C.byref(desc), _stream(), C.byref(handle)), "psdr_scene_create")
@@ -398,7 +429,7 @@ class Scene(VarContex):
             L.check(self._lib.psdr_scene_update(self._handle, _stream()), "psdr_scene_update")
 
     def _camera_descs(self):
-        return (L.CameraDesc * len(self.cameras))(*[c._desc() for c in self.cameras])
+        return _camera_descs(self.cameras)
 
     def __del__(self):
         h = getattr(self, "_handle", None)
@@ -431,17 +462,17 @@ class _RenderD(torch.autograd.Function):
         return (None, None) + tuple(out)
 
 
-def _grad_buf(param, internal):
-    """Zeroed gradient buffer shaped like `internal`, or None when `param` does not
-    require grad."""
+def _grad_buf(param, internal, new=torch.zeros_like):
+    """Gradient buffer shaped like `internal` (zeroed unless `new` says otherwise), or None
+    when `param` does not require grad."""
     if isinstance(param, Tensor) and param.requires_grad:
-        return torch.zeros_like(internal)
+        return new(internal)
     return None
 
 
-def _tex_grad(tex):
+def _tex_grad(tex, new=torch.zeros_like):
     """Gradient buffer of an optional Texture (None when absent or not requiring grad)."""
-    return None if tex is None else _grad_buf(tex.tensor, tex.data)
+    return None if tex is None else _grad_buf(tex.tensor, tex.data, new)
 
 
 def _ptrs(bufs):
@@ -653,14 +684,16 @@ class PathIntegrator:
         nm, nl = len(scene.meshes), len(scene.lights)
         # vertex gradients only for the meshes/lights whose vertices require grad (the
         # library then skips the others' scatters)
-        vert_g = [_grad_buf(m.vertices, m.v) for m in scene.meshes] + [_grad_buf(lt.vertices, lt.v)
-                                                                        for lt in scene.lights]
-        tex_g = [_grad_buf(m.material.texture.tensor, m.material.texture.data) for m in scene.meshes]
-        rough_g = [_tex_grad(m.material.roughness) for m in scene.meshes]
-        nrm_g = [_tex_grad(m.material.normal) for m in scene.meshes]
-        emit_g = [torch.zeros(3, dtype=torch.float32, device=dev) for _ in scene.lights]
-        light_g = [_grad_buf(lt.params, lt.params_data) if _is_env(lt) else None for lt in scene.lights]
-        cam_g = [torch.zeros(3, dtype=torch.float32, device=dev) for _ in scene.cameras]
+        # (the buffers are written in full: none needs to be cleared first)
+        new = torch.empty_like
+        vert_g = [_grad_buf(m.vertices, m.v, new) for m in scene.meshes] + [_grad_buf(lt.vertices, lt.v, new)
+                                                                             for lt in scene.lights]
+        tex_g = [_grad_buf(m.material.texture.tensor, m.material.texture.data, new) for m in scene.meshes]
+        rough_g = [_tex_grad(m.material.roughness, new) for m in scene.meshes]
+        nrm_g = [_tex_grad(m.material.normal, new) for m in scene.meshes]
+        emit_g = list(torch.empty((nl, 3), dtype=torch.float32, device=dev))
+        light_g = [_grad_buf(lt.params, lt.params_data, new) if _is_env(lt) else None for lt in scene.lights]
+        cam_g = list(torch.empty((len(scene.cameras), 3), dtype=torch.float32, device=dev))
         unb = self.cfg.estimator == L.EST_UNBIASED
         lens_g = [_lens_buf(c, unb) for c in scene.cameras]
         P = C.c_void_p
@@ -697,7 +730,7 @@ class PathIntegrator:
                 add(lt.params, light_g[j])
         for k, c in enumerate(scene.cameras):
             _add_camera_grads(add, c, cam_g[k], lens_g[k])
-        return [acc.get(id(t), torch.zeros_like(t)) for t in torch_vars]
+        return [acc[id(t)] if id(t) in acc else torch.zeros_like(t) for t in torch_vars]
 
     def renderC(self, scene: Scene) -> List[Tensor]:
         """Plain render (path_integrator.cc:408-410): one (H, W, 3) image per camera."""
@@ -779,7 +812,7 @@ class BatchRender:
         self._keep += [cp, lp_cam]
         tgt = (L.GradTargets * len(targets))(*targets)
         sh = (P * len(self.scenes))(*[s.handle for s in self.scenes])
-        cd = (L.CameraDesc * len(cams))(*[c._desc() for c in cams])
+        cd = _camera_descs(cams)
         csc = (C.c_int32 * len(cams))(*cam_scene)
         ip = (P * len(cams))(*[t.data_ptr() for t in self.images])
         dp = (P * len(cams))(*[t.data_ptr() for t in self.d_images]) if differentiable else None
@@ -846,7 +879,7 @@ class BatchRender:
             for c in sc.cameras:
                 _add_camera_grads(add, c, self.cam_grads[k], self.lens_grads[k])
                 k += 1
-        return [acc.get(id(t), torch.zeros_like(t)) for t in torch_vars]
+        return [acc[id(t)] if id(t) in acc else torch.zeros_like(t) for t in torch_vars]
 
     def __del__(self):
         h = getattr(self, "_handle", None)

@@ -127,23 +127,27 @@ long long light_param_count(const psdr_scene* s, int l) {
 }
 
 
-// Min and max of n indices into out[0] / out[1] (initialised to INT_MAX / INT_MIN):
-// grid-stride loads, warp reduction, one atomic pair per warp.
-__global__ void k_index_range(const int* __restrict__ idx, long long n, int* __restrict__ out) {
-  int lo = INT_MAX, hi = INT_MIN;
+// Extremes of several index buffers (blockIdx.y), as maxima of order-preserving unsigned images
+// (of the complement for the minimum), so that both start from zeroed memory.
+constexpr int kIndexJobs = 32;
+struct IndexJobs {
+  const int* p[kIndexJobs];
+  long long n[kIndexJobs];
+};
+__global__ void k_index_bounds(IndexJobs jobs, unsigned* __restrict__ out) {
+  const int* __restrict__ p = jobs.p[blockIdx.y];
+  const long long n = jobs.n[blockIdx.y];
+  unsigned lo = 0u, hi = 0u;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const int v = __ldg(idx + i);
-    lo = min(lo, v);
-    hi = max(hi, v);
+    const unsigned u = (unsigned)p[i] ^ 0x80000000u;
+    lo = max(lo, ~u);
+    hi = max(hi, u);
   }
-#pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-    hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-  }
-  if ((threadIdx.x & 31) == 0) {
-    atomicMin(out, lo);
-    atomicMax(out + 1, hi);
+  lo = __reduce_max_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if ((threadIdx.x & 31) == 0 && (lo | hi)) {
+    atomicMax(out + 2 * blockIdx.y, lo);
+    atomicMax(out + 2 * blockIdx.y + 1, hi);
   }
 }
 
@@ -167,6 +171,36 @@ using namespace psdr;
     return PSDR_ERR_CUDA;                                                \
   }                                                                      \
   return PSDR_OK;
+
+// Smallest and largest entry of each of n device buffers: one kernel (per 32 buffers) and one
+// host read.
+static void index_bounds(const int* const* ptr, const long long* cnt, int n, int* out, cudaStream_t st) {
+  if (n == 0) return;
+  DBuf res;
+  res.alloc(sizeof(unsigned) * 2 * n, st);
+  PSDR_CUDA(cudaMemsetAsync(res.p, 0, sizeof(unsigned) * 2 * n, st));
+  for (int j0 = 0; j0 < n; j0 += kIndexJobs) {
+    IndexJobs jobs{};
+    const int m = std::min(kIndexJobs, n - j0);
+    long long most = 0;
+    for (int j = 0; j < m; ++j) {
+      jobs.p[j] = ptr[j0 + j];
+      jobs.n[j] = cnt[j0 + j];
+      most = std::max(most, cnt[j0 + j]);
+    }
+    if (most == 0) continue;
+    const dim3 grid((unsigned)std::min<long long>((most + 255) / 256, 148LL * 8), m);
+    k_index_bounds<<<grid, 256, 0, st>>>(jobs, res.as<unsigned>() + 2 * j0);
+  }
+  PSDR_CUDA(cudaGetLastError());
+  std::vector<unsigned> h(2 * n);
+  PSDR_CUDA(cudaMemcpyAsync(h.data(), res.p, sizeof(unsigned) * 2 * n, cudaMemcpyDeviceToHost, st));
+  PSDR_CUDA(cudaStreamSynchronize(st));
+  for (int j = 0; j < n; ++j) {
+    out[2 * j] = (int)(~h[2 * j] ^ 0x80000000u);
+    out[2 * j + 1] = (int)(h[2 * j + 1] ^ 0x80000000u);
+  }
+}
 
 // Every face index of a mesh or area light in [0, num_vertices), every uv index in
 // [0, num_uvs): one min/max reduction per index buffer and one host read. Throws
@@ -195,22 +229,12 @@ static void check_index_ranges(const psdr_scene_desc* desc, void* stream) {
     PSDR_CHECK(L.num_faces == 0 || L.faces != nullptr, "null face buffer");
     jobs.push_back({L.faces, 3LL * L.num_faces, L.num_vertices, "light " + std::to_string(l) + " face"});
   }
-  cudaStream_t st = (cudaStream_t)stream;
   const int k = (int)jobs.size();
-  if (k == 0) return;
-  DBuf range;
-  range.alloc(sizeof(int) * 2 * k, st);
+  std::vector<const int*> ptr(k);
+  std::vector<long long> cnt(k);
   std::vector<int> h(2 * k);
-  for (int j = 0; j < k; ++j) { h[2 * j] = INT_MAX; h[2 * j + 1] = INT_MIN; }
-  PSDR_CUDA(cudaMemcpyAsync(range.p, h.data(), sizeof(int) * 2 * k, cudaMemcpyHostToDevice, st));
-  for (int j = 0; j < k; ++j) {
-    if (jobs[j].n == 0) continue;
-    const int blocks = (int)std::min<long long>((jobs[j].n + 255) / 256, 148LL * 8);
-    k_index_range<<<blocks, 256, 0, st>>>(jobs[j].p, jobs[j].n, range.as<int>() + 2 * j);
-  }
-  PSDR_CUDA(cudaGetLastError());
-  PSDR_CUDA(cudaMemcpyAsync(h.data(), range.p, sizeof(int) * 2 * k, cudaMemcpyDeviceToHost, st));
-  PSDR_CUDA(cudaStreamSynchronize(st));
+  for (int j = 0; j < k; ++j) { ptr[j] = jobs[j].p; cnt[j] = jobs[j].n; }
+  index_bounds(ptr.data(), cnt.data(), k, h.data(), (cudaStream_t)stream);
   for (int j = 0; j < k; ++j) {
     if (jobs[j].n == 0) continue;
     PSDR_CHECK(h[2 * j] >= 0 && h[2 * j + 1] < jobs[j].bound,
@@ -385,14 +409,11 @@ psdr_status psdr_scene_create(const psdr_scene_desc* desc, void* stream, psdr_sc
     s->dev.ltri_base = nl > 0 ? s->obj_tri_off[nm] : 0;
     // the build gathers vertices and uvs through the index buffers: check them first
     check_index_ranges(desc, stream);
+    s->grad_texels = texoff;
     psdr_scene_alloc(s);
     // fp64 gradient accumulators live with the scene
     cudaStream_t st = s->stream;
-    s->g_verts.alloc(sizeof(GradAcc) * 3 * s->nvert, st);
-    s->g_tex.alloc(sizeof(GradAcc) * std::max<size_t>(1, texoff), st);
-    s->g_emit.alloc(sizeof(GradAcc) * 3 * std::max(1, nl), st);
     s->dev.grad_verts = s->g_verts.as<GradAcc>();
-    s->vmask.alloc(std::max<size_t>(1, s->nvert), st);
     PSDR_CUDA(cudaMemsetAsync(s->vmask.p, 1, std::max<size_t>(1, s->nvert), st));
     s->dev.vmask = s->vmask.as<unsigned char>();
     for (int o = 0; o < nm; ++o) {
@@ -600,6 +621,20 @@ psdr_status psdr_autotune(psdr_scene* scene, psdr_workspace* ws, const psdr_came
   cfg->trace_queue = bq;
   if (best_leaf) *best_leaf = bl;
   if (best_ms) *best_ms = best;
+  API_END
+}
+
+psdr_status psdr_index_bounds(const int32_t* const* buffers, const int64_t* counts, int32_t n, int32_t* out,
+                              void* stream) {
+  API_BEGIN
+  PSDR_CHECK(n >= 0, "negative count");
+  PSDR_CHECK(n == 0 || (buffers != nullptr && counts != nullptr && out != nullptr), "null argument");
+  std::vector<long long> cnt(n);
+  for (int i = 0; i < n; ++i) {
+    PSDR_CHECK(counts[i] >= 0 && (counts[i] == 0 || buffers[i] != nullptr), "null or negative buffer");
+    cnt[i] = counts[i];
+  }
+  index_bounds(buffers, cnt.data(), n, out, (cudaStream_t)stream);
   API_END
 }
 

@@ -28,26 +28,45 @@ struct Error {
 #define PSDR_CHECK(cond, msg) \
   do { if (!(cond)) throw ::psdr::Error{PSDR_ERR_INVALID_ARG, msg}; } while (0)
 
+// The library's stream-ordered memory pool of one device. It keeps up to kPoolKeep bytes of freed
+// memory while any of the library's allocations is alive (a program that makes a new scene per
+// step would otherwise map its memory anew each time: 7.8 ms for 1.31 M triangles, 0.5 ms from
+// kept memory) and gives everything back when the last one is freed.
+struct DevicePool;
+constexpr unsigned long long kPoolKeep = 2ull << 30;
+DevicePool* pool_alloc(void** p, size_t bytes, cudaStream_t st);  // on the current device
+void pool_free(DevicePool* pool, void* p, cudaStream_t st);
+
 // Device allocation owned by the library (stream-ordered allocator).
 struct DBuf {
   void* p = nullptr;
   size_t bytes = 0;
   cudaStream_t st = nullptr;
+  bool view = false;  // a part of another allocation (place)
+  DevicePool* pool = nullptr;
   DBuf() = default;
   DBuf(const DBuf&) = delete;
   DBuf& operator=(const DBuf&) = delete;
   ~DBuf() { release(); }
   void release() {
-    if (p) cudaFreeAsync(p, st);
+    if (p && !view) pool_free(pool, p, st);
     p = nullptr;
     bytes = 0;
+    view = false;
+  }
+  void place(void* q, size_t n, cudaStream_t s) {
+    release();
+    p = q;
+    bytes = n;
+    st = s;
+    view = true;
   }
   void alloc(size_t n, cudaStream_t s) {
     if (n <= bytes && p) return;
     release();
     st = s;
     size_t nb = n ? n : 16;
-    PSDR_CUDA(cudaMallocAsync(&p, nb, s));
+    pool = pool_alloc(&p, nb, s);
     bytes = nb;
   }
   template <class T> T* as() const { return reinterpret_cast<T*>(p); }
@@ -66,6 +85,7 @@ void inclusive_scan_widen(const float* in, const int* n_dev, double* out, int n,
 struct SortTmp {
   DBuf keys2, vals2, hist;
 };
+size_t sort_hist_ints(int n, int bits);  // ints of SortTmp::hist for n pairs
 // Sorted pairs: in the caller's arrays or in the temporary ones, whichever the last pass wrote.
 struct SortedKeys {
   uint64_t* k64 = nullptr;  // 64-bit keys, or
@@ -103,7 +123,9 @@ struct psdr_scene {
   std::vector<psdr::DevObj> h_objs;
   std::vector<psdr::DevLight> h_lights;
   std::vector<psdr::DevSrc> h_srcs;
-  // device storage
+  // device storage: one allocation, the buffers below are parts of it
+  psdr::DBuf slab;
+  size_t grad_texels = 0;  // entries of g_tex
   psdr::DBuf verts, tri, tri_v, objs, srcs, lights_buf, light_pmf, light_cmf, ltri_pmf, ltri_cmf;
   psdr::DBuf n_edges, edge, edge_v, edge_f, edge_pmf, edge_cmf;
   psdr::DBuf nodes, leaf, err;

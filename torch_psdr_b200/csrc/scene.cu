@@ -13,6 +13,10 @@
 //    parent and leaves of up to `leaf_size` triangles.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
+#include <mutex>
+#include <utility>
+#include <vector>
 
 #include "psdr_internal.h"
 
@@ -658,6 +662,68 @@ inline int nblk(int64_t n, int t = 256) { return (int)std::max<int64_t>(1, (n + 
 
 }  // namespace
 
+struct DevicePool {
+  std::mutex m;
+  cudaMemPool_t pool = nullptr;
+  long long live = 0;
+};
+
+static DevicePool* device_pool() {
+  constexpr int kMaxDevices = 64;
+  static DevicePool pools[kMaxDevices];
+  int dev = 0;
+  PSDR_CUDA(cudaGetDevice(&dev));
+  PSDR_CHECK(dev >= 0 && dev < kMaxDevices, "device index out of range");
+  DevicePool& P = pools[dev];
+  std::lock_guard<std::mutex> lock(P.m);
+  if (!P.pool) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    PSDR_CUDA(cudaMemPoolCreate(&P.pool, &props));
+    unsigned long long keep = kPoolKeep;
+    PSDR_CUDA(cudaMemPoolSetAttribute(P.pool, cudaMemPoolAttrReleaseThreshold, &keep));
+  }
+  return &P;
+}
+
+DevicePool* pool_alloc(void** p, size_t bytes, cudaStream_t st) {
+  DevicePool* P = device_pool();
+  {
+    std::lock_guard<std::mutex> lock(P->m);
+    ++P->live;
+  }
+  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, P->pool, st);
+  if (e == cudaErrorMemoryAllocation) {
+    // what the pool keeps may be what is missing
+    cudaGetLastError();
+    cudaMemPoolTrimTo(P->pool, 0);
+    e = cudaMallocFromPoolAsync(p, bytes, P->pool, st);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    *p = nullptr;
+    std::lock_guard<std::mutex> lock(P->m);
+    --P->live;
+    PSDR_CUDA(e);
+  }
+  return P;
+}
+
+void pool_free(DevicePool* P, void* p, cudaStream_t st) {
+  cudaFreeAsync(p, st);
+  bool last;
+  {
+    std::lock_guard<std::mutex> lock(P->m);
+    last = --P->live == 0;
+  }
+  if (last) {
+    cudaStreamSynchronize(st);
+    cudaMemPoolTrimTo(P->pool, 0);
+  }
+}
+
 int num_sms() {
   static int n = 0;
   if (!n) {
@@ -667,6 +733,13 @@ int num_sms() {
     if (n <= 0) n = 148;
   }
   return n;
+}
+
+// Bits of a vertex id in the half-edge keys.
+static int vertex_bits(const psdr_scene* s) {
+  int b = 1;
+  while ((1ll << b) < (long long)s->nvert) ++b;
+  return b;
 }
 
 // Builds everything that depends on vertex positions (records, edges, CDFs, BVH) on
@@ -689,8 +762,7 @@ static int build_records_and_edges(psdr_scene* s, cudaStream_t st) {
   // triangles) has no edges (scene.cc:59-62 takes them from the other meshes only)
   const int n_edge_tri = s->env_light >= 0 ? s->obj_tri_off[s->meshes.size() + s->env_light] : s->ntri;
   const int nh = 3 * n_edge_tri;
-  int vbits = 1;
-  while ((1ll << vbits) < (long long)s->nvert) ++vbits;
+  const int vbits = vertex_bits(s);
   uint32_t* vals = s->vals.as<uint32_t>();
   const int gh = nblk(std::max(1, nh));
   SortedKeys he;
@@ -809,45 +881,68 @@ void scene_refit_geometry(psdr_scene* s, cudaStream_t st) {
   PSDR_CUDA(cudaGetLastError());
 }
 
+// One allocation for all of a scene's buffers (45 stream-ordered allocations took as long as
+// building a small scene's geometry).
 void psdr_scene_alloc(psdr_scene* s) {
   cudaStream_t st = s->stream;
   const int n = std::max(1, s->ntri), nh = 3 * n;
-  s->verts.alloc(sizeof(float) * 3 * std::max(1, s->nvert), st);
-  s->tri.alloc(sizeof(float4) * 6 * n, st);
-  s->tri_v.alloc(sizeof(int4) * n, st);
-  s->objs.alloc(sizeof(DevObj) * std::max(1, s->nobj), st);
-  s->srcs.alloc(sizeof(DevSrc) * std::max(1, s->nobj), st);
-  s->lights_buf.alloc(sizeof(DevLight) * std::max(1, s->nlight), st);
-  s->light_pmf.alloc(sizeof(float) * std::max(1, s->nlight), st);
-  s->light_cmf.alloc(sizeof(float) * std::max(1, s->nlight), st);
   int nlt = 0;
   for (auto& l : s->h_lights) nlt += l.ntri;
-  s->ltri_pmf.alloc(sizeof(float) * std::max(1, nlt), st);
-  s->ltri_cmf.alloc(sizeof(float) * std::max(1, nlt), st);
-  s->n_edges.alloc(sizeof(int), st);
-  s->edge.alloc(sizeof(float4) * 4 * nh, st);
-  s->edge_v.alloc(sizeof(int2) * nh, st);
-  s->edge_f.alloc(sizeof(int2) * nh, st);
-  s->edge_pmf.alloc(sizeof(float) * nh, st);
-  s->edge_cmf.alloc(sizeof(float) * nh, st);
-  s->nodes.alloc(sizeof(float4) * kNodeF4 * n, st);
-  s->leaf.alloc(sizeof(float4) * 3 * n, st);
-  s->err.alloc(sizeof(int), st);
-  s->keys.alloc(sizeof(uint64_t) * nh, st);
-  s->vals.alloc(sizeof(uint32_t) * nh, st);
-  s->aux_i.alloc(sizeof(int2) * n, st);
-  s->aux_i2.alloc(sizeof(int) * nh, st);
-  s->aux_d.alloc(sizeof(int2) * n, st);
-  s->aux_d2.alloc(sizeof(double) * nh + sizeof(float) * nh, st);
-  s->aabb.alloc(sizeof(float) * 6 * (2 * (size_t)n), st);
-  s->box_levels.alloc(2 * sizeof(float) * box_level_floats(n), st);
-  s->range.alloc(sizeof(int2) * n, st);
-  s->flags.alloc(sizeof(int) * (2 * scan_tmp_ints(nh) + 64), st);
-  s->cbox.alloc(sizeof(unsigned int) * 12, st);
-  s->bvh_order.alloc(sizeof(uint32_t) * n, st);
-  s->bvh_counters.alloc(sizeof(int) * 3, st);
-  s->bvh_slots.alloc(sizeof(int) * 4 * (size_t)n, st);
-  s->d_dev.alloc(sizeof(DevScene), st);
+  std::vector<std::pair<DBuf*, size_t>> plan;
+  auto want = [&](DBuf& b, size_t bytes) { plan.emplace_back(&b, bytes); };
+  // the tables uploaded at creation come first (upload_tables copies them in one piece)
+  want(s->objs, sizeof(DevObj) * std::max(1, s->nobj));
+  want(s->srcs, sizeof(DevSrc) * std::max(1, s->nobj));
+  want(s->lights_buf, sizeof(DevLight) * std::max(1, s->nlight));
+  want(s->d_dev, sizeof(DevScene));
+  want(s->err, sizeof(int));
+  want(s->verts, sizeof(float) * 3 * std::max(1, s->nvert));
+  want(s->tri, sizeof(float4) * 6 * n);
+  want(s->tri_v, sizeof(int4) * n);
+  want(s->light_pmf, sizeof(float) * std::max(1, s->nlight));
+  want(s->light_cmf, sizeof(float) * std::max(1, s->nlight));
+  want(s->ltri_pmf, sizeof(float) * std::max(1, nlt));
+  want(s->ltri_cmf, sizeof(float) * std::max(1, nlt));
+  want(s->n_edges, sizeof(int));
+  want(s->edge, sizeof(float4) * 4 * nh);
+  want(s->edge_v, sizeof(int2) * nh);
+  want(s->edge_f, sizeof(int2) * nh);
+  want(s->edge_pmf, sizeof(float) * nh);
+  want(s->edge_cmf, sizeof(float) * nh);
+  want(s->nodes, sizeof(float4) * kNodeF4 * n);
+  want(s->leaf, sizeof(float4) * 3 * n);
+  want(s->bvh_order, sizeof(uint32_t) * n);
+  want(s->range, sizeof(int2) * n);
+  want(s->bvh_slots, sizeof(int) * 4 * (size_t)n);
+  want(s->bvh_counters, sizeof(int) * 3);
+  // build scratch
+  const size_t key = 2 * vertex_bits(s) <= 32 ? sizeof(uint32_t) : sizeof(uint64_t);
+  want(s->keys, key * nh);
+  want(s->vals, sizeof(uint32_t) * nh);
+  want(s->sort_tmp.keys2, key * nh);
+  want(s->sort_tmp.vals2, sizeof(uint32_t) * nh);
+  want(s->sort_tmp.hist, sizeof(int) * std::max(sort_hist_ints(nh, 2 * vertex_bits(s)), sort_hist_ints(n, 31)));
+  want(s->aux_i, sizeof(int2) * n);
+  want(s->aux_i2, sizeof(int) * nh);
+  want(s->aux_d, sizeof(int2) * n);
+  want(s->aux_d2, sizeof(double) * nh + sizeof(float) * nh);
+  want(s->aabb, sizeof(float) * 6 * (2 * (size_t)n));
+  want(s->box_levels, 2 * sizeof(float) * box_level_floats(n));
+  want(s->flags, sizeof(int) * (2 * scan_tmp_ints(nh) + 64));
+  want(s->cbox, sizeof(unsigned int) * 12);
+  // gradient accumulators
+  want(s->g_verts, sizeof(GradAcc) * 3 * std::max(1, s->nvert));
+  want(s->g_tex, sizeof(GradAcc) * std::max<size_t>(1, s->grad_texels));
+  want(s->g_emit, sizeof(GradAcc) * 3 * std::max(1, s->nlight));
+  want(s->vmask, std::max(1, s->nvert));
+  size_t total = 0;
+  for (auto& w : plan) total += (w.second + 255) & ~size_t(255);
+  s->slab.alloc(total, st);
+  size_t off = 0;
+  for (auto& w : plan) {
+    w.first->place(s->slab.as<unsigned char>() + off, w.second, st);
+    off += (w.second + 255) & ~size_t(255);
+  }
   PSDR_CUDA(cudaMemsetAsync(s->err.p, 0, sizeof(int), st));
   DevScene& d = s->dev;
   d.ntri = s->ntri; d.nvert = s->nvert; d.nobj = s->nobj; d.nlight = s->nlight;
@@ -876,8 +971,6 @@ void psdr_scene_alloc(psdr_scene* s) {
 // recorded into a batch graph) is made of device work only.
 void psdr_scene::upload_tables() {
   using namespace psdr;
-  PSDR_CUDA(cudaMemcpyAsync(objs.p, h_objs.data(), sizeof(DevObj) * std::max<size_t>(1, h_objs.size()),
-                            cudaMemcpyHostToDevice, stream));
   h_srcs.clear();
   for (int o = 0; o < nobj; ++o) {
     const bool is_mesh = o < (int)meshes.size();
@@ -897,9 +990,14 @@ void psdr_scene::upload_tables() {
     d.tri_off = obj_tri_off[o];
     h_srcs.push_back(d);
   }
-  PSDR_CUDA(cudaMemcpyAsync(srcs.p, h_srcs.data(), sizeof(DevSrc) * h_srcs.size(), cudaMemcpyHostToDevice, stream));
-  if (nlight > 0)
-    PSDR_CUDA(cudaMemcpyAsync(lights_buf.p, h_lights.data(), sizeof(DevLight) * nlight, cudaMemcpyHostToDevice,
-                              stream));
-  PSDR_CUDA(cudaMemcpyAsync(d_dev.p, &dev, sizeof(DevScene), cudaMemcpyHostToDevice, stream));
+  unsigned char* base = slab.as<unsigned char>();
+  std::vector<unsigned char> tables(d_dev.as<unsigned char>() - base + sizeof(DevScene), 0);
+  auto put = [&](const DBuf& b, const void* src, size_t bytes) {
+    if (bytes) memcpy(tables.data() + (b.as<unsigned char>() - base), src, bytes);
+  };
+  put(objs, h_objs.data(), sizeof(DevObj) * h_objs.size());
+  put(srcs, h_srcs.data(), sizeof(DevSrc) * h_srcs.size());
+  put(lights_buf, h_lights.data(), sizeof(DevLight) * h_lights.size());
+  put(d_dev, &dev, sizeof(DevScene));
+  PSDR_CUDA(cudaMemcpyAsync(base, tables.data(), tables.size(), cudaMemcpyHostToDevice, stream));
 }

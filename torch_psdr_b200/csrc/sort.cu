@@ -265,6 +265,11 @@ void inclusive_scan_widen(const float* in, const int* n_dev, double* out, int n,
   scan_impl<double, true>(PrefixOf{in, n_dev}, out, n, tmp, st);
 }
 
+size_t sort_hist_ints(int n, int bits) {
+  const size_t passes = (bits + 7) / 8, nt = ((size_t)n + kSortTile - 1) / kSortTile;
+  return passes * (256 + 1) + passes * nt * 256;
+}
+
 template <class K>
 static SortedKeys sort_impl(K* keys, uint32_t* vals, int n, int bits, SortTmp& tmp, cudaStream_t st) {
   const int passes = (bits + 7) / 8;
@@ -273,7 +278,7 @@ static SortedKeys sort_impl(K* keys, uint32_t* vals, int n, int bits, SortTmp& t
   if (n > 1) {
     const int nt = (n + kSortTile - 1) / kSortTile;
     // digit counts and tickets of every pass, then the tiles' status words
-    const size_t ints = (size_t)passes * (256 + 1) + (size_t)passes * nt * 256;
+    const size_t ints = sort_hist_ints(n, bits);
     tmp.keys2.alloc(sizeof(K) * n, st);
     tmp.vals2.alloc(sizeof(uint32_t) * n, st);
     tmp.hist.alloc(sizeof(int) * ints, st);
