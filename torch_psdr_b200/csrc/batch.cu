@@ -192,7 +192,9 @@ PSDR_API psdr_status psdr_batch_create(psdr_scene* const* scenes, int32_t n_scen
     }
     const int rec_needed = b->backward && !b->kept ? 1 : 0;
     b->ws.ensure(b->cap, Rmax, cfg->max_bounce, n_cams, rec_needed, st);
-    if (b->backward) ensure_border(&b->ws, *cfg, b->views, st);
+    bool jump = false;
+    for (int i = 0; i < n_scenes; ++i) jump = jump || scenes[i]->has_bsdf;
+    if (b->backward) ensure_border(&b->ws, *cfg, b->views, jump, b->cap, st);
     upload_views(&b->ws, b->views, st);
     // lanes: no more than the job has independent parts
     {
@@ -206,7 +208,7 @@ PSDR_API psdr_status psdr_batch_create(psdr_scene* const* scenes, int32_t n_scen
       b->lane_ws.emplace_back(new psdr_workspace());
       psdr_workspace* lw = b->lane_ws.back().get();
       lw->ensure(b->cap, Rmax, cfg->max_bounce, 1, rec_needed, st);
-      if (b->backward) ensure_border(lw, *cfg, b->views, st);
+      if (b->backward) ensure_border(lw, *cfg, b->views, jump, b->cap, st);
       cudaStream_t ls = nullptr;
       PSDR_CUDA(cudaStreamCreateWithFlags(&ls, cudaStreamNonBlocking));
       b->lane_st.push_back(ls);

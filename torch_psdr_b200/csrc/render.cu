@@ -3650,8 +3650,7 @@ static void run_tile(WF& w, const DevScene* scenes, const DevView* views, const 
 // Device bytes of a workspace per path of tile capacity (psdr_workspace::ensure).
 static size_t path_bytes(const psdr_config& cfg, bool records) {
   const size_t R = (size_t)cfg.mis_light_samples + std::max(cfg.mis_bsdf_samples, 1) + 1, D = cfg.max_bounce;
-  return 2 * 8 + 2 * 4 + 4 * 16 + 3 * 4 + 4 * 16 * R + 4 * 16 + 2 * 4 + 20 +
-         (records ? 16 * (1 + D * R + 2 * D) : 0);
+  return 2 * 8 + 2 * 4 + 4 * 16 + 3 * 4 + 4 * 16 * R + (records ? 16 * (1 + D * R + 2 * D) : 0);
 }
 
 // Paths of a wavefront tile when the caller leaves it to the library: 2^22, halved until the
@@ -3661,7 +3660,7 @@ static size_t path_bytes(const psdr_config& cfg, bool records) {
 // empty out; larger tiles pay for it less often. 1.31 M triangles, 1024^2 x 16 spp, depth 5:
 // traversal 18.2 ms with 2^20-path tiles, 14.7 with 2^21, 13.0 with 2^22.
 // A workspace that already holds such a tile keeps it without asking for the free memory.
-constexpr long long kTileMax = 1 << 22, kTileMin = 1 << 20;
+constexpr long long kTileMax = 1 << 22, kTileBatch = 1 << 21, kTileMin = 1 << 20;
 constexpr size_t kTileBytes = size_t(4) << 30;
 static long long auto_tile(const psdr_config& cfg, long long need, bool records, const psdr_workspace* ws) {
   if (need <= kTileMin) return kTileMin;
@@ -3679,7 +3678,8 @@ static long long auto_tile(const psdr_config& cfg, long long need, bool records,
 }
 
 // lanes: concurrent tiles of a batch; its automatic tile is small enough for each lane to
-// get one (but no smaller than 2^20).
+// get one, and at most 2^21 (the lanes' tiles fill one another's tails: 2^22 is no faster), but no
+// smaller than 2^20.
 int choose_cap(const psdr_config& cfg, const std::vector<DevView>& views, bool backward, int lanes,
                const psdr_workspace* ws) {
   int maxspp = 1;
@@ -3699,7 +3699,7 @@ int choose_cap(const psdr_config& cfg, const std::vector<DevView>& views, bool b
   long long cap = cfg.tile_paths > 0 ? cfg.tile_paths : auto_tile(cfg, need, backward, ws);
   if (backward) {
     if (cfg.tile_paths == 0) {
-      if (lanes > 1) cap = std::min(cap, std::max(kTileMin, (total + lanes - 1) / lanes));
+      if (lanes > 1) cap = std::min({cap, kTileBatch, std::max(kTileMin, (total + lanes - 1) / lanes)});
       cap = std::min(cap, need);
     }
     long long cells = std::max<long long>(cfg.primary_edge_hypercube_resolution,
@@ -3740,10 +3740,7 @@ void psdr_workspace::ensure(int c, int r, int d, int nv, int rec_needed, cudaStr
     q0.alloc(4 * n, st); q1.alloc(4 * n, st); qs.alloc(4 * n, st);
     cnt.alloc(sizeof(int) * 2 * (kMaxDepth + 2), st);
     ro.alloc(16 * n * R, st); rd.alloc(16 * n * R, st); ra.alloc(16 * n * R, st); hit.alloc(16 * n * R, st);
-    eb_a.alloc(16 * n, st); eb_n.alloc(16 * n, st); eb_hb.alloc(16 * n, st); eb_La.alloc(16 * n, st);
-    hc_pmf.alloc(4 * n, st); hc_cmf.alloc(4 * n, st);
   }
-  ensure_mass(cap, st);
   if (rec_needed) rec.alloc(16 * (size_t)cap * (1 + (size_t)D * R + 2 * (size_t)D), st);
   if (nv > nviews_cap) {
     nviews_cap = nv;
@@ -3932,19 +3929,35 @@ long long border_segments(const DevView& V) {
   return (long long)(V.W + 1) * V.H + (long long)V.W * (V.H + 1);
 }
 
-void ensure_border(psdr_workspace* ws, const psdr_config& cfg, const std::vector<DevView>& views, cudaStream_t st) {
+// Buffers of the boundary terms, sized for the job: the side buffers for the samples a tile of
+// `cap` holds at most (jump: the BSDF-jump term, one sample per path, is among the terms), the
+// masses and prefix sums for the guides' cells and the border segments.
+void ensure_border(psdr_workspace* ws, const psdr_config& cfg, const std::vector<DevView>& views, bool jump, int cap,
+                   cudaStream_t st) {
   const bool unb = cfg.estimator == PSDR_EST_UNBIASED;
   const int* r3 = cfg.secondary_edge_hypercube_resolution;
+  const long long cells1 = cfg.primary_edge_hypercube_resolution, cells2 = (long long)r3[0] * r3[1] * r3[2];
   const int rounds = std::min(kGuideRounds, cfg.secondary_edge_preprocess_rounds * (unb ? kDirectGuideRounds : 1));
-  ws->mass_rounds.alloc(sizeof(float) * (size_t)r3[0] * r3[1] * r3[2] * rounds, st);
-  if (!unb) return;
-  long long s = kCreaseCap, nt = 1;
+  long long samples = cells1, mass = std::max(cells1, cells2);
   for (const DevView& v : views) {
-    s = std::max(s, border_segments(v));
-    nt = std::max<long long>(nt, v.scene_ntri);
+    const long long px = (long long)v.H * v.W;
+    samples = std::max(samples, px * cfg.spp_primary_edge);
+    if (!unb) continue;
+    const long long S = border_segments(v);
+    samples = std::max({samples, S * cfg.spp_pixel_boundary, (long long)kCreaseSamplesPerSpp * cfg.spp_primary_edge,
+                        px * cfg.spp_secondary_edge / kIndirectSampleDiv + 1, jump ? px * v.spp : 0});
+    mass = std::max({mass, S, (long long)kCreaseCap, (long long)v.scene_ntri});
   }
-  ws->ensure_mass(std::max(s, nt), st);
-  ws->crease.alloc(80 * (size_t)kCreaseCap + 256 + 2 * 24 * (size_t)kCreaseBoxObjs, st);
+  const size_t n = (size_t)std::min<long long>(samples, cap);
+  ws->eb_a.alloc(16 * n, st);
+  ws->eb_n.alloc(16 * n, st);
+  ws->eb_hb.alloc(16 * n, st);
+  ws->eb_La.alloc(16 * n, st);
+  ws->hc_pmf.alloc(4 * (size_t)std::max(cells1, cells2), st);
+  ws->hc_cmf.alloc(4 * (size_t)std::max(cells1, cells2), st);
+  ws->ensure_mass(mass, st);
+  ws->mass_rounds.alloc(sizeof(float) * (size_t)cells2 * rounds, st);
+  if (unb) ws->crease.alloc(80 * (size_t)kCreaseCap + 256 + 2 * 24 * (size_t)kCreaseBoxObjs, st);
 }
 
 void set_scene_ntri(std::vector<DevView>& views, const psdr_scene* const* scenes) {
@@ -3989,7 +4002,7 @@ void render_backward_impl(const DevScene* scenes_dev, std::vector<DevView>& view
   const int cap = choose_cap(cfg, views, true, 1, ws);
   const int Rmax = cfg.mis_light_samples + std::max(cfg.mis_bsdf_samples, 1) + 1;
   ws->ensure(cap, Rmax, cfg.max_bounce, (int)views.size(), 1, st);
-  ensure_border(ws, cfg, views, st);
+  ensure_border(ws, cfg, views, gi.jump != 0, cap, st);
   upload_views(ws, views, st);
   backward_launch(scenes_dev, views, cfg, cap, ws, gi, st);
 }

@@ -189,7 +189,8 @@ constexpr int kLensAcc = 12;  // accumulators per view: S0, Sx, Sy, B (3x3)
 // out[10] (fp32, overwritten or accumulated) from a view's accumulators.
 void lens_out(const GradAcc* acc, const LensChain& ch, float* out, int accumulate, cudaStream_t st);
 long long border_segments(const DevView& V);
-void ensure_border(psdr_workspace* ws, const psdr_config& cfg, const std::vector<DevView>& views, cudaStream_t st);
+void ensure_border(psdr_workspace* ws, const psdr_config& cfg, const std::vector<DevView>& views, bool jump, int cap,
+                   cudaStream_t st);
 // Views of a backward job: their scene triangle counts (DevView::scene_ntri), before ensure_border.
 void set_scene_ntri(std::vector<DevView>& views, const psdr_scene* const* scenes);
 }  // namespace psdr
