@@ -147,7 +147,7 @@ typedef struct {
                           backward the interior tiles and every boundary term of every view
                           (1..8, 0 = 4; psdr_render_* run them one after another). Gradients
                           are bitwise the same for every value. */
-  int32_t batch_records; /* ABI 6: psdr_batch_* only: the forward keeps the replay records of
+  int32_t batch_records; /* ABI 6: psdr_batch_*: the forward keeps the replay records of
                             every interior path (16 B x (1 + D x R + 2 D) + 8 B per path, D =
                             max_bounce, R = light + BSDF samples + 1) and the backward runs the
                             adjoint from them instead of re-tracing the paths. 0 = when they
@@ -289,6 +289,19 @@ PSDR_API psdr_status psdr_render_samples(psdr_scene* scene, psdr_workspace* ws, 
 PSDR_API psdr_status psdr_autotune(psdr_scene* scene, psdr_workspace* ws, const psdr_camera_desc* cams,
                                    int32_t n_cams, psdr_config* cfg, int32_t* best_leaf, float* best_ms,
                                    void* stream);
+/* psdr_render_fwd that also writes the replay records of every interior path into `records`
+ * (device memory of psdr_records_bytes, 16-byte aligned; null: none), and psdr_render_bwd
+ * that runs the interior adjoint from them instead of re-tracing the paths (null: it
+ * re-traces). Scene, cameras and configuration must be those of the forward. Gradients
+ * are bitwise the same either way. */
+PSDR_API psdr_status psdr_records_bytes(const psdr_camera_desc* cams, int32_t n_cams, const psdr_config* cfg,
+                                        int64_t* bytes);
+PSDR_API psdr_status psdr_render_fwd_records(psdr_scene* scene, psdr_workspace* ws, const psdr_camera_desc* cams,
+                                             int32_t n_cams, const psdr_config* cfg, float** images, void* records,
+                                             void* stream);
+PSDR_API psdr_status psdr_render_bwd_records(psdr_scene* scene, psdr_workspace* ws, const psdr_camera_desc* cams,
+                                             int32_t n_cams, const psdr_config* cfg, const float** d_images,
+                                             const psdr_grad_targets* grads, void* records, void* stream);
 /* Path-replay adjoint of renderD (replaces Wrap2torch.backward + enoki's reverse
  * sweep, torch_psdr.py:48-72): interior term + the boundary terms of the selected
  * estimator. d_images[c] is dLoss/dImage (H,W,3) per camera. */

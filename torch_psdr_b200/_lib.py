@@ -93,6 +93,10 @@ SIGNATURES = {
     "psdr_workspace_create": ([C.POINTER(P)], C.c_int),
     "psdr_workspace_destroy": ([P], C.c_int),
     "psdr_render_fwd": ([P, P, C.POINTER(CameraDesc), C.c_int32, C.POINTER(Config), C.POINTER(P), P], C.c_int),
+    "psdr_records_bytes": ([C.POINTER(CameraDesc), C.c_int32, C.POINTER(Config), C.POINTER(C.c_int64)], C.c_int),
+    "psdr_render_fwd_records": ([P, P, C.POINTER(CameraDesc), C.c_int32, C.POINTER(Config), C.POINTER(P), P, P], C.c_int),
+    "psdr_render_bwd_records": ([P, P, C.POINTER(CameraDesc), C.c_int32, C.POINTER(Config), C.POINTER(P),
+                                 C.POINTER(GradTargets), P, P], C.c_int),
     "psdr_render_samples": ([P, P, C.POINTER(CameraDesc), C.POINTER(Config), P, P], C.c_int),
     "psdr_autotune": ([P, P, C.POINTER(CameraDesc), C.c_int32, C.POINTER(Config), C.POINTER(C.c_int32),
                        C.POINTER(C.c_float), P], C.c_int),

@@ -402,6 +402,15 @@ class Scene(VarContex):
         L.check(lib.psdr_scene_create(C.byref(desc), _stream(), C.byref(handle)), "psdr_scene_create")
         self._handle = handle
         self._lib = lib
+        self._builds = 0  # rebuilds since creation
+
+    def _stamp(self):
+        """Changes whenever the native scene, or a buffer it reads while rendering, does."""
+        tex = [t.data for m in self.meshes for t in (m.material.texture, m.material.roughness, m.material.normal)
+               if t is not None]
+        tex += [lt.cube_map.data for lt in self.lights if isinstance(lt, EnvLight)]
+        tex += [o.v for o in self.meshes + self.lights if o.v is not None]
+        return self._builds, tuple((t.data_ptr(), t._version) for t in tex)
 
     @property
     def handle(self):
@@ -423,6 +432,7 @@ class Scene(VarContex):
         """Rebuild triangle records, edges, CDFs and the BVH after Mesh.set_vertices.
         refit=True keeps the BVH's tree and recomputes only its boxes (same hits; for small
         vertex moves between full rebuilds)."""
+        self._builds += 1
         if refit:
             L.check(self._lib.psdr_scene_refit(self._handle, _stream()), "psdr_scene_refit")
         else:
@@ -443,11 +453,14 @@ class Scene(VarContex):
 
 class _RenderD(torch.autograd.Function):
     """Replaces Wrap2torch (torch_psdr.py:29-72): forward renders, backward runs the
-    path-replay adjoint and returns the gradient of every input tensor."""
+    path-replay adjoint and returns the gradient of every input tensor. The forward keeps
+    the paths' replay records for the backward when they fit (_Records)."""
 
     @staticmethod
-    def forward(ctx, integrator, scene, *torch_vars):
-        imgs = integrator._render(scene)
+    def forward(ctx, integrator, scene, keep, *torch_vars):
+        cams = scene._camera_descs()
+        ctx.records = integrator._new_records(scene, cams) if keep else None
+        imgs = integrator._render(scene, cams, ctx.records)
         ctx.integrator = integrator
         ctx.scene = scene
         ctx.n_vars = len(torch_vars)
@@ -458,8 +471,29 @@ class _RenderD(torch.autograd.Function):
     @torch.autograd.function.once_differentiable
     def backward(ctx, *grads):
         grads = [g if g is not None else None for g in grads]
-        out = ctx.integrator._backward(ctx.scene, grads, ctx.vars)
-        return (None, None) + tuple(out)
+        records, ctx.records = ctx.records, None  # a second backward re-traces the paths
+        out = ctx.integrator._backward(ctx.scene, grads, ctx.vars, records)
+        return (None, None, None) + tuple(out)
+
+
+class _Records:
+    """Replay records of one renderD forward: the device memory (a tensor, so it goes back to
+    torch's allocator with the autograd graph) and what they were made from. The backward
+    uses them only when the scene, cameras and configuration are still the same; otherwise
+    it re-traces the paths, as it does without records."""
+
+    def __init__(self, data, stamp):
+        self.data, self.stamp = data, stamp
+        self.stream = torch.cuda.current_stream()
+
+    def pointer(self, stamp):
+        """Address for a backward with this stamp; None: re-trace."""
+        if stamp != self.stamp:
+            return None
+        cur = torch.cuda.current_stream()
+        if cur != self.stream:
+            self.data.record_stream(cur)
+        return self.data.data_ptr()
 
 
 def _grad_buf(param, internal, new=torch.zeros_like):
@@ -537,7 +571,7 @@ class PathIntegrator:
         128; 0 = 8, the autotuner picks it), batch_lanes (BatchRender only: concurrent
         streams, each with its own workspace, over which a batch spreads its forward tiles
         and its backward's interior tiles and per-view boundary terms; 1..8, 0 = 4; the
-        gradients do not depend on it), batch_records (BatchRender only: the forward keeps
+        gradients do not depend on it), batch_records (renderD and BatchRender: the forward keeps
         every interior path's replay record and the backward runs the adjoint from them
         instead of re-tracing; 0 = when they fit in a quarter of the free device memory,
         1 = always, -1 = never; the gradients do not depend on it).
@@ -584,6 +618,7 @@ class PathIntegrator:
         self.cfg = cfg
         self._lib = L.load()
         self._ws = None
+        self._records_granted = 0  # bytes of replay records that fitted before
 
     def _workspace(self):
         if self._ws is None:
@@ -599,13 +634,39 @@ class PathIntegrator:
             except Exception:
                 pass
 
-    def _render(self, scene: Scene) -> List[Tensor]:
+    def _render(self, scene: Scene, cams=None, records=None) -> List[Tensor]:
         imgs = [torch.empty((c.height, c.width, 3), dtype=torch.float32, device="cuda") for c in scene.cameras]
         ptrs = (C.c_void_p * len(imgs))(*[i.data_ptr() for i in imgs])
-        cams = scene._camera_descs()
-        L.check(self._lib.psdr_render_fwd(scene.handle, self._workspace(), cams, len(imgs), C.byref(self.cfg),
-                                          ptrs, _stream()), "psdr_render_fwd")
+        cams = scene._camera_descs() if cams is None else cams
+        L.check(self._lib.psdr_render_fwd_records(scene.handle, self._workspace(), cams, len(imgs), C.byref(self.cfg),
+                                                  ptrs, None if records is None else records.data.data_ptr(),
+                                                  _stream()), "psdr_render_fwd")
         return imgs
+
+    def _stamp(self, scene: Scene, cams):
+        return bytes(cams), bytes(self.cfg), scene._stamp()
+
+    def _new_records(self, scene: Scene, cams):
+        """Memory for the replay records of a renderD forward, or None when they are not wanted
+        (batch_records = -1, no interior term) or take more than a quarter of the free memory."""
+        if self.cfg.batch_records < 0 or (self.cfg.terms and not self.cfg.terms & 1):
+            return None
+        n = C.c_int64()
+        L.check(self._lib.psdr_records_bytes(cams, len(cams), C.byref(self.cfg), C.byref(n)), "psdr_records_bytes")
+        n = int(n.value)
+        # (the free memory is asked for once per size: the query takes a third of a millisecond, and
+        # memory granted before stays in torch's cache)
+        if self.cfg.batch_records == 0 and n > max(64 << 20, self._records_granted):
+            free = torch.cuda.mem_get_info()[0] + torch.cuda.memory_reserved() - torch.cuda.memory_allocated()
+            if n > free // 4:
+                return None
+        try:
+            data = torch.empty(n, dtype=torch.uint8, device="cuda")
+        except torch.OutOfMemoryError:
+            self._records_granted = 0
+            return None
+        self._records_granted = max(n, self._records_granted)
+        return _Records(data, self._stamp(scene, cams))
 
     def autotune(self, scene: Scene, cache: Optional[str] = None) -> dict:
         """Pick the wavefront tile size and the scene's BVH leaf size by timing forward
@@ -640,6 +701,7 @@ class PathIntegrator:
         leaf = C.c_int32()
         ms = C.c_float()
         cams = scene._camera_descs()
+        scene._builds += 1
         L.check(self._lib.psdr_autotune(scene.handle, self._workspace(), cams, len(cams), C.byref(self.cfg),
                                         C.byref(leaf), C.byref(ms), _stream()), "psdr_autotune")
         return {"tile_paths": int(self.cfg.tile_paths), "leaf_size": int(leaf.value),
@@ -648,6 +710,7 @@ class PathIntegrator:
     def _apply_tuning(self, scene: Scene, entry: dict) -> None:
         self.cfg.tile_paths = int(entry["tile_paths"])
         self.cfg.trace_queue = int(entry.get("trace_queue", 0))
+        scene._builds += 1
         L.check(self._lib.psdr_scene_set_leaf_size(scene.handle, int(entry["leaf_size"]), _stream()),
                 "psdr_scene_set_leaf_size")
 
@@ -674,7 +737,7 @@ class PathIntegrator:
                                               C.byref(self.cfg), out.data_ptr(), _stream()), "psdr_render_samples")
         return out
 
-    def _backward(self, scene: Scene, grads, torch_vars):
+    def _backward(self, scene: Scene, grads, torch_vars, records=None):
         dev = "cuda"
         dimgs = []
         for g, c in zip(grads, scene.cameras):
@@ -704,8 +767,9 @@ class PathIntegrator:
         tg = L.GradTargets(vp, tp, ep, cp, 0, _ptrs(rough_g), _ptrs(nrm_g), _ptrs(light_g), _ptrs(lens_g))
         dp = (P * len(dimgs))(*[d.data_ptr() for d in dimgs])
         cams = scene._camera_descs()
-        L.check(self._lib.psdr_render_bwd(scene.handle, self._workspace(), cams, len(dimgs), C.byref(self.cfg), dp,
-                                          C.byref(tg), _stream()), "psdr_render_bwd")
+        rec = None if records is None else records.pointer(self._stamp(scene, cams))
+        L.check(self._lib.psdr_render_bwd_records(scene.handle, self._workspace(), cams, len(dimgs), C.byref(self.cfg),
+                                                  dp, C.byref(tg), rec, _stream()), "psdr_render_bwd")
         # map the accumulators onto the input tensors (a tensor may play several roles)
         acc = {}
 
@@ -745,7 +809,7 @@ class PathIntegrator:
             return self._render(scene)
         for c in scene.cameras:  # refuse unsupported camera gradients before rendering
             _lens_buf(c, self.cfg.estimator == L.EST_UNBIASED)
-        imgs = _RenderD.apply(self, scene, *torch_vars)
+        imgs = _RenderD.apply(self, scene, torch.is_grad_enabled(), *torch_vars)
         return list(imgs)
 
 
@@ -827,6 +891,8 @@ class BatchRender:
         """Rebuild geometry and render every camera (returns the bound image buffers)."""
         cur = torch.cuda.current_stream()
         self.stream.wait_stream(cur)
+        for sc in self.scenes:
+            sc._builds += 1  # the graph rebuilds every scene
         L.check(self.lib.psdr_batch_forward(self._handle, C.c_void_p(self.stream.cuda_stream)), "psdr_batch_forward")
         cur.wait_stream(self.stream)
         return self.images

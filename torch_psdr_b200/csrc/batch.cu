@@ -41,7 +41,7 @@ struct psdr_batch {
   int nlanes = 1;
   // replay records of every interior path, written by the forward (cfg.batch_records)
   bool kept = false;
-  psdr::DBuf keep_rec, keep_view, keep_pix;
+  psdr::DBuf keep_rec;
   psdr::KeptRecords keep;
   std::vector<std::unique_ptr<psdr_workspace>> lane_ws;
   std::vector<cudaStream_t> lane_st;
@@ -174,20 +174,13 @@ PSDR_API psdr_status psdr_batch_create(psdr_scene* const* scenes, int32_t n_scen
     if (b->backward && cfg->batch_records >= 0) {
       long long paths = 0;
       for (const DevView& v : b->views) paths += (long long)v.H * v.W * v.spp;
-      const int R = cfg->mis_light_samples + cfg->mis_bsdf_samples + 1;
-      const size_t stride = 1 + (size_t)cfg->max_bounce * R + 2 * (size_t)cfg->max_bounce;
-      const size_t bytes = (size_t)paths * (16 * stride + 8);
+      const size_t bytes = records_bytes(*cfg, paths);
       size_t free_b = 0, total_b = 0;
       PSDR_CUDA(cudaMemGetInfo(&free_b, &total_b));
       b->kept = cfg->batch_records == 1 || bytes <= free_b / 4;
       if (b->kept) {
-        b->keep_rec.alloc(16 * stride * (size_t)paths, st);
-        b->keep_view.alloc(4 * (size_t)paths, st);
-        b->keep_pix.alloc(4 * (size_t)paths, st);
-        b->keep.rec = b->keep_rec.as<float4>();
-        b->keep.plane = (size_t)paths;
-        b->keep.view = b->keep_view.as<int>();
-        b->keep.pix = b->keep_pix.as<int>();
+        b->keep_rec.alloc(bytes, st);
+        b->keep = place_records(b->keep_rec.p, *cfg, paths);
       }
     }
     const int rec_needed = b->backward && !b->kept ? 1 : 0;

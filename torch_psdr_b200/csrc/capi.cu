@@ -243,6 +243,13 @@ static void check_index_ranges(const psdr_scene_desc* desc, void* stream) {
   }
 }
 
+// Interior paths of a job.
+static long long job_paths(const psdr_camera_desc* cams, int n, const psdr_config& cfg) {
+  long long p = 0;
+  for (int i = 0; i < n; ++i) p += (long long)cams[i].height * cams[i].width * cfg.spp_interior;
+  return p;
+}
+
 extern "C" {
 
 const char* psdr_last_error(void) { return psdr::g_err.c_str(); }
@@ -529,8 +536,23 @@ psdr_status psdr_workspace_destroy(psdr_workspace* ws) {
   API_END
 }
 
+psdr_status psdr_records_bytes(const psdr_camera_desc* cams, int32_t n_cams, const psdr_config* cfg, int64_t* bytes) {
+  API_BEGIN
+  PSDR_CHECK(bytes != nullptr, "null argument");
+  check_cfg(cfg);
+  check_cams(cams, n_cams);
+  *bytes = (int64_t)records_bytes(*cfg, job_paths(cams, n_cams, *cfg));
+  API_END
+}
+
 psdr_status psdr_render_fwd(psdr_scene* scene, psdr_workspace* ws, const psdr_camera_desc* cams, int32_t n_cams,
                             const psdr_config* cfg, float** images, void* stream) {
+  return psdr_render_fwd_records(scene, ws, cams, n_cams, cfg, images, nullptr, stream);
+}
+
+psdr_status psdr_render_fwd_records(psdr_scene* scene, psdr_workspace* ws, const psdr_camera_desc* cams,
+                                    int32_t n_cams, const psdr_config* cfg, float** images, void* records,
+                                    void* stream) {
   API_BEGIN
   PSDR_CHECK(scene && ws && images, "null argument");
   check_cfg(cfg);
@@ -543,7 +565,12 @@ psdr_status psdr_render_fwd(psdr_scene* scene, psdr_workspace* ws, const psdr_ca
     make_view(cams[i], cfg->spp_interior, views[i]);
     views[i].image = images[i];
   }
-  render_forward_impl(dev_scene(scene), views, *cfg, ws, (cudaStream_t)stream, nullptr);
+  KeptRecords keep;
+  if (records) {
+    PSDR_CHECK(reinterpret_cast<uintptr_t>(records) % 16 == 0, "records must be 16-byte aligned");
+    keep = place_records(records, *cfg, job_paths(cams, n_cams, *cfg));
+  }
+  render_forward_impl(dev_scene(scene), views, *cfg, ws, (cudaStream_t)stream, nullptr, records ? &keep : nullptr);
   API_END
 }
 
@@ -654,6 +681,12 @@ psdr_status psdr_camera_lens_jacobian(const psdr_camera_desc* cam, double* m9, d
 psdr_status psdr_render_bwd(psdr_scene* scene, psdr_workspace* ws, const psdr_camera_desc* cams, int32_t n_cams,
                             const psdr_config* cfg, const float** d_images, const psdr_grad_targets* grads,
                             void* stream) {
+  return psdr_render_bwd_records(scene, ws, cams, n_cams, cfg, d_images, grads, nullptr, stream);
+}
+
+psdr_status psdr_render_bwd_records(psdr_scene* scene, psdr_workspace* ws, const psdr_camera_desc* cams,
+                                    int32_t n_cams, const psdr_config* cfg, const float** d_images,
+                                    const psdr_grad_targets* grads, void* records, void* stream) {
   API_BEGIN
   PSDR_CHECK(scene && ws && d_images && grads, "null argument");
   check_cfg(cfg);
@@ -705,7 +738,12 @@ psdr_status psdr_render_bwd(psdr_scene* scene, psdr_workspace* ws, const psdr_ca
     const psdr_scene* sl[1] = {scene};
     set_scene_ntri(views, sl);
   }
-  render_backward_impl(dev_scene(scene), views, *cfg, ws, grad_info(scene), st);
+  KeptRecords keep;
+  if (records) {
+    PSDR_CHECK(reinterpret_cast<uintptr_t>(records) % 16 == 0, "records must be 16-byte aligned");
+    keep = place_records(records, *cfg, job_paths(cams, n_cams, *cfg));
+  }
+  render_backward_impl(dev_scene(scene), views, *cfg, ws, grad_info(scene), st, records ? &keep : nullptr);
   const int nm = (int)scene->meshes.size();
   for (int o = 0; o < scene->nobj; ++o) {
     if (grads->vertices && grads->vertices[o])

@@ -3681,7 +3681,7 @@ static long long auto_tile(const psdr_config& cfg, long long need, bool records,
 // get one, and at most 2^21 (the lanes' tiles fill one another's tails: 2^22 is no faster), but no
 // smaller than 2^20.
 int choose_cap(const psdr_config& cfg, const std::vector<DevView>& views, bool backward, int lanes,
-               const psdr_workspace* ws) {
+               const psdr_workspace* ws, bool records) {
   int maxspp = 1;
   long long total = 0, need = 0;
   for (auto& v : views) {
@@ -3696,7 +3696,7 @@ int choose_cap(const psdr_config& cfg, const std::vector<DevView>& views, bool b
                        2ll * kCreaseSamplesPerSpp * cfg.spp_primary_edge, px * v.spp});
   }
   need = std::max(need, total);
-  long long cap = cfg.tile_paths > 0 ? cfg.tile_paths : auto_tile(cfg, need, backward, ws);
+  long long cap = cfg.tile_paths > 0 ? cfg.tile_paths : auto_tile(cfg, need, backward && records, ws);
   if (backward) {
     if (cfg.tile_paths == 0) {
       if (lanes > 1) cap = std::min({cap, kTileBatch, std::max(kTileMin, (total + lanes - 1) / lanes)});
@@ -3803,19 +3803,19 @@ void forward_tile(const DevScene* scenes_dev, const std::vector<DevView>& views,
 // Device work of a forward job whose views are already in ws->views (tiles of `cap`
 // paths). Makes no allocation and no host copy, so it can be recorded into a graph.
 void forward_launch(const DevScene* scenes_dev, const std::vector<DevView>& views, const psdr_config& cfg, int cap,
-                    psdr_workspace* ws, cudaStream_t st, float* samples_out) {
+                    psdr_workspace* ws, cudaStream_t st, float* samples_out, const KeptRecords* keep) {
   const DevView* vd = ws->views.as<DevView>();
-  for (const Tile& t : plan_tiles(views, cap)) forward_tile(scenes_dev, views, vd, t, cfg, ws, st, samples_out);
+  for (const Tile& t : plan_tiles(views, cap)) forward_tile(scenes_dev, views, vd, t, cfg, ws, st, samples_out, keep);
 }
 
 void render_forward_impl(const DevScene* scenes_dev, std::vector<DevView>& views, const psdr_config& cfg,
-                         psdr_workspace* ws, cudaStream_t st, float* samples_out) {
+                         psdr_workspace* ws, cudaStream_t st, float* samples_out, const KeptRecords* keep) {
   assign_offsets(views);
   const int cap = choose_cap(cfg, views, false, 1, ws);
   const int R = cfg.mis_light_samples + cfg.mis_bsdf_samples + 1;
   ws->ensure(cap, R, cfg.max_bounce, (int)views.size(), 0, st);
   upload_views(ws, views, st);
-  forward_launch(scenes_dev, views, cfg, cap, ws, st, samples_out);
+  forward_launch(scenes_dev, views, cfg, cap, ws, st, samples_out, keep);
 }
 
 static void edge_phase(WF w, const DevScene* scenes, const DevView* vd, int v, const EdgeBuf& eb, long long begin,
@@ -3993,18 +3993,15 @@ static HCube build_hcube(psdr_workspace* ws, int ncells, const int* res, int N, 
 
 // Backward: interior path replay + adjoint, then the primary- and direct-edge terms
 // of every view. Views must carry dimage (and grad_pos when wanted).
-void backward_launch(const DevScene* scenes_dev, const std::vector<DevView>& views, const psdr_config& cfg,
-                     int cap, psdr_workspace* ws, const SceneGradInfo& gi, cudaStream_t st);
-
 void render_backward_impl(const DevScene* scenes_dev, std::vector<DevView>& views, const psdr_config& cfg,
-                          psdr_workspace* ws, const SceneGradInfo& gi, cudaStream_t st) {
+                          psdr_workspace* ws, const SceneGradInfo& gi, cudaStream_t st, const KeptRecords* keep) {
   assign_offsets(views);
-  const int cap = choose_cap(cfg, views, true, 1, ws);
+  const int cap = choose_cap(cfg, views, true, 1, ws, keep == nullptr);
   const int Rmax = cfg.mis_light_samples + std::max(cfg.mis_bsdf_samples, 1) + 1;
-  ws->ensure(cap, Rmax, cfg.max_bounce, (int)views.size(), 1, st);
+  ws->ensure(cap, Rmax, cfg.max_bounce, (int)views.size(), keep ? 0 : 1, st);
   ensure_border(ws, cfg, views, gi.jump != 0, cap, st);
   upload_views(ws, views, st);
-  backward_launch(scenes_dev, views, cfg, cap, ws, gi, st);
+  backward_launch(scenes_dev, views, cfg, cap, ws, gi, st, keep);
 }
 
 // The terms of a backward job: cfg.terms, or by default interior + primary + direct edges
@@ -4278,10 +4275,10 @@ void backward_unit(const DevScene* scenes_dev, const std::vector<DevView>& views
 // Device work of a backward job (views already uploaded); no allocation, no host copy.
 // The units run one after another on st with one workspace.
 void backward_launch(const DevScene* scenes_dev, const std::vector<DevView>& views, const psdr_config& cfg,
-                     int cap, psdr_workspace* ws, const SceneGradInfo& gi, cudaStream_t st) {
+                     int cap, psdr_workspace* ws, const SceneGradInfo& gi, cudaStream_t st, const KeptRecords* keep) {
   const DevView* vd = ws->views.as<DevView>();
   for (const BwdUnit& u : backward_units(views, cfg, cap, gi))
-    backward_unit(scenes_dev, views, vd, u, cfg, cap, ws, gi, st);
+    backward_unit(scenes_dev, views, vd, u, cfg, cap, ws, gi, st, keep);
 }
 
 void grad_out(const GradAcc* acc, float* out, long long n, int accumulate, cudaStream_t st) {

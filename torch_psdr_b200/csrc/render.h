@@ -84,6 +84,22 @@ struct KeptRecords {
   int* pix = nullptr;
 };
 
+// float4 records of a path, and bytes of the kept records (with views and pixels) of a job.
+inline size_t record_planes(const psdr_config& c) {
+  const size_t R = (size_t)c.mis_light_samples + c.mis_bsdf_samples + 1;
+  return 1 + (size_t)c.max_bounce * R + 2 * (size_t)c.max_bounce;
+}
+inline size_t records_bytes(const psdr_config& c, long long paths) { return (size_t)paths * (16 * record_planes(c) + 8); }
+// The parts of a buffer of records_bytes.
+inline KeptRecords place_records(void* p, const psdr_config& c, long long paths) {
+  KeptRecords k;
+  k.rec = static_cast<float4*>(p);
+  k.plane = (size_t)paths;
+  k.view = reinterpret_cast<int*>(k.rec + record_planes(c) * (size_t)paths);
+  k.pix = k.view + paths;
+  return k;
+}
+
 struct psdr_ws_impl;
 
 }  // namespace psdr
@@ -128,22 +144,24 @@ Profiler& profiler();
 struct SceneGradInfo;
 void make_view(const psdr_camera_desc& c, int spp, DevView& v);
 void render_forward_impl(const DevScene* scenes_dev, std::vector<DevView>& views, const psdr_config& cfg,
-                         psdr_workspace* ws, cudaStream_t st, float* samples_out);
+                         psdr_workspace* ws, cudaStream_t st, float* samples_out, const KeptRecords* keep = nullptr);
 struct SceneGradInfo {
   int bsdf = 0;  // a DiffuseBsdfMaterial mesh or an environment light (extended adjoint kernel)
   int jump = 0;  // a DiffuseBsdfMaterial mesh: the unbiased default terms include its BRDF jumps
 };
 void render_backward_impl(const DevScene* scenes_dev, std::vector<DevView>& views, const psdr_config& cfg,
-                          psdr_workspace* ws, const SceneGradInfo& gi, cudaStream_t st);
+                          psdr_workspace* ws, const SceneGradInfo& gi, cudaStream_t st,
+                          const KeptRecords* keep = nullptr);
 void grad_out(const GradAcc* acc, float* out, long long n, int accumulate, cudaStream_t st);
 void assign_offsets(std::vector<DevView>& views);
 int choose_cap(const psdr_config& cfg, const std::vector<DevView>& views, bool backward, int lanes,
-               const psdr_workspace* ws);
+               const psdr_workspace* ws, bool records = true);
 void upload_views(psdr_workspace* ws, const std::vector<DevView>& views, cudaStream_t st);
 void forward_launch(const DevScene* scenes_dev, const std::vector<DevView>& views, const psdr_config& cfg, int cap,
-                    psdr_workspace* ws, cudaStream_t st, float* samples_out);
+                    psdr_workspace* ws, cudaStream_t st, float* samples_out, const KeptRecords* keep = nullptr);
 void backward_launch(const DevScene* scenes_dev, const std::vector<DevView>& views, const psdr_config& cfg,
-                     int cap, psdr_workspace* ws, const SceneGradInfo& gi, cudaStream_t st);
+                     int cap, psdr_workspace* ws, const SceneGradInfo& gi, cudaStream_t st,
+                     const KeptRecords* keep = nullptr);
 // One forward tile (camera paths, depth loop, film) on workspace ws; views at vd.
 // With `keep`, the tile's replay records, views and pixels go to its place in `keep`.
 void forward_tile(const DevScene* scenes_dev, const std::vector<DevView>& views, const DevView* vd, const Tile& t,
