@@ -46,3 +46,30 @@ def test_list_adjoint_matches_path_walk(cuda, estimator, size, spp, depth, nl, n
         # sums of the same fp32 terms in another grouping: about sqrt(terms) 2^-24 of their size,
         # and terms of both signs cancel to about a tenth of it
         assert rel_l2(a[k], b[k]) < 2e-5, (k, rel_l2(a[k], b[k]))
+
+
+@pytest.mark.parametrize("estimator", ["reference", "unbiased"])
+@pytest.mark.parametrize("size,spp,depth,nl,nb", [((1, 1), 1, 1, 1, 1), ((7, 9), 3, 1, 0, 1), ((33, 31), 32, 3, 1, 1),
+                                                  ((40, 24), 5, 6, 2, 3)])
+@pytest.mark.parametrize("batch", [False, True])
+def test_other_gradients_do_not_depend_on_vertex_gradients(cuda, estimator, size, spp, depth, nl, nb, batch):
+    """The kernel without vertex gradients forms the same texel, emission and camera adjoints."""
+    spec = synth.sphere_scene(level=2, tex_hw=9, noise_sigma=0.05, height=size[0], width=size[1])
+    d_image = torch.as_tensor(np.random.default_rng(1).normal(size=size + (3,)), dtype=torch.float32, device="cuda")
+    out = []
+    for kinds in ({"tex", "emit", "cam"}, {"tex", "emit", "cam", "verts", "light_verts"}):
+        scene, T = to_torch_scene(spec, requires_grad=kinds)
+        it = dr.PathIntegrator(gradient_terms=1, estimator=estimator, spp_interior=spp, max_bounce=depth,
+                               mis_light_samples=nl, mis_bsdf_samples=nb, enable_light_visable=True)
+        img = dr.BatchRender(it, [scene]).renderD()[0] if batch else it.renderD(scene)[0]
+        img.backward(d_image)
+        out.append((img.detach().clone(), {k: t.grad.clone() for k, t in T.items() if k.startswith(("tex", "emit", "cam"))
+                                           and t is not None and t.grad is not None}))
+    assert torch.equal(out[0][0], out[1][0])
+    assert out[0][1] and out[0][1].keys() == out[1][1].keys()
+    for k, a in out[0][1].items():
+        if torch.equal(a, out[1][1][k]):
+            continue
+        # the same fp32 terms up to the rounding of differently contracted products, summed in
+        # fixed point
+        assert rel_l2(a.cpu().numpy(), out[1][1][k].cpu().numpy()) < 1e-6, k

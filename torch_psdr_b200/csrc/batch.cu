@@ -251,6 +251,9 @@ PSDR_API psdr_status psdr_batch_create(psdr_scene* const* scenes, int32_t n_scen
       if (scenes[i]->has_bsdf) b->gi.jump = 1;
     }
     for (auto& lw : b->lane_ws) lw->bsdf = b->ws.bsdf;
+    b->gi.verts = 0;
+    for (int i = 0; b->backward && i < n_scenes; ++i)
+      for (int o = 0; grads[i].vertices && o < scenes[i]->nobj; ++o) b->gi.verts |= grads[i].vertices[o] != nullptr;
     if (b->backward) {
       b->gv.resize(n_scenes);
       b->gt.resize(n_scenes);

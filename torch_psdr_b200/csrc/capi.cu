@@ -743,7 +743,10 @@ psdr_status psdr_render_bwd_records(psdr_scene* scene, psdr_workspace* ws, const
     PSDR_CHECK(reinterpret_cast<uintptr_t>(records) % 16 == 0, "records must be 16-byte aligned");
     keep = place_records(records, *cfg, job_paths(cams, n_cams, *cfg));
   }
-  render_backward_impl(dev_scene(scene), views, *cfg, ws, grad_info(scene), st, records ? &keep : nullptr);
+  SceneGradInfo gi = grad_info(scene);
+  gi.verts = 0;
+  for (int o = 0; grads->vertices && o < scene->nobj; ++o) gi.verts |= grads->vertices[o] != nullptr;
+  render_backward_impl(dev_scene(scene), views, *cfg, ws, gi, st, records ? &keep : nullptr);
   const int nm = (int)scene->meshes.size();
   for (int o = 0; o < scene->nobj; ++o) {
     if (grads->vertices && grads->vertices[o])

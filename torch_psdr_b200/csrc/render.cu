@@ -909,7 +909,10 @@ PSDR_D void geom_adj_points(float adjG, const Surf& x, const Surf& q, SurfAdj& a
 // BSDF (DiffuseBsdfMaterial in the scene): the BSDF value depends on the shading normal
 // (mp), the incoming direction x.wi and the outgoing direction; their adjoints and the
 // color / roughness adjoints gather in ma (adj_tex is unused).
-template <bool BSDF>
+// VERTS: some vertex gradient is wanted; without it only the texel and emission adjoints are
+// formed (a material of direction-dependent value also passes adjoints on through
+// directions, so its kernel always has VERTS).
+template <bool BSDF, bool VERTS>
 PSDR_D void light_sample_adj(const WF& w, const DevScene& sc, const Surf& x, float3 bsdf, float rx, float ry, float4 h,
                              float3 adjC, SurfAdj& ax, HotAcc& hot, float3& adj_tex, const MatPt* mp, MatAdj* ma) {
   const int tri = __float_as_int(h.x);
@@ -935,6 +938,7 @@ PSDR_D void light_sample_adj(const WF& w, const DevScene& sc, const Surf& x, flo
   const float3 eb = mul(emit, f);
   const float3 ae = mul(av, f) * s_;
   add_light_emit<BSDF>(sc, hot, ls.light, q, ae, ax);
+  if (!VERTS) return;
   const float adj_gam = dot(av, eb) / ls.pdf;
   SurfAdj aq = zero_adj();
   aq.area = adj_gam * G / q.area;
@@ -953,7 +957,7 @@ PSDR_D void light_sample_adj(const WF& w, const DevScene& sc, const Surf& x, flo
   scatter_surf(sc, hot, tri, h.y, h.z, q.front, aq);
 }
 
-template <bool UNB, bool BSDF>
+template <bool UNB, bool BSDF, bool VERTS>
 PSDR_D void bsdf_sample_adj(const WF& w, const DevScene& sc, const Surf& x, float3 bsdf, float rx, float ry, float4 h,
                             float3 adjC, SurfAdj& ax, HotAcc& hot, float3& adj_tex, const MatPt* mp, MatAdj* ma) {
   const int tri = __float_as_int(h.x);
@@ -981,6 +985,7 @@ PSDR_D void bsdf_sample_adj(const WF& w, const DevScene& sc, const Surf& x, floa
   const float3 eb = mul(emit, f);
   const float3 ae = mul(av, f) * s_;
   add_light_emit<BSDF>(sc, hot, q.light, q, ae, ax);
+  if (!VERTS) return;
   const float adj_gam = dot(av, eb) / pdf_b;
   SurfAdj aq = zero_adj();
   aq.area = adj_gam * G / q.area;
@@ -997,7 +1002,7 @@ PSDR_D void bsdf_sample_adj(const WF& w, const DevScene& sc, const Surf& x, floa
 
 // Returns false when the path ends here; otherwise carry = the adjoint of the next vertex nx,
 // passed to the next depth.
-template <bool UNB, bool BSDF>
+template <bool UNB, bool BSDF, bool VERTS>
 PSDR_D bool continuation_adj(const DevScene& sc, const Surf& x, float3 bsdf, float rx, float ry, float4 h, float3 adjB,
                              SurfAdj& ax, SurfAdj& carry, Surf& nx, float3& adj_tex, const MatPt* mp, MatAdj* ma) {
   const int tri = __float_as_int(h.x);
@@ -1014,6 +1019,7 @@ PSDR_D bool continuation_adj(const DevScene& sc, const Surf& x, float3 bsdf, flo
   float3 f = bsdf;
   if (BSDF) f = bsdf_adj(*mp, x.wi, UNB ? normalize(nx.p - x.p) : wo, adjB * s_, *ma, adjL);
   else adj_tex += adjB * (s_ * kInvPi);
+  if (!VERTS) return true;
   const float adj_gam = dot(adjB, f) / pdf;
   carry = zero_adj();
   carry.area = adj_gam * G / nx.area;
@@ -1199,7 +1205,10 @@ __host__ __device__ constexpr int adj_warp_words(int nB) { return kVertFields * 
 // block starting together. Bound by instruction fetch (7.2 of 18.3 cycles per issued
 // instruction before that, 25 % occupancy at 128 registers) and by the latency of its record
 // loads; DRAM 7 % busy.
-template <bool UNB>
+// Without vertex gradients (VERTS false: texture and emission optimisation) the lists carry no
+// surface adjoint and the vertex scatters go; 256^2 x 64 spp: 0.83 -> 0.55 ms (three blocks per
+// SM spill: 0.63 ms).
+template <bool UNB, bool VERTS>
 __global__ void __launch_bounds__(32 * kAdjWarps, 2) k_adjoint(WF w, const DevScene* __restrict__ scenes,
                                                                const DevView* __restrict__ views, Tile tile) {
   extern __shared__ float adj_lists[];
@@ -1242,10 +1251,10 @@ __global__ void __launch_bounds__(32 * kAdjWarps, 2) k_adjoint(WF w, const DevSc
         const int off = texel_offset(ob.color, x.u, x.v);
         SurfAdj ax = zero_adj();
         float3 atx = f3(0.f, 0.f, 0.f);
-        bsdf_sample_adj<UNB, false>(w, sc, x, tex_rgb(ob.color, off) * kInvPi, rx, ry,
+        bsdf_sample_adj<UNB, false, VERTS>(w, sc, x, tex_rgb(ob.color, off) * kInvPi, rx, ry,
                                     rec_hit(w, s, d, w.nL + j), adjC, ax, hot, atx, nullptr, nullptr);
         scatter_tex(ob.color, off, atx, false);
-        scatter_mesh(sc, tri, hx.y, hx.z, x.front, ax);
+        if (VERTS) scatter_mesh(sc, tri, hx.y, hx.z, x.front, ax);
       }
       __syncwarp();
       continue;
@@ -1303,10 +1312,12 @@ __global__ void __launch_bounds__(32 * kAdjWarps, 2) k_adjoint(WF w, const DevSc
         T = f3(vget(5, e), vget(6, e), vget(7, e));
         rng.state = (unsigned long long)__float_as_uint(vget(8, e)) | (unsigned long long)__float_as_uint(vget(9, e)) << 32;
         rng.inc = (unsigned long long)__float_as_uint(vget(10, e)) | (unsigned long long)__float_as_uint(vget(11, e)) << 32;
-        ax.p = f3(vget(12, e), vget(13, e), vget(14, e));
-        ax.n = f3(vget(15, e), vget(16, e), vget(17, e));
-        ax.t = f3(vget(18, e), vget(19, e), vget(20, e));
-        ax.area = vget(21, e);
+        if (VERTS) {
+          ax.p = f3(vget(12, e), vget(13, e), vget(14, e));
+          ax.n = f3(vget(15, e), vget(16, e), vget(17, e));
+          ax.t = f3(vget(18, e), vget(19, e), vget(20, e));
+          ax.area = vget(21, e);
+        }
         const DevView& V = views[w.view[s]];
         scp = &scenes[V.scene];
         hot_bind(hot, scp);
@@ -1328,7 +1339,7 @@ __global__ void __launch_bounds__(32 * kAdjWarps, 2) k_adjoint(WF w, const DevSc
       bsdf = tex_rgb(*tx, toff) * kInvPi;
       for (int i = 0; i < w.nL; ++i) {
         const float rx = rng.next_float(), ry = rng.next_float();
-        light_sample_adj<false>(w, *scp, x, bsdf, rx, ry, rec_hit(w, s, d, i), adjC, ax, hot, atx, nullptr, nullptr);
+        light_sample_adj<false, VERTS>(w, *scp, x, bsdf, rx, ry, rec_hit(w, s, d, i), adjC, ax, hot, atx, nullptr, nullptr);
       }
     }
     for (int j = 0; j < w.nB; ++j) {
@@ -1359,16 +1370,16 @@ __global__ void __launch_bounds__(32 * kAdjWarps, 2) k_adjoint(WF w, const DevSc
     if (act && d < w.D - 1) {
       const float rx = rng.next_float(), ry = rng.next_float();
       const float3 adjB = mul(adjC, suffix_radiance(w, s, d + 1));
-      go = continuation_adj<UNB, false>(*scp, x, bsdf, rx, ry, rec_hit(w, s, d, w.nL + w.nB), adjB, ax, carry, nx, atx,
+      go = continuation_adj<UNB, false, VERTS>(*scp, x, bsdf, rx, ry, rec_hit(w, s, d, w.nL + w.nB), adjB, ax, carry, nx, atx,
                                         nullptr, nullptr) &&
            !nx.is_light;  // a path that ends on a light has nothing downstream
     }
     if (fresh) {
-      scatter_surf_warp(scp, hot, tri, hx.y, hx.z, x.front, ax, has0);
+      if (VERTS) scatter_surf_warp(scp, hot, tri, hx.y, hx.z, x.front, ax, has0);
       scatter_tex_warp(tx, toff, atx, has0);
     } else if (act) {
       scatter_tex(*tx, toff, atx, false);
-      scatter_mesh(*scp, tri, hx.y, hx.z, x.front, ax);
+      if (VERTS) scatter_mesh(*scp, tri, hx.y, hx.z, x.front, ax);
     }
     const unsigned m = __ballot_sync(0xffffffffu, go);
     if (go) {
@@ -1380,10 +1391,12 @@ __global__ void __launch_bounds__(32 * kAdjWarps, 2) k_adjoint(WF w, const DevSc
       vput(5, e, Tn.x); vput(6, e, Tn.y); vput(7, e, Tn.z);
       vput(8, e, __uint_as_float((unsigned)rng.state)); vput(9, e, __uint_as_float((unsigned)(rng.state >> 32)));
       vput(10, e, __uint_as_float((unsigned)rng.inc)); vput(11, e, __uint_as_float((unsigned)(rng.inc >> 32)));
-      vput(12, e, carry.p.x); vput(13, e, carry.p.y); vput(14, e, carry.p.z);
-      vput(15, e, carry.n.x); vput(16, e, carry.n.y); vput(17, e, carry.n.z);
-      vput(18, e, carry.t.x); vput(19, e, carry.t.y); vput(20, e, carry.t.z);
-      vput(21, e, carry.area);
+      if (VERTS) {
+        vput(12, e, carry.p.x); vput(13, e, carry.p.y); vput(14, e, carry.p.z);
+        vput(15, e, carry.n.x); vput(16, e, carry.n.y); vput(17, e, carry.n.z);
+        vput(18, e, carry.t.x); vput(19, e, carry.t.y); vput(20, e, carry.t.z);
+        vput(21, e, carry.area);
+      }
     }
     nv += __popc(m);
     __syncwarp();
@@ -1466,16 +1479,16 @@ __global__ void __launch_bounds__(128, 2) k_adjoint_ext(WF w, const DevScene* __
             float3 none;
             for (int i = 0; i < w.nL; ++i) {
               const float rx = rng.next_float(), ry = rng.next_float();
-              light_sample_adj<true>(w, sc, xc, mp.color * kInvPi, rx, ry, rec_hit(w, s, d, i), adjC, ax, hot, none, &mp,
+              light_sample_adj<true, true>(w, sc, xc, mp.color * kInvPi, rx, ry, rec_hit(w, s, d, i), adjC, ax, hot, none, &mp,
                                      &ma);
             }
             for (int j = 0; j < w.nB; ++j) {
               const float rx = rng.next_float(), ry = rng.next_float();
-              bsdf_sample_adj<UNB, true>(w, sc, xc, mp.color * kInvPi, rx, ry, rec_hit(w, s, d, w.nL + j), adjC, ax, hot, none,
+              bsdf_sample_adj<UNB, true, true>(w, sc, xc, mp.color * kInvPi, rx, ry, rec_hit(w, s, d, w.nL + j), adjC, ax, hot, none,
                                          &mp, &ma);
             }
             const float rx = rng.next_float(), ry = rng.next_float();
-            const bool next = d < w.D - 1 && continuation_adj<UNB, true>(sc, xc, mp.color * kInvPi, rx, ry,
+            const bool next = d < w.D - 1 && continuation_adj<UNB, true, true>(sc, xc, mp.color * kInvPi, rx, ry,
                                                                          rec_hit(w, s, d, w.nL + w.nB), adjB, ax, nextc, nx, none, &mp, &ma);
             const float3 aorg = mat_finalize(ob, xc, mp, ma, ax);
             if (d == 0) cam.add(&V, aorg);
@@ -4093,15 +4106,15 @@ std::vector<std::vector<Tile>> schedule_tiles(const std::vector<Tile>& tiles, in
 
 // Interior adjoint of a tile: persistent blocks (their warps' work lists fill better over many
 // paths), as many as are resident.
-template <bool UNB>
+template <bool UNB, bool VERTS>
 static void launch_adjoint(const WF& w, const DevScene* scenes, const DevView* vd, const Tile& t, cudaStream_t st) {
   // fewer warps where many BSDF samples make the lists long (nB > 13)
   int warps = kAdjWarps;
   constexpr int kMost = 200 << 10;  // shared memory of a block
   while (warps > 1 && (int)sizeof(float) * warps * adj_warp_words(w.nB) > kMost) warps >>= 1;
   const int bytes = (int)sizeof(float) * warps * adj_warp_words(w.nB);
-  PSDR_CUDA(cudaFuncSetAttribute(k_adjoint<UNB>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
-  k_adjoint<UNB><<<grid_for(t.n, 32 * warps, 2), 32 * warps, bytes, st>>>(w, scenes, vd, t);
+  PSDR_CUDA(cudaFuncSetAttribute(k_adjoint<UNB, VERTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
+  k_adjoint<UNB, VERTS><<<grid_for(t.n, 32 * warps, 2), 32 * warps, bytes, st>>>(w, scenes, vd, t);
 }
 
 // Device work of one backward unit on workspace ws (views at vd); no allocation, no
@@ -4134,9 +4147,11 @@ void backward_unit(const DevScene* scenes_dev, const std::vector<DevView>& views
       if (unb) k_adjoint_ext<true><<<g, 128, 0, st>>>(w, scenes_dev, vd, t);
       else k_adjoint_ext<false><<<g, 128, 0, st>>>(w, scenes_dev, vd, t);
     } else if (unb) {
-      launch_adjoint<true>(w, scenes_dev, vd, t, st);
+      if (gi.verts) launch_adjoint<true, true>(w, scenes_dev, vd, t, st);
+      else launch_adjoint<true, false>(w, scenes_dev, vd, t, st);
     } else {
-      launch_adjoint<false>(w, scenes_dev, vd, t, st);
+      if (gi.verts) launch_adjoint<false, true>(w, scenes_dev, vd, t, st);
+      else launch_adjoint<false, false>(w, scenes_dev, vd, t, st);
     }
     PSDR_LAUNCHED(1);
     if (lens) {

@@ -146,6 +146,7 @@ void make_view(const psdr_camera_desc& c, int spp, DevView& v);
 void render_forward_impl(const DevScene* scenes_dev, std::vector<DevView>& views, const psdr_config& cfg,
                          psdr_workspace* ws, cudaStream_t st, float* samples_out, const KeptRecords* keep = nullptr);
 struct SceneGradInfo {
+  int verts = 1;  // the gradient of some mesh's or light's vertices is wanted
   int bsdf = 0;  // a DiffuseBsdfMaterial mesh or an environment light (extended adjoint kernel)
   int jump = 0;  // a DiffuseBsdfMaterial mesh: the unbiased default terms include its BRDF jumps
 };
