@@ -42,6 +42,21 @@ PSDR_D int warp_append(int* counter, bool pred) {
   return pred ? base + __popc(m & lanemask_lt()) : -1;
 }
 
+// Warp-aggregated append of n entries per lane: the lane's first entry. All lanes call it.
+PSDR_D int warp_reserve(int* counter, int n) {
+  const int lane = threadIdx.x & 31;
+  int sum = n;
+  for (int k = 1; k < 32; k <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, sum, k);
+    if (lane >= k) sum += v;
+  }
+  const int total = __shfl_sync(0xffffffffu, sum, 31);
+  if (total == 0) return 0;
+  int base = 0;
+  if (lane == 0) base = atomicAdd(counter, total);
+  return __shfl_sync(0xffffffffu, base, 0) + sum - n;
+}
+
 PSDR_D void xform_pos(const float* m, float3 p, float3& out) {
   const float w = m[12] * p.x + m[13] * p.y + m[14] * p.z + m[15];
   out = f3((m[0] * p.x + m[1] * p.y + m[2] * p.z + m[3]) / w, (m[4] * p.x + m[5] * p.y + m[6] * p.z + m[7]) / w,
@@ -172,8 +187,46 @@ __global__ void __launch_bounds__(256, MODE != MODE_FWD ? 4 : 1) k_camera(WF w, 
 }
 
 // ------------------------------------------------------------------ shade kernel
-// Hit-light test and all samples of one depth; rays are written to the shaded slot.
-template <int MODE, bool BSDF>
+// A MIS BSDF-sample ray counts only if it ends on a light (the accumulate and adjoint kernels
+// skip any other hit): the closest light triangle along it, by the traversal's test and tie
+// rule, bounds an occlusion query of k_trace, and a ray with no light along it (nineteen in
+// twenty under a small lamp) needs none. For lights of at most this many triangles in all.
+constexpr int kMisLightTris = 16;
+
+// Returns the bound of the query: the light's distance; < 0: no light along the ray; infinity: too
+// many light triangles, trace for the closest hit.
+PSDR_D float mis_light_bound(const DevScene& sc, float3 o, float3 d) {
+  int nlt = 0;
+  for (int l = 0; l < sc.nlight; ++l) nlt += sc.lights[l].ntri;
+  if (sc.nlight == 0 || nlt > kMisLightTris) return INFINITY;
+  const RayPre rp = ray_pre(o, d);
+  float tl = INFINITY;
+  int best = -1;
+  for (int l = 0; l < sc.nlight; ++l) {
+    const DevLight& Lt = sc.lights[l];
+    for (int t = Lt.tri0; t < Lt.tri0 + Lt.ntri; ++t) {
+      const float4* q = sc.tri + 6 * (size_t)t;
+      float tt, b1, b2;
+      if (tri_test(rp, xyz(__ldg(q)), xyz(__ldg(q + 1)), xyz(__ldg(q + 2)), kTmin, tl, tt, b1, b2) &&
+          (tt < tl || best < 0 || t < best)) {
+        tl = tt;
+        best = t;
+      }
+    }
+  }
+  return best < 0 ? -1.f : tl;
+}
+
+// Hit-light test and all samples of one depth; rays are written to the shaded slot. From
+// kListMin paths on, the BSDF-sample rays that need a traversal are listed (slots past
+// nL * cap, in ra[].y from slot nL * cap on, counted in cnt[2D+3]) and the others get their miss
+// here, where 32 lanes make the light test together; below, k_trace makes it as a lane takes
+// the ray, while the other rays of the warp wait. The test adds 6 us to a small launch of this
+// kernel, which is what k_trace saves on 2^18 paths (plain 128^2 x 16 spp render); 2^20 paths
+// of 256^2 x 16 spp: k_trace 595 -> 566 us for 11 us more here; 2^22 of 256^2 x 64 spp: 1.18 ->
+// 1.05 ms for 0.02.
+constexpr int kListMin = 1 << 19;
+template <int MODE, bool BSDF, bool LIST>
 __global__ void __launch_bounds__(256) k_shade(WF w, const DevScene* __restrict__ scenes,
                                                const DevView* __restrict__ views, int d) {
   const int* qin = (d & 1) ? w.q1 : w.q0;
@@ -206,16 +259,20 @@ __global__ void __launch_bounds__(256) k_shade(WF w, const DevScene* __restrict_
       }
     }
     const int k = warp_append(&w.cnt[2 * d + 1], go);
-    if (!go) continue;
-    w.qs[k] = s;
-    Rng rng{w.rs[s], w.ri[s]};
-    float3 mm;
-    bool mapped;
-    const float3 Ns = BSDF ? shading_normal(sc->objs[x.obj], x, mm, mapped) : x.n;
+    Rng rng{0, 0};
+    float3 Ns;
+    if (go) {
+      w.qs[k] = s;
+      rng.state = w.rs[s];
+      rng.inc = w.ri[s];
+      float3 mm;
+      bool mapped;
+      Ns = BSDF ? shading_normal(sc->objs[x.obj], x, mm, mapped) : x.n;
+    }
     // rays are stored type-major (slot r * cap + k): a warp of k_trace then traces
     // rays of one kind from neighbouring paths
     const size_t cs = (size_t)w.cap;
-    for (int i = 0; i < w.nL; ++i) {
+    for (int i = 0; go && i < w.nL; ++i) {
       const float rx = rng.next_float(), ry = rng.next_float();
       const LightSample ls = sample_light(*sc, rx, ry);
       const float3 dv = ls.y - x.p;
@@ -226,16 +283,31 @@ __global__ void __launch_bounds__(256) k_shade(WF w, const DevScene* __restrict_
       w.rd[slot] = make_float4(dir.x, dir.y, dir.z, __int_as_float(ls.light));
       w.ra[slot] = make_float4(ls.y.x, ls.y.y, ls.y.z, ls.pdf);
     }
+    unsigned listed = 0;  // samples to list (kMaxRays bounds them)
     for (int j = 0; j < w.nB; ++j) {
-      const float rx = rng.next_float(), ry = rng.next_float();
-      float ct, st, sp, cp;
-      const float3 wo = BSDF ? material_dir(x, Ns, rx, ry, ct, st, sp, cp) : diffuse_dir(x.n, x.t, rx, ry, ct, st, sp, cp);
-      const size_t slot = (w.nL + j) * cs + k;
-      w.ro[slot] = make_float4(x.p.x, x.p.y, x.p.z, INFINITY);
-      w.rd[slot] = make_float4(wo.x, wo.y, wo.z, 0.f);
-      w.ra[slot] = make_float4(ct, 0.f, 0.f, 0.f);
+      if (go) {
+        const float rx = rng.next_float(), ry = rng.next_float();
+        float ct, st, sp, cp;
+        const float3 wo =
+            BSDF ? material_dir(x, Ns, rx, ry, ct, st, sp, cp) : diffuse_dir(x.n, x.t, rx, ry, ct, st, sp, cp);
+        const float tl = LIST ? mis_light_bound(*sc, x.p, wo) : INFINITY;
+        const size_t slot = (w.nL + j) * cs + k;
+        if (!(tl < 0.f)) {
+          listed |= 1u << j;
+          w.ro[slot] = make_float4(x.p.x, x.p.y, x.p.z, tl);
+          w.rd[slot] = make_float4(wo.x, wo.y, wo.z, 0.f);
+          w.ra[slot].x = ct;
+        } else {
+          w.hit[slot] = make_float4(__int_as_float(-1), 0.f, 0.f, INFINITY);
+        }
+      }
     }
-    {
+    if (LIST) {
+      int i = warp_reserve(&w.cnt[2 * w.D + 3], __popc(listed));  // one atomic per warp
+      for (; listed; listed &= listed - 1)
+        w.ra[w.nL * cs + i++].y = __uint_as_float((unsigned)((__ffs(listed) - 1) * cs + k));
+    }
+    if (go) {
       const float rx = rng.next_float(), ry = rng.next_float();
       if (!last) {
         float ct, st, sp, cp;
@@ -246,8 +318,8 @@ __global__ void __launch_bounds__(256) k_shade(WF w, const DevScene* __restrict_
         w.rd[slot] = make_float4(wo.x, wo.y, wo.z, 0.f);
         w.ra[slot] = make_float4(ct, 0.f, 0.f, 0.f);
       }
+      w.rs[s] = rng.state;
     }
-    w.rs[s] = rng.state;
   }
 }
 
@@ -264,9 +336,6 @@ __global__ void __launch_bounds__(256) k_shade(WF w, const DevScene* __restrict_
 // waited for one another at leaves, trav_step), L1 33 % and L2 6 % of their peaks. Traversal
 // of the 512^2 x 32 spp icosphere step: 14.0 ms before, 12.2 ms now (2^20-path tiles).
 constexpr int kRefill = 16;
-// Lights of at most this many triangles in all let k_trace answer MIS BSDF-sample rays
-// with a light test and a bounded occlusion query.
-constexpr int kMisLightTris = 16;
 // Per-lane memory of k_trace: the first kShort stack entries, the ray as the triangle test
 // takes it and the hit's barycentrics live in shared memory (one column per lane, so a
 // warp's accesses hit 32 banks), which keeps them out of the registers of the node visits;
@@ -315,13 +384,16 @@ struct TraceMem {
   }
   PSDR_D int pop(int i) const { return i < kShort ? sh->stack[i][lane] : deep[i - kShort]; }
 };
+template <bool LIST>
 __global__ void __launch_bounds__(128, kTraceBlocks) k_trace(WF w, const DevScene* __restrict__ scenes,
                                                              const DevView* __restrict__ views, int d,
                                                              unsigned long long* __restrict__ ray_count) {
   const unsigned nk = (unsigned)w.cnt[2 * d + 1];
   const int Rd = (d == w.D - 1) ? w.R - 1 : w.R;
-  const unsigned total = nk * (unsigned)Rd;
-  if (ray_count && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(ray_count, (unsigned long long)total);
+  if (ray_count && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(ray_count, (unsigned long long)nk * Rd);
+  // the queue: light-sample rays, BSDF-sample rays (all or those k_shade listed), indirect rays
+  const unsigned n_light = nk * (unsigned)w.nL, n_list = n_light + (LIST ? (unsigned)w.cnt[2 * w.D + 3] : nk * (unsigned)w.nB);
+  const unsigned total = n_list + (d == w.D - 1 ? 0u : nk);
   unsigned* fetch = reinterpret_cast<unsigned*>(w.cnt + 2 * w.D + 2);
   __shared__ TraceShared sh;
   TraceMem mem;
@@ -349,45 +421,33 @@ __global__ void __launch_bounds__(128, kTraceBlocks) k_trace(WF w, const DevScen
       next = base + __popc(idle);
       const unsigned idx = base + __popc(idle & lanemask_lt());
       if (!open && idx < total) {
-        const unsigned r = idx / nk;
-        const unsigned k = idx - r * nk;
-        slot = (size_t)r * w.cap + k;
+        unsigned k;
+        if (idx < (LIST ? n_light : n_list)) {
+          const unsigned r = idx / nk;
+          k = idx - r * nk;
+          slot = (size_t)r * w.cap + k;
+        } else if (LIST && idx < n_list) {
+          const unsigned loc = __float_as_uint(w.ra[(size_t)w.nL * w.cap + (idx - n_light)].y);
+          k = loc % (unsigned)w.cap;
+          slot = (size_t)w.nL * w.cap + loc;
+        } else {
+          k = idx - n_list;
+          slot = (size_t)(w.nL + w.nB) * w.cap + k;
+        }
         sc = scenes + (w.one_scene >= 0 ? w.one_scene : views[w.view[w.qs[k]]].scene);
         const float4 o = w.ro[slot], dd = w.rd[slot];
-        const float t_occ = (int)r < w.nL ? (o.w - 4e-3f) / 1.0001f - 4e-3f : -INFINITY;
-        const RayPre rp = ray_pre(xyz(o), xyz(dd));
-        mem.set_ray(rp);
-        trav_begin(s, xyz(o), xyz(dd), o.w, t_occ, sc->ntri > 0 ? sc->root : kNoNode);
+        // a bounded ray stops at the first hit short of its light: a light sample's target, or
+        // the closest light triangle along a BSDF sample
+        float tmax = o.w;
+        if (!LIST && idx >= n_light && idx < n_list) tmax = mis_light_bound(*sc, xyz(o), xyz(dd));
+        const bool none = tmax < 0.f;
+        if (none) tmax = INFINITY;
+        const float t_occ = idx < n_light ? (tmax - 4e-3f) / 1.0001f - 4e-3f : (tmax < INFINITY ? tmax : -INFINITY);
+        mem.set_ray(ray_pre(xyz(o), xyz(dd)));
+        trav_begin(s, xyz(o), xyz(dd), tmax, t_occ, sc->ntri > 0 && !none ? sc->root : kNoNode);
         nodes = sc->nodes;
         leaf = sc->leaf;
         open = true;
-        if ((int)r >= w.nL && (int)r < w.nL + w.nB && sc->nlight > 0) {
-          // MIS BSDF-sample ray: only a light hit contributes (the shade, accumulate and
-          // adjoint kernels skip any other hit). The closest light triangle along the ray
-          // (the traversal's test and tie rule) bounds an occlusion query: a nearer hit is
-          // reported as a miss, and with no light along the ray nothing is traversed.
-          int nlt = 0;
-          for (int l = 0; l < sc->nlight; ++l) nlt += sc->lights[l].ntri;
-          if (nlt <= kMisLightTris) {
-            float tl = o.w;
-            int best = -1;
-            for (int l = 0; l < sc->nlight; ++l) {
-              const DevLight& Lt = sc->lights[l];
-              for (int t = Lt.tri0; t < Lt.tri0 + Lt.ntri; ++t) {
-                const float4* q = sc->tri + 6 * (size_t)t;
-                float tt, b1, b2;
-                if (tri_test(rp, xyz(__ldg(q)), xyz(__ldg(q + 1)), xyz(__ldg(q + 2)), kTmin, tl, tt, b1, b2) &&
-                    (tt < tl || best < 0 || t < best)) {
-                  tl = tt;
-                  best = t;
-                }
-              }
-            }
-            s.t = tl;
-            s.t_occ = tl;
-            if (best < 0) s.node = kNoNode;
-          }
-        }
       }
       continue;
     }
@@ -406,6 +466,7 @@ __global__ void __launch_bounds__(256) k_accum(WF w, const DevScene* __restrict_
                                                const DevView* __restrict__ views, int d) {
   const int n = w.cnt[2 * d + 1];
   int* qout = (d & 1) ? w.q0 : w.q1;
+  if (blockIdx.x == 0 && threadIdx.x == 0) w.cnt[2 * w.D + 3] = 0;  // listed rays of k_shade
   const int stride = gridDim.x * blockDim.x;
   const int n32 = (n + 31) & ~31;
   const bool last = d == w.D - 1;
@@ -3615,19 +3676,19 @@ static void launch_direct(const WF& w, cudaStream_t st, const DevScene* scenes, 
 // Zeroes the queue counters of a wavefront before a new set of paths enters its depth
 // loop (k_shade resets the ray fetch counter of k_trace itself).
 static void clear_counts(const WF& w, cudaStream_t st) {
-  PSDR_CUDA(cudaMemsetAsync(w.cnt, 0, sizeof(int) * 2 * (w.D + 1), st));
+  PSDR_CUDA(cudaMemsetAsync(w.cnt, 0, sizeof(int) * 2 * (w.D + 2), st));
 }
 
-template <int MODE>
+template <int MODE, bool LIST>
 static void depth_loop_t(WF& w, const DevScene* scenes, const DevView* views, cudaStream_t st) {
   const int cap = w.cap;
   Profiler& pf = profiler();
   for (int d = 0; d < w.D; ++d) {
     const int gs = grid_for(cap, 256, 8);
-    if (w.bsdf) k_shade<MODE, true><<<gs, 256, 0, st>>>(w, scenes, views, d);
-    else k_shade<MODE, false><<<gs, 256, 0, st>>>(w, scenes, views, d);
+    if (w.bsdf) k_shade<MODE, true, LIST><<<gs, 256, 0, st>>>(w, scenes, views, d);
+    else k_shade<MODE, false, LIST><<<gs, 256, 0, st>>>(w, scenes, views, d);
     pf.begin_trace(st);
-    k_trace<<<num_sms() * w.trace_bps, 128, 0, st>>>(w, scenes, views, d, pf.on ? pf.d_rays : nullptr);
+    k_trace<LIST><<<num_sms() * w.trace_bps, 128, 0, st>>>(w, scenes, views, d, pf.on ? pf.d_rays : nullptr);
     pf.end_trace(st);
     PSDR_LAUNCHED(3);
     if (w.bsdf) k_accum<MODE, true><<<gs, 256, 0, st>>>(w, scenes, views, d);
@@ -3636,10 +3697,16 @@ static void depth_loop_t(WF& w, const DevScene* scenes, const DevView* views, cu
   PSDR_CUDA(cudaGetLastError());
 }
 
-static void depth_loop(WF& w, const DevScene* scenes, const DevView* views, int mode, cudaStream_t st) {
-  if (mode == MODE_REPLAY) depth_loop_t<MODE_REPLAY>(w, scenes, views, st);
-  else if (mode == MODE_KEEP) depth_loop_t<MODE_KEEP>(w, scenes, views, st);
-  else depth_loop_t<MODE_FWD>(w, scenes, views, st);
+// n paths at most enter the loop.
+static void depth_loop(WF& w, const DevScene* scenes, const DevView* views, int mode, int n, cudaStream_t st) {
+  const bool list = n >= kListMin && w.nB > 0;
+  auto run = [&](auto m) {
+    if (list) depth_loop_t<m.value, true>(w, scenes, views, st);
+    else depth_loop_t<m.value, false>(w, scenes, views, st);
+  };
+  if (mode == MODE_REPLAY) run(std::integral_constant<int, MODE_REPLAY>{});
+  else if (mode == MODE_KEEP) run(std::integral_constant<int, MODE_KEEP>{});
+  else run(std::integral_constant<int, MODE_FWD>{});
 }
 
 template <int MODE>
@@ -3657,7 +3724,7 @@ static void run_tile(WF& w, const DevScene* scenes, const DevView* views, const 
   else if (mode == MODE_KEEP) launch_camera<MODE_KEEP>(w, scenes, views, tile, g, st);
   else launch_camera<MODE_FWD>(w, scenes, views, tile, g, st);
   PSDR_LAUNCHED(1);
-  depth_loop(w, scenes, views, mode, st);
+  depth_loop(w, scenes, views, mode, tile.n, st);
 }
 
 // Device bytes of a workspace per path of tile capacity (psdr_workspace::ensure).
@@ -3837,11 +3904,11 @@ static void edge_phase(WF w, const DevScene* scenes, const DevView* vd, int v, c
   if (pre) k_edge_init<true><<<grid_for(n, 256, 8), 256, 0, st>>>(w, scenes, vd, v, eb, begin, n, hc, round, 0);
   else k_edge_init<false><<<grid_for(n, 256, 8), 256, 0, st>>>(w, scenes, vd, v, eb, begin, n, hc, round, 0);
   PSDR_LAUNCHED(1);
-  depth_loop(w, scenes, vd, MODE_FWD, st);
+  depth_loop(w, scenes, vd, MODE_FWD, n, st);
   clear_counts(w, st);
   k_edge_mid<<<grid_for(n, 256, 8), 256, 0, st>>>(w, vd, v, eb, n);
   PSDR_LAUNCHED(1);
-  depth_loop(w, scenes, vd, MODE_FWD, st);
+  depth_loop(w, scenes, vd, MODE_FWD, n, st);
   if (pre) k_edge_final<true><<<grid_for(n, 256, 8), 256, 0, st>>>(w, scenes, vd, v, eb, begin, n, mass, spp);
   else k_edge_final<false><<<grid_for(n, 256, 8), 256, 0, st>>>(w, scenes, vd, v, eb, begin, n, mass, spp);
   PSDR_LAUNCHED(1);
@@ -3854,7 +3921,7 @@ static void edge_phase_unb(WF w, const DevScene* scenes, const DevView* vd, int 
   clear_counts(w, st);
   k_edge_init<false><<<grid_for(n, 256, 8), 256, 0, st>>>(w, scenes, vd, v, eb, begin, n, hc, 0, 1);
   PSDR_LAUNCHED(2);
-  depth_loop(w, scenes, vd, MODE_FWD, st);
+  depth_loop(w, scenes, vd, MODE_FWD, n, st);
   k_edge_final_unb<<<grid_for(n, 256, 8), 256, 0, st>>>(w, scenes, vd, v, eb, n, (float)hc.ncells, spp);
   PSDR_CUDA(cudaGetLastError());
 }
@@ -3866,7 +3933,7 @@ static void border_phase(WF w, const DevScene* scenes, const DevView* vd, int v,
   clear_counts(w, st);
   k_border_init<<<grid_for(n, 256, 8), 256, 0, st>>>(w, scenes, vd, v, eb, mw, mpre, S, begin, n, N);
   PSDR_LAUNCHED(2);
-  depth_loop(w, scenes, vd, MODE_FWD, st);
+  depth_loop(w, scenes, vd, MODE_FWD, n, st);
   k_border_final<<<grid_for(n, 256, 8), 256, 0, st>>>(w, scenes, vd, v, eb, n, N);
   if (lens) {
     k_lens_border<<<grid_for(n, 256, 8), 256, 0, st>>>(w, vd, v, eb, n, N);
@@ -3884,7 +3951,7 @@ static void indirect_phase(WF w, const DevScene* scenes, const DevView* vd, int 
   WF wy = w;
   wy.D = w.D - 1;  // the source y is the second vertex of the camera path
   wy.light_vis = 0;
-  depth_loop(wy, scenes, vd, MODE_FWD, st);
+  depth_loop(wy, scenes, vd, MODE_FWD, n, st);
   k_indirect_final<<<grid_for(n, 128, 16), 128, 0, st>>>(w, scenes, vd, v, eb, n, (float)hc.ncells, N);
   PSDR_LAUNCHED(1);
   PSDR_CUDA(cudaGetLastError());
@@ -3898,7 +3965,7 @@ static void crease_phase(WF w, const DevScene* scenes, const DevView* vd, int v,
   clear_counts(w, st);
   k_crease_init<<<grid_for(n, 256, 8), 256, 0, st>>>(w, scenes, vd, v, eb, cb, mw, mpre, begin, n, N);
   PSDR_LAUNCHED(1);
-  depth_loop(w, scenes, vd, MODE_FWD, st);
+  depth_loop(w, scenes, vd, MODE_FWD, n, st);
   k_crease_final<<<grid_for(n, 256, 8), 256, 0, st>>>(w, scenes, vd, v, eb, cb, n);
   PSDR_LAUNCHED(1);
   PSDR_CUDA(cudaGetLastError());
@@ -3931,7 +3998,7 @@ static void jump_phase(WF w, const DevScene* scenes, const DevView* vd, int v, c
     WF wk = w;
     wk.D = D - k;
     wk.light_vis = 0;
-    depth_loop(wk, scenes, vd, MODE_FWD, st);
+    depth_loop(wk, scenes, vd, MODE_FWD, n, st);
   }
   k_jump_final<<<grid_for(n, 256, 8), 256, 0, st>>>(w, scenes, vd, v, eb, n, k);
   PSDR_LAUNCHED(1);
