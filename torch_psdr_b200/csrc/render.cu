@@ -7,11 +7,11 @@
 //               with warp-aggregated compaction) -> k_trace (closest hit per ray)
 //               -> k_accum (NEE + MIS contributions, throughput, compaction)
 //   k_film    : per-pixel average of its spp paths (deterministic, no atomics).
-// Backward (Wrap2torch.backward + enoki reverse sweep, torch_psdr.py:48-72): the tile
-// is re-traced from the stored seeds recording only hit records, then k_adjoint
-// replays every path's sampler stream and applies the hand-written adjoint of the
-// estimator, scattering into fp64 accumulators (warp-aggregated where a warp shares
-// the target). Primary-edge (path_integrator.cc:188-272) and direct-edge (:274-353)
+// Backward (Wrap2torch.backward + enoki reverse sweep, torch_psdr.py:48-72): from the hit
+// records that the forward kept (or that re-tracing the tile from its seeds gives),
+// k_adjoint replays every path's sampler stream and applies the hand-written adjoint of
+// the estimator, scattering into fixed-point accumulators (warp-aggregated where a warp
+// shares the target). Primary-edge (path_integrator.cc:188-272) and direct-edge (:274-353)
 // boundary terms follow the reference formulas (PSDR_EST_REFERENCE).
 #include <algorithm>
 #include <cmath>
@@ -140,10 +140,10 @@ PSDR_D void vert_add(const DevScene& sc, int v, float3 a) {
 
 // ------------------------------------------------------------------ camera kernel
 // ORTHO: the instance for jobs with an orthographic view (it handles both camera types).
-// The replay instance is held to 4 blocks per SM (64 registers): its record writes
-// otherwise take it to 76 registers and 3 blocks.
+// 64 registers (8 blocks of 128 threads per SM): the record writes of the replay instances
+// otherwise take 76.
 template <int MODE, bool ORTHO>
-__global__ void __launch_bounds__(256, MODE != MODE_FWD ? 4 : 1) k_camera(WF w, const DevScene* __restrict__ scenes,
+__global__ void __launch_bounds__(128, 8) k_camera(WF w, const DevScene* __restrict__ scenes,
                                                 const DevView* __restrict__ views, Tile tile) {
   const int stride = gridDim.x * blockDim.x;
   const int n32 = (tile.n + 31) & ~31;
@@ -1631,7 +1631,7 @@ PSDR_D bool tri_has_edge(const DevScene& sc, int tri, int2 ev) {
 // (foreground); the path of the other side (background, possibly a miss) is traced,
 // and eb.hb keeps that background hit with flag 1 (background on the +eps side) or 2.
 template <bool PRE>
-__global__ void __launch_bounds__(256, 3) k_edge_init(WF w, const DevScene* __restrict__ scenes,
+__global__ void __launch_bounds__(128, 6) k_edge_init(WF w, const DevScene* __restrict__ scenes,
                                                    const DevView* __restrict__ views, int v, EdgeBuf eb,
                                                    long long begin, int n, HCube hc, int round, int unb) {
   const int stride = gridDim.x * blockDim.x;
@@ -1975,7 +1975,7 @@ PSDR_D long long border_locate(const double* __restrict__ w, const double* __res
   return lo;
 }
 
-__global__ void __launch_bounds__(256) k_border_init(WF w, const DevScene* __restrict__ scenes,
+__global__ void __launch_bounds__(128) k_border_init(WF w, const DevScene* __restrict__ scenes,
                                                      const DevView* __restrict__ views, int v, EdgeBuf eb,
                                                      const double* __restrict__ mw, const double* __restrict__ mpre,
                                                      long long S, long long begin, int n, long long N) {
@@ -2530,7 +2530,7 @@ PSDR_D CreasePt crease_point(const DevView& V, CreaseBuf cb, const double* mw, c
 // (tmin) in world units: closer to the crease, rays leaving one surface skip the other
 // within tmin and the rendered radiance there is not the image's limit at the crease.
 constexpr float kCreaseOffset = 5.f * kTmin;  // world units
-__global__ void __launch_bounds__(256) k_crease_init(WF w, const DevScene* __restrict__ scenes,
+__global__ void __launch_bounds__(128) k_crease_init(WF w, const DevScene* __restrict__ scenes,
                                                      const DevView* __restrict__ views, int v, EdgeBuf eb,
                                                      CreaseBuf cb, const double* __restrict__ mw,
                                                      const double* __restrict__ mpre, long long begin, int n,
@@ -2679,7 +2679,7 @@ __global__ void __launch_bounds__(256) k_crease_final(WF w, const DevScene* __re
 // hb = x_{k+1}'s hit; La = x_{k-1}'s hit (tri -1: the camera).
 constexpr unsigned long long kJumpStreams = 16;  // max_bounce <= 16
 
-__global__ void __launch_bounds__(256) k_jump_init(WF w, const DevScene* __restrict__ scenes,
+__global__ void __launch_bounds__(128) k_jump_init(WF w, const DevScene* __restrict__ scenes,
                                                    const DevView* __restrict__ views, int v, EdgeBuf eb,
                                                    long long begin, int n, int k, int D) {
   const int stride = gridDim.x * blockDim.x;
@@ -3401,6 +3401,15 @@ __global__ void k_grad_out(const GradAcc* __restrict__ acc, float* __restrict__ 
 
 // ================================================================== host side
 namespace {
+// per_sm caps the grid; kEachBlock leaves it uncapped. The kernels that trace a ray per thread
+// (k_camera and the *_init of the boundary terms) take a block per 128 samples: threads end
+// at very different times, and a grid of a few blocks per SM, each over several batches, ends
+// with most SMs waiting for their last blocks. k_camera 2.65 -> 2.03 ms (1.31 M triangles,
+// 1024^2 x 16 spp), k_edge_init 1.15 -> 1.02 and k_border_init 0.43 -> 0.37 ms (512^2 x 32 spp
+// step) against 8 blocks of 256 per SM. k_direct, whose queue is mostly shorter than its
+// launch, takes 64 blocks per SM (1.48 -> 1.33 ms against 16). k_shade and k_accum stay at 8:
+// every thread does the same work, and uncapped they take 10-15 % longer on a single job.
+constexpr int kEachBlock = 1 << 20;
 inline int grid_for(long long n, int threads, int per_sm) {
   const long long want = (n + threads - 1) / threads;
   const long long cap = (long long)num_sms() * per_sm;
@@ -3665,7 +3674,7 @@ static void launch_direct(const WF& w, cudaStream_t st, const DevScene* scenes, 
     const int nb = (int)std::min<long long>(chunk, n - b);
     PSDR_CUDA(cudaMemsetAsync(w.cnt, 0, sizeof(int), st));
     k_direct_pick<PRE, UNB><<<grid_for(nb, 256, 8), 256, 0, st>>>(w, scenes, vd, v, b, nb, hc, round0);
-    const int g = grid_for(nb, 128, 16);
+    const int g = grid_for(nb, 128, 64);
     if (w.bsdf) k_direct<PRE, UNB, true><<<g, 128, 0, st>>>(w, scenes, vd, v, b, hc, round0, mass, spp);
     else k_direct<PRE, UNB, false><<<g, 128, 0, st>>>(w, scenes, vd, v, b, hc, round0, mass, spp);
     PSDR_LAUNCHED(2);
@@ -3712,14 +3721,14 @@ static void depth_loop(WF& w, const DevScene* scenes, const DevView* views, int 
 template <int MODE>
 static void launch_camera(const WF& w, const DevScene* scenes, const DevView* views, const Tile& tile, int g,
                           cudaStream_t st) {
-  if (w.ortho) k_camera<MODE, true><<<g, 256, 0, st>>>(w, scenes, views, tile);
-  else k_camera<MODE, false><<<g, 256, 0, st>>>(w, scenes, views, tile);
+  if (w.ortho) k_camera<MODE, true><<<g, 128, 0, st>>>(w, scenes, views, tile);
+  else k_camera<MODE, false><<<g, 128, 0, st>>>(w, scenes, views, tile);
 }
 
 static void run_tile(WF& w, const DevScene* scenes, const DevView* views, const Tile& tile, int mode,
                      cudaStream_t st) {
   clear_counts(w, st);
-  const int g = grid_for(tile.n, 256, 8);
+  const int g = grid_for(tile.n, 128, kEachBlock);
   if (mode == MODE_REPLAY) launch_camera<MODE_REPLAY>(w, scenes, views, tile, g, st);
   else if (mode == MODE_KEEP) launch_camera<MODE_KEEP>(w, scenes, views, tile, g, st);
   else launch_camera<MODE_FWD>(w, scenes, views, tile, g, st);
@@ -3901,8 +3910,8 @@ void render_forward_impl(const DevScene* scenes_dev, std::vector<DevView>& views
 static void edge_phase(WF w, const DevScene* scenes, const DevView* vd, int v, const EdgeBuf& eb, long long begin,
                        int n, const HCube& hc, int round, bool pre, float* mass, int spp, cudaStream_t st) {
   clear_counts(w, st);
-  if (pre) k_edge_init<true><<<grid_for(n, 256, 8), 256, 0, st>>>(w, scenes, vd, v, eb, begin, n, hc, round, 0);
-  else k_edge_init<false><<<grid_for(n, 256, 8), 256, 0, st>>>(w, scenes, vd, v, eb, begin, n, hc, round, 0);
+  if (pre) k_edge_init<true><<<grid_for(n, 128, kEachBlock), 128, 0, st>>>(w, scenes, vd, v, eb, begin, n, hc, round, 0);
+  else k_edge_init<false><<<grid_for(n, 128, kEachBlock), 128, 0, st>>>(w, scenes, vd, v, eb, begin, n, hc, round, 0);
   PSDR_LAUNCHED(1);
   depth_loop(w, scenes, vd, MODE_FWD, n, st);
   clear_counts(w, st);
@@ -3919,7 +3928,7 @@ static void edge_phase(WF w, const DevScene* scenes, const DevView* vd, int v, c
 static void edge_phase_unb(WF w, const DevScene* scenes, const DevView* vd, int v, const EdgeBuf& eb,
                            long long begin, int n, const HCube& hc, int spp, cudaStream_t st) {
   clear_counts(w, st);
-  k_edge_init<false><<<grid_for(n, 256, 8), 256, 0, st>>>(w, scenes, vd, v, eb, begin, n, hc, 0, 1);
+  k_edge_init<false><<<grid_for(n, 128, kEachBlock), 128, 0, st>>>(w, scenes, vd, v, eb, begin, n, hc, 0, 1);
   PSDR_LAUNCHED(2);
   depth_loop(w, scenes, vd, MODE_FWD, n, st);
   k_edge_final_unb<<<grid_for(n, 256, 8), 256, 0, st>>>(w, scenes, vd, v, eb, n, (float)hc.ncells, spp);
@@ -3931,7 +3940,7 @@ static void border_phase(WF w, const DevScene* scenes, const DevView* vd, int v,
                          const double* mw, const double* mpre, long long S, long long begin, int n, long long N,
                          bool lens, cudaStream_t st) {
   clear_counts(w, st);
-  k_border_init<<<grid_for(n, 256, 8), 256, 0, st>>>(w, scenes, vd, v, eb, mw, mpre, S, begin, n, N);
+  k_border_init<<<grid_for(n, 128, kEachBlock), 128, 0, st>>>(w, scenes, vd, v, eb, mw, mpre, S, begin, n, N);
   PSDR_LAUNCHED(2);
   depth_loop(w, scenes, vd, MODE_FWD, n, st);
   k_border_final<<<grid_for(n, 256, 8), 256, 0, st>>>(w, scenes, vd, v, eb, n, N);
@@ -3946,7 +3955,7 @@ static void border_phase(WF w, const DevScene* scenes, const DevView* vd, int v,
 static void indirect_phase(WF w, const DevScene* scenes, const DevView* vd, int v, const EdgeBuf& eb,
                            long long begin, int n, const HCube& hc, long long N, cudaStream_t st) {
   clear_counts(w, st);
-  k_indirect<false><<<grid_for(n, 128, 16), 128, 0, st>>>(w, scenes, vd, v, eb, begin, n, hc, 0, nullptr);
+  k_indirect<false><<<grid_for(n, 128, kEachBlock), 128, 0, st>>>(w, scenes, vd, v, eb, begin, n, hc, 0, nullptr);
   PSDR_LAUNCHED(1);
   WF wy = w;
   wy.D = w.D - 1;  // the source y is the second vertex of the camera path
@@ -3963,7 +3972,7 @@ static void crease_phase(WF w, const DevScene* scenes, const DevView* vd, int v,
                          const CreaseBuf& cb, const double* mw, const double* mpre, long long begin, int n,
                          long long N, cudaStream_t st) {
   clear_counts(w, st);
-  k_crease_init<<<grid_for(n, 256, 8), 256, 0, st>>>(w, scenes, vd, v, eb, cb, mw, mpre, begin, n, N);
+  k_crease_init<<<grid_for(n, 128, kEachBlock), 128, 0, st>>>(w, scenes, vd, v, eb, cb, mw, mpre, begin, n, N);
   PSDR_LAUNCHED(1);
   depth_loop(w, scenes, vd, MODE_FWD, n, st);
   k_crease_final<<<grid_for(n, 256, 8), 256, 0, st>>>(w, scenes, vd, v, eb, cb, n);
@@ -3992,7 +4001,7 @@ static void jump_phase(WF w, const DevScene* scenes, const DevView* vd, int v, c
                        int n, int k, cudaStream_t st) {
   const int D = w.D;
   clear_counts(w, st);
-  k_jump_init<<<grid_for(n, 256, 8), 256, 0, st>>>(w, scenes, vd, v, eb, begin, n, k, D);
+  k_jump_init<<<grid_for(n, 128, kEachBlock), 128, 0, st>>>(w, scenes, vd, v, eb, begin, n, k, D);
   PSDR_LAUNCHED(1);
   if (k < D) {
     WF wk = w;
@@ -4312,7 +4321,7 @@ void backward_unit(const DevScene* scenes_dev, const std::vector<DevView>& views
       HCube pre{};
       for (int k = 0; k < 3; ++k) { pre.res[k] = r3[k]; pre.unit[k] = 1.0f / (float)r3[k]; }
       for (int r = 0; r < cfg.secondary_edge_preprocess_rounds; ++r) {
-        k_indirect<true><<<grid_for(cells, 128, 16), 128, 0, st>>>(w, scenes_dev, vd, v, eb, 0, cells, pre, r,
+        k_indirect<true><<<grid_for(cells, 128, kEachBlock), 128, 0, st>>>(w, scenes_dev, vd, v, eb, 0, cells, pre, r,
                                                                    ws->mass.as<float>());
         PSDR_LAUNCHED(1);
       }
