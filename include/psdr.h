@@ -147,12 +147,12 @@ typedef struct {
                           backward the interior tiles and every boundary term of every view
                           (1..8, 0 = 4; psdr_render_* run them one after another). Gradients
                           are bitwise the same for every value. */
-  int32_t batch_records; /* ABI 6: psdr_batch_*: the forward keeps the replay records of
+  int32_t batch_records; /* ABI 6: psdr_batch_* (and the Python renderD): the forward keeps the replay records of
                             every interior path (16 B x (1 + D x R + 2 D) + 8 B per path, D =
                             max_bounce, R = light + BSDF samples + 1) and the backward runs the
                             adjoint from them instead of re-tracing the paths. 0 = when they
-                            fit in a quarter of the device memory free at psdr_batch_create,
-                            1 = always, -1 = never (re-trace, memory O(tile)). Gradients are
+                            fit in a quarter of the free device memory (a batch asks at
+                            psdr_batch_create), 1 = always, -1 = never (re-trace, memory O(tile)). Gradients are
                             bitwise the same either way. */
 } psdr_config;
 
@@ -235,8 +235,8 @@ PSDR_API psdr_status psdr_index_bounds(const int32_t* const* buffers, const int6
 /* Closest hit for n rays (device, 8 floats per ray: ox oy oz tmin dx dy dz tmax).
  * Outputs the global triangle id (-1 on miss), OptiX-convention barycentrics
  * (weights of p1, p2) and t. brute_force 1 tests every triangle (the KAT path); 2 runs
- * the resumable traversal of the wavefront closest-hit kernel instead of the one-shot
- * traversal of 0 (both must return brute force's hits). 
+ * the traversal with the stack and ray memory of the wavefront closest-hit kernel instead
+ * of the one of 0 (both must return brute force's hits).
  * Replaces SceneOptix::hit (scene_optix.cc:240-277) + device_programs.cu:13-47. */
 PSDR_API psdr_status psdr_intersect(psdr_scene* scene, const float* rays, int64_t n, int32_t* tri, float* bary,
                            float* t, int32_t brute_force, void* stream);
