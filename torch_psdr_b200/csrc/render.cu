@@ -331,9 +331,10 @@ __global__ void __launch_bounds__(256) k_shade(WF w, const DevScene* __restrict_
 // of a warp differ in traversal length by an order of magnitude) and the ray set-up runs on
 // at least half a warp. The fetch counter is w.cnt[2D+2], reset by k_shade.
 //
-// Bound by instruction issue and divergence, not by memory: on 512^2 x 8 spp rays of the
-// icosphere scene the SMs issue 64 % of the cycles with 14 of 32 lanes active (11 before lanes
-// waited for one another at leaves, trav_step), L1 33 % and L2 6 % of their peaks. Traversal
+// Bound by instruction issue and divergence, not by memory: on 256^2 x 32 spp rays of the
+// icosphere scene the SMs issue on 79 % of the cycles with 18.8 of 32 lanes active at the first
+// depth, 68 % and 16 at the third (11 before lanes waited for one another at leaves,
+// trav_step); L1 64-82 %, L2 12-18 %, DRAM 2-3 % of their peaks. Traversal
 // of the 512^2 x 32 spp icosphere step: 14.0 ms before, 12.2 ms now (2^20-path tiles).
 constexpr int kRefill = 16;
 // Per-lane memory of k_trace: the first kShort stack entries, the ray as the triangle test
@@ -1263,9 +1264,9 @@ __host__ __device__ constexpr int adj_warp_words(int nB) { return kVertFields * 
 // each path to its end instead (one thread per path over all depths) ran every depth's code
 // for the few paths still alive, and the BSDF-sample code for two lanes of a warp on average:
 // 5.8 ms per 512^2 x 32 spp x depth 3 step against 2.9 ms with lists; 2.3 ms with the warps of a
-// block starting together. Bound by instruction fetch (7.2 of 18.3 cycles per issued
-// instruction before that, 25 % occupancy at 128 registers) and by the latency of its record
-// loads; DRAM 7 % busy.
+// block starting together. Bound by the latency of its record loads (6.4 cycles per issued
+// instruction at 24 % occupancy, 128 registers; DRAM 8 % busy); instruction fetch is down from
+// 7.2 cycles to 1.0, for 3.3 at the block's barrier.
 // Without vertex gradients (VERTS false: texture and emission optimisation) the lists carry no
 // surface adjoint and the vertex scatters go; 256^2 x 64 spp: 0.83 -> 0.55 ms (three blocks per
 // SM spill: 0.63 ms).
