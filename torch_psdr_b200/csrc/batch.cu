@@ -185,23 +185,23 @@ PSDR_API psdr_status psdr_batch_create(psdr_scene* const* scenes, int32_t n_scen
     }
     const int rec_needed = b->backward && !b->kept ? 1 : 0;
     b->ws.ensure(b->cap, Rmax, cfg->max_bounce, n_cams, rec_needed, st);
-    bool jump = false;
-    for (int i = 0; i < n_scenes; ++i) jump = jump || scenes[i]->has_bsdf;
-    if (b->backward) ensure_border(&b->ws, *cfg, b->views, jump, b->cap, st);
+    for (int i = 0; i < n_scenes; ++i) {
+      if (scenes[i]->has_bsdf || scenes[i]->env_light >= 0) b->gi.bsdf = 1;
+      if (scenes[i]->has_bsdf) b->gi.jump = 1;
+    }
+    if (b->backward) ensure_border(&b->ws, *cfg, b->views, b->gi, b->cap, st);
     upload_views(&b->ws, b->views, st);
     // lanes: no more than the job has independent parts
     {
-      SceneGradInfo any;
-      any.bsdf = any.jump = 1;
       const size_t parts = std::max(plan_tiles(b->views, b->cap).size(),
-                                    b->backward ? backward_units(b->views, *cfg, b->cap, any).size() : (size_t)1);
+                                    b->backward ? backward_units(b->views, *cfg, b->cap, b->gi).size() : (size_t)1);
       b->nlanes = (int)std::min<size_t>(cfg->batch_lanes > 0 ? cfg->batch_lanes : 4, parts);
     }
     for (int k = 1; k < b->nlanes; ++k) {
       b->lane_ws.emplace_back(new psdr_workspace());
       psdr_workspace* lw = b->lane_ws.back().get();
       lw->ensure(b->cap, Rmax, cfg->max_bounce, 1, rec_needed, st);
-      if (b->backward) ensure_border(lw, *cfg, b->views, jump, b->cap, st);
+      if (b->backward) ensure_border(lw, *cfg, b->views, b->gi, b->cap, st);
       cudaStream_t ls = nullptr;
       PSDR_CUDA(cudaStreamCreateWithFlags(&ls, cudaStreamNonBlocking));
       b->lane_st.push_back(ls);
@@ -244,12 +244,7 @@ PSDR_API psdr_status psdr_batch_create(psdr_scene* const* scenes, int32_t n_scen
     }
     b->scenes_dev.alloc(sizeof(DevScene) * n_scenes, st);
     PSDR_CUDA(cudaMemcpyAsync(b->scenes_dev.p, ds.data(), sizeof(DevScene) * n_scenes, cudaMemcpyHostToDevice, st));
-    if (n_scenes == 1) b->gi = grad_info(scenes[0]);
-    b->ws.bsdf = 0;
-    for (int i = 0; i < n_scenes; ++i) {
-      if (scenes[i]->has_bsdf || scenes[i]->env_light >= 0) b->gi.bsdf = b->ws.bsdf = 1;
-      if (scenes[i]->has_bsdf) b->gi.jump = 1;
-    }
+    b->ws.bsdf = b->gi.bsdf;
     for (auto& lw : b->lane_ws) lw->bsdf = b->ws.bsdf;
     b->gi.verts = 0;
     for (int i = 0; b->backward && i < n_scenes; ++i)

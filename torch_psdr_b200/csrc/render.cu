@@ -4019,26 +4019,26 @@ long long border_segments(const DevView& V) {
   return (long long)(V.W + 1) * V.H + (long long)V.W * (V.H + 1);
 }
 
-// Buffers of the boundary terms, sized for the job: the side buffers for the samples a tile of
-// `cap` holds at most (jump: the BSDF-jump term, one sample per path, is among the terms), the
-// masses and prefix sums for the guides' cells and the border segments.
-void ensure_border(psdr_workspace* ws, const psdr_config& cfg, const std::vector<DevView>& views, bool jump, int cap,
-                   cudaStream_t st) {
+// Indirect shadow-boundary samples of a view.
+static long long indirect_samples(const DevView& V, const psdr_config& cfg) {
+  return std::max(1LL, (long long)V.H * V.W * cfg.spp_secondary_edge / kIndirectSampleDiv);
+}
+
+// Buffers of the boundary terms, sized for the job: the side buffers for the largest launch of
+// its units (a tile of `cap` samples at most), the masses and prefix sums for the guides' cells
+// and the border segments.
+void ensure_border(psdr_workspace* ws, const psdr_config& cfg, const std::vector<DevView>& views,
+                   const SceneGradInfo& gi, int cap, cudaStream_t st) {
   const bool unb = cfg.estimator == PSDR_EST_UNBIASED;
   const int* r3 = cfg.secondary_edge_hypercube_resolution;
   const long long cells1 = cfg.primary_edge_hypercube_resolution, cells2 = (long long)r3[0] * r3[1] * r3[2];
   const int rounds = std::min(kGuideRounds, cfg.secondary_edge_preprocess_rounds * (unb ? kDirectGuideRounds : 1));
-  long long samples = cells1, mass = std::max(cells1, cells2);
-  for (const DevView& v : views) {
-    const long long px = (long long)v.H * v.W;
-    samples = std::max(samples, px * cfg.spp_primary_edge);
-    if (!unb) continue;
-    const long long S = border_segments(v);
-    samples = std::max({samples, S * cfg.spp_pixel_boundary, (long long)kCreaseSamplesPerSpp * cfg.spp_primary_edge,
-                        px * cfg.spp_secondary_edge / kIndirectSampleDiv + 1, jump ? px * v.spp : 0});
-    mass = std::max({mass, S, (long long)kCreaseCap, (long long)v.scene_ntri});
-  }
-  const size_t n = (size_t)std::min<long long>(samples, cap);
+  long long samples = 0, mass = std::max(cells1, cells2);
+  for (const BwdUnit& u : backward_units(views, cfg, cap, gi)) samples = std::max(samples, u.samples);
+  for (const DevView& v : views)
+    if (unb) mass = std::max({mass, border_segments(v), (long long)kCreaseCap, (long long)v.scene_ntri});
+  ws->eb_cap = std::max(ws->eb_cap, std::min<long long>(samples, cap));
+  const size_t n = (size_t)ws->eb_cap;
   ws->eb_a.alloc(16 * n, st);
   ws->eb_n.alloc(16 * n, st);
   ws->eb_hb.alloc(16 * n, st);
@@ -4089,7 +4089,7 @@ void render_backward_impl(const DevScene* scenes_dev, std::vector<DevView>& view
   const int cap = choose_cap(cfg, views, true, 1, ws, keep == nullptr);
   const int Rmax = cfg.mis_light_samples + std::max(cfg.mis_bsdf_samples, 1) + 1;
   ws->ensure(cap, Rmax, cfg.max_bounce, (int)views.size(), keep ? 0 : 1, st);
-  ensure_border(ws, cfg, views, gi.jump != 0, cap, st);
+  ensure_border(ws, cfg, views, gi, cap, st);
   upload_views(ws, views, st);
   backward_launch(scenes_dev, views, cfg, cap, ws, gi, st, keep);
 }
@@ -4115,39 +4115,45 @@ std::vector<BwdUnit> backward_units(const std::vector<DevView>& views, const psd
   const double R = cfg.mis_light_samples + cfg.mis_bsdf_samples + 1;
   const double R1 = cfg.mis_light_samples + 2;  // boundary paths of the reference estimator: one BSDF sample
   if (terms & 1)
-    for (const Tile& t : plan_tiles(views, cap)) u.push_back(BwdUnit{1, -1, t, 2.0 * t.n * (1 + D * R)});
+    for (const Tile& t : plan_tiles(views, cap)) u.push_back(BwdUnit{1, -1, t, 2.0 * t.n * (1 + D * R), 0});
   for (int v = 0; v < (int)views.size(); ++v) {
     const DevView& V = views[v];
     const double px = (double)V.H * V.W;
+    const long long npx = (long long)V.H * V.W;
     if (terms & 2) {
       const double pre = (double)cfg.primary_edge_hypercube_resolution * cfg.primary_edge_preprocess_rounds *
                          2.0 * (1 + D * R1);
       const double n = px * cfg.spp_primary_edge * (unb ? 2 + D * R : 2.0 * (1 + D * R1));
-      u.push_back(BwdUnit{2, v, Tile{}, pre + n});
+      u.push_back(BwdUnit{2, v, Tile{}, pre + n,
+                          std::max<long long>(cfg.primary_edge_hypercube_resolution, npx * cfg.spp_primary_edge)});
     }
     if (terms & 4) {
       const int* r3 = cfg.secondary_edge_hypercube_resolution;
       const double per = unb ? 3.0 + 2.0 * (D - 1) : 3.0;
       const double pre = (double)r3[0] * r3[1] * r3[2] * cfg.secondary_edge_preprocess_rounds *
                          (unb ? kDirectGuideRounds : 1) * per;
-      u.push_back(BwdUnit{4, v, Tile{}, pre + px * cfg.spp_secondary_edge * per});
+      u.push_back(BwdUnit{4, v, Tile{}, pre + px * cfg.spp_secondary_edge * per, 0});
     }
     if (unb && (terms & 8) && cfg.spp_pixel_boundary > 0 && V.dimage)
-      u.push_back(BwdUnit{8, v, Tile{}, (double)border_segments(V) * cfg.spp_pixel_boundary * (1 + D * R)});
+      u.push_back(BwdUnit{8, v, Tile{}, (double)border_segments(V) * cfg.spp_pixel_boundary * (1 + D * R),
+                          border_segments(V) * cfg.spp_pixel_boundary});
     if (unb && (terms & 64) && V.dimage && !V.ortho && cfg.max_bounce >= 2) {
       const int* rs = cfg.secondary_edge_hypercube_resolution;
       const double cells = (double)std::max(1, rs[0] / kIndirectCellDiv) * rs[1] * rs[2];
-      const double n = std::max(1.0, px * cfg.spp_secondary_edge / kIndirectSampleDiv);
+      const double n = (double)indirect_samples(V, cfg);
       u.push_back(BwdUnit{64, v, Tile{}, (cells * cfg.secondary_edge_preprocess_rounds + n) * 3.0 +
-                                             n * (D - 1) * R});
+                                             n * (D - 1) * R,
+                          indirect_samples(V, cfg)});
     }
     if (unb && (terms & 32) && V.dimage && !V.ortho)
       u.push_back(BwdUnit{32, v, Tile{}, 8.0 * V.scene_ntri +
-                                             (double)cfg.spp_primary_edge * kCreaseSamplesPerSpp * 2.0 * (1 + D * R)});
-    if (unb && (terms & 16) && gi.bsdf && V.dimage) {
+                                             (double)cfg.spp_primary_edge * kCreaseSamplesPerSpp * 2.0 * (1 + D * R),
+                          (long long)cfg.spp_primary_edge * kCreaseSamplesPerSpp});
+    // (without a DiffuseBsdfMaterial mesh the term is zero)
+    if (unb && (terms & 16) && gi.jump && V.dimage) {
       double c = 0.0;
       for (int k = 1; k <= cfg.max_bounce; ++k) c += k + 1 + (D - k) * R;
-      u.push_back(BwdUnit{16, v, Tile{}, px * V.spp * c});
+      u.push_back(BwdUnit{16, v, Tile{}, px * V.spp * c, npx * V.spp});
     }
   }
   return u;
@@ -4172,7 +4178,7 @@ std::vector<std::vector<BwdUnit>> schedule_units(const std::vector<BwdUnit>& uni
 
 std::vector<std::vector<Tile>> schedule_tiles(const std::vector<Tile>& tiles, int lanes) {
   std::vector<BwdUnit> u;
-  for (const Tile& t : tiles) u.push_back(BwdUnit{1, -1, t, (double)t.n});
+  for (const Tile& t : tiles) u.push_back(BwdUnit{1, -1, t, (double)t.n, 0});
   std::vector<std::vector<Tile>> out;
   for (const auto& l : schedule_units(u, lanes)) {
     out.emplace_back();
@@ -4240,6 +4246,7 @@ void backward_unit(const DevScene* scenes_dev, const std::vector<DevView>& views
     return;
   }
   // ---- boundary terms of view v
+  PSDR_CHECK(std::min<long long>(u.samples, cap) <= ws->eb_cap, "a boundary term has more samples than side buffers");
   WF w = ws->wf;
   w.cap = ws->cap;
   set_wf(w, cfg, (int)views.size(), 1, 0);
@@ -4327,7 +4334,7 @@ void backward_unit(const DevScene* scenes_dev, const std::vector<DevView>& views
         PSDR_LAUNCHED(1);
       }
       const HCube hc = build_hcube(ws, cells, r3, 3, true, st);
-      const long long N = std::max(1LL, (long long)V.H * V.W * cfg.spp_secondary_edge / kIndirectSampleDiv);
+      const long long N = indirect_samples(V, cfg);
       for (long long b0 = 0; b0 < N; b0 += cap)
         indirect_phase(wi, scenes_dev, vd, v, eb, b0, (int)std::min<long long>(cap, N - b0), hc, N, st);
       break;

@@ -111,6 +111,7 @@ struct psdr_workspace {
   psdr::DBuf campos_acc, lens_acc;
   psdr::DBuf crease;  // interpenetration segments (unbiased estimator): kCreaseCap records + count
   long long mass_cap = 0;
+  long long eb_cap = 0;  // entries of eb_a, eb_n, eb_hb and eb_La
   // a DiffuseBsdfMaterial mesh or an environment light is in the scenes of the current job
   // (each entry point sets it; the extended kernel instances also handle the plain
   // scenes, so 1 is always safe)
@@ -148,7 +149,7 @@ void render_forward_impl(const DevScene* scenes_dev, std::vector<DevView>& views
 struct SceneGradInfo {
   int verts = 1;  // the gradient of some mesh's or light's vertices is wanted
   int bsdf = 0;  // a DiffuseBsdfMaterial mesh or an environment light (extended adjoint kernel)
-  int jump = 0;  // a DiffuseBsdfMaterial mesh: the unbiased default terms include its BRDF jumps
+  int jump = 0;  // a DiffuseBsdfMaterial mesh: its BRDF jumps are among the unbiased terms
 };
 void render_backward_impl(const DevScene* scenes_dev, std::vector<DevView>& views, const psdr_config& cfg,
                           psdr_workspace* ws, const SceneGradInfo& gi, cudaStream_t st,
@@ -178,6 +179,9 @@ struct BwdUnit {
   int view;      // boundary terms: the view
   Tile tile;     // interior: the tile
   double cost;   // relative device work (rays traced), for scheduling
+  // boundary terms: samples of its largest launch that keeps side data (EdgeBuf), one entry
+  // each; a launch takes at most a tile of them
+  long long samples;
 };
 std::vector<BwdUnit> backward_units(const std::vector<DevView>& views, const psdr_config& cfg, int cap,
                                     const SceneGradInfo& gi);
@@ -208,8 +212,8 @@ constexpr int kLensAcc = 12;  // accumulators per view: S0, Sx, Sy, B (3x3)
 // out[10] (fp32, overwritten or accumulated) from a view's accumulators.
 void lens_out(const GradAcc* acc, const LensChain& ch, float* out, int accumulate, cudaStream_t st);
 long long border_segments(const DevView& V);
-void ensure_border(psdr_workspace* ws, const psdr_config& cfg, const std::vector<DevView>& views, bool jump, int cap,
-                   cudaStream_t st);
+void ensure_border(psdr_workspace* ws, const psdr_config& cfg, const std::vector<DevView>& views,
+                   const SceneGradInfo& gi, int cap, cudaStream_t st);
 // Views of a backward job: their scene triangle counts (DevView::scene_ntri), before ensure_border.
 void set_scene_ntri(std::vector<DevView>& views, const psdr_scene* const* scenes);
 }  // namespace psdr
