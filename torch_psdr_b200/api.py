@@ -43,18 +43,20 @@ def check_indices(idx: Tensor, n: int, what: str) -> None:
 
 def _check_index_buffers(jobs) -> None:
     """check_indices for the (int32 CUDA tensor, bound, name) triples of one object, with one
-    kernel and one host read for all of them."""
+    kernel and one host read for all of them, on the GPU that holds them (which need not be
+    the current one)."""
     jobs = [j for j in jobs if j[0].numel()]
-    n = len(jobs)
-    if n == 0:
-        return
-    ptrs = (C.c_void_p * n)(*[t.data_ptr() for t, _, _ in jobs])
-    counts = (C.c_int64 * n)(*[t.numel() for t, _, _ in jobs])
-    out = (C.c_int32 * (2 * n))()
-    L.check(L.load().psdr_index_bounds(ptrs, counts, n, out, _stream()), "psdr_index_bounds")
-    for i, (_, bound, what) in enumerate(jobs):
-        if out[2 * i] < 0 or out[2 * i + 1] >= bound:
-            raise ValueError(f"{what} must lie in [0, {bound}): found values in [{out[2 * i]}, {out[2 * i + 1]}]")
+    for dev in dict.fromkeys(t.device for t, _, _ in jobs):
+        own = [j for j in jobs if j[0].device == dev]
+        n = len(own)
+        ptrs = (C.c_void_p * n)(*[t.data_ptr() for t, _, _ in own])
+        counts = (C.c_int64 * n)(*[t.numel() for t, _, _ in own])
+        out = (C.c_int32 * (2 * n))()
+        with torch.cuda.device(dev):
+            L.check(L.load().psdr_index_bounds(ptrs, counts, n, out, _stream()), "psdr_index_bounds")
+        for i, (_, bound, what) in enumerate(own):
+            if out[2 * i] < 0 or out[2 * i + 1] >= bound:
+                raise ValueError(f"{what} must lie in [0, {bound}): found values in [{out[2 * i]}, {out[2 * i + 1]}]")
 
 
 def _stream():
