@@ -54,3 +54,27 @@ def test_index_check_runs_on_the_gpu_of_the_buffers(monkeypatch):
     assert len(calls) == 3 and all(of == on and stream == on.index for of, on, stream in calls)
     with pytest.raises(ValueError, match=r"uv_indices must lie in \[0, 3\): found values in \[0, 3\]"):
         api._check_index_buffers([(f, 3, "face_indices"), (u, 3, "uv_indices")])
+
+
+def _scene_of(buffers):
+    """A Scene without its native part, over these internal texture buffers."""
+    scene = api.Scene.__new__(api.Scene)
+    mat = [types.SimpleNamespace(texture=types.SimpleNamespace(data=b), roughness=None, normal=None) for b in buffers]
+    scene.meshes = [types.SimpleNamespace(material=m, v=m.texture.data) for m in mat]
+    scene.lights, scene._builds = [], 0
+    return scene
+
+
+def test_scene_made_under_inference_mode_has_no_stamp():
+    """Its buffers track no versions: renderD re-traces the paths instead of keeping records."""
+    src = torch.ones(3)
+    with torch.inference_mode():
+        inside = src.detach().to(copy=True)
+    outside = src.detach().to(copy=True)
+    assert _scene_of([outside, inside])._stamp() is None
+    integ = api.PathIntegrator.__new__(api.PathIntegrator)
+    integ.cfg = api.L.Config()
+    assert integ._new_records(_scene_of([inside]), (api.L.CameraDesc * 1)()) is None
+    stamp = _scene_of([outside])._stamp()
+    outside.mul_(2.0)
+    assert stamp is not None and _scene_of([outside])._stamp() != stamp

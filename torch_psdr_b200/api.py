@@ -407,11 +407,14 @@ class Scene(VarContex):
         self._builds = 0  # rebuilds since creation
 
     def _stamp(self):
-        """Changes whenever the native scene, or a buffer it reads while rendering, does."""
+        """Changes whenever the native scene, or a buffer it reads while rendering, does; None when
+        that cannot be told (buffers made under inference mode track no versions)."""
         tex = [t.data for m in self.meshes for t in (m.material.texture, m.material.roughness, m.material.normal)
                if t is not None]
         tex += [lt.cube_map.data for lt in self.lights if isinstance(lt, EnvLight)]
         tex += [o.v for o in self.meshes + self.lights if o.v is not None]
+        if any(t.is_inference() for t in tex):
+            return None
         return self._builds, tuple((t.data_ptr(), t._version) for t in tex)
 
     @property
@@ -646,12 +649,17 @@ class PathIntegrator:
         return imgs
 
     def _stamp(self, scene: Scene, cams):
-        return bytes(cams), bytes(self.cfg), scene._stamp()
+        own = scene._stamp()
+        return None if own is None else (bytes(cams), bytes(self.cfg), own)
 
     def _new_records(self, scene: Scene, cams):
         """Memory for the replay records of a renderD forward, or None when they are not wanted
-        (batch_records = -1, no interior term) or take more than a quarter of the free memory."""
+        (batch_records = -1, no interior term), could not be checked against the scene of the
+        backward, or take more than a quarter of the free memory."""
         if self.cfg.batch_records < 0 or (self.cfg.terms and not self.cfg.terms & 1):
+            return None
+        stamp = self._stamp(scene, cams)
+        if stamp is None:
             return None
         n = C.c_int64()
         L.check(self._lib.psdr_records_bytes(cams, len(cams), C.byref(self.cfg), C.byref(n)), "psdr_records_bytes")
@@ -668,7 +676,7 @@ class PathIntegrator:
             self._records_granted = 0
             return None
         self._records_granted = max(n, self._records_granted)
-        return _Records(data, self._stamp(scene, cams))
+        return _Records(data, stamp)
 
     def autotune(self, scene: Scene, cache: Optional[str] = None) -> dict:
         """Pick the wavefront tile size and the scene's BVH leaf size by timing forward
