@@ -2,6 +2,7 @@
 native library."""
 import contextlib
 import types
+import weakref
 
 import pytest
 import torch
@@ -78,3 +79,70 @@ def test_scene_made_under_inference_mode_has_no_stamp():
     stamp = _scene_of([outside])._stamp()
     outside.mul_(2.0)
     assert stamp is not None and _scene_of([outside])._stamp() != stamp
+
+
+class _Memory:
+    """A GPU's memory as _new_records sees it: free bytes outside torch's cache, the cache, and
+    the tensors allocated from it (kept by the records that hold them)."""
+
+    def __init__(self, monkeypatch, free):
+        self.free, self.reserved, self.tensors, self.queries = free, 0, weakref.WeakSet(), 0
+        monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+        monkeypatch.setattr(torch.cuda, "current_stream", lambda: "stream")
+        monkeypatch.setattr(torch.cuda, "memory_stats_as_nested_dict", lambda d=None: {
+            k: {"all": {"current": v}} for k, v in (("reserved_bytes", self.reserved), ("allocated_bytes", self.allocated()))})
+        monkeypatch.setattr(torch.cuda, "mem_get_info", self.query)
+        monkeypatch.setattr(torch, "empty", self.empty)
+
+    def allocated(self):
+        return sum(t.numel() for t in self.tensors)
+
+    def query(self, d=None):
+        self.queries += 1
+        return self.free, 0
+
+    def empty(self, n, dtype=None, device=None):
+        grow = max(0, self.allocated() + n - self.reserved)
+        if grow > self.free:
+            raise torch.OutOfMemoryError()
+        self.free -= grow
+        self.reserved += grow
+        t = _OnGpu([], 0)
+        t.numel = lambda: n
+        self.tensors.add(t)
+        return t
+
+
+@pytest.mark.parametrize("size", [1 << 30, 40 << 20])
+def test_records_of_all_graphs_share_one_limit(monkeypatch, size):
+    """Graphs kept alive, whichever integrator made them: together their records take at most a
+    quarter of the memory, and a graph that would go beyond it re-traces its paths."""
+    mem = _Memory(monkeypatch, 16 << 30)
+    monkeypatch.setattr(api.PathIntegrator, "_stamp", lambda *a: "stamp")
+
+    def records_bytes(cams, n, cfg, out):
+        out._obj.value = size
+        return 0
+
+    def integrator():
+        it = api.PathIntegrator.__new__(api.PathIntegrator)
+        it.cfg, it._records_granted = api.L.Config(), 0
+        it._lib = types.SimpleNamespace(psdr_records_bytes=records_bytes)
+        return it
+
+    first, second = integrator(), integrator()
+    kept = []
+    for k in range(150):
+        kept.append((first if k % 2 else second)._new_records(None, [None]))
+    held = [r for r in kept if r is not None]
+    assert len(held) == (4 << 30) // size and mem.allocated() <= 4 << 30
+    # with the graphs gone, the next ones take the cache's memory, without asking again
+    mem.queries = 0
+    del kept, held
+    free = mem.free
+    for _ in range(5):
+        assert first._new_records(None, [None]) is not None
+    assert mem.free == free and mem.queries == 0
+    # memory that went elsewhere since is asked for, not assumed
+    mem.free, mem.reserved = size // 2, 0
+    assert first._new_records(None, [None]) is None or size <= 64 << 20

@@ -11,6 +11,8 @@ from __future__ import annotations
 import ctypes as C
 import json
 import os
+import threading
+import weakref
 from typing import List, Optional, Union
 
 import numpy as np
@@ -487,9 +489,20 @@ class _Records:
     uses them only when the scene, cameras and configuration are still the same; otherwise
     it re-traces the paths, as it does without records."""
 
+    _alive = weakref.WeakSet()
+    _lock = threading.Lock()
+
     def __init__(self, data, stamp):
         self.data, self.stamp = data, stamp
         self.stream = torch.cuda.current_stream()
+        with _Records._lock:
+            _Records._alive.add(self)
+
+    @staticmethod
+    def held(device) -> int:
+        """Bytes of the records on a GPU that autograd graphs hold now."""
+        with _Records._lock:
+            return sum(r.data.numel() for r in _Records._alive if r.data.device == device)
 
     def pointer(self, stamp):
         """Address for a backward with this stamp; None: re-trace."""
@@ -623,7 +636,7 @@ class PathIntegrator:
         self.cfg = cfg
         self._lib = L.load()
         self._ws = None
-        self._records_granted = 0  # bytes of replay records that fitted before
+        self._records_granted = 0  # bytes of replay records, all graphs' together, that fitted before
 
     def _workspace(self):
         if self._ws is None:
@@ -664,18 +677,24 @@ class PathIntegrator:
         n = C.c_int64()
         L.check(self._lib.psdr_records_bytes(cams, len(cams), C.byref(self.cfg), C.byref(n)), "psdr_records_bytes")
         n = int(n.value)
-        # (the free memory is asked for once per size: the query takes a third of a millisecond, and
-        # memory granted before stays in torch's cache)
-        if self.cfg.batch_records == 0 and n > max(64 << 20, self._records_granted):
-            free = torch.cuda.mem_get_info()[0] + torch.cuda.memory_reserved() - torch.cuda.memory_allocated()
-            if n > free // 4:
-                return None
+        # All graphs' records together may take a quarter of the memory there would be without
+        # them. The query takes a third of a millisecond: it is left out up to 64 MB in all, and
+        # for what was granted before as long as torch's cache still holds the memory.
+        dev = torch.device("cuda", torch.cuda.current_device())
+        total = _Records.held(dev) + n
+        if self.cfg.batch_records == 0 and total > 64 << 20:
+            stats = torch.cuda.memory_stats_as_nested_dict(dev)
+            cached = stats["reserved_bytes"]["all"]["current"] - stats["allocated_bytes"]["all"]["current"]
+            if total > self._records_granted or n > cached:
+                if total > (torch.cuda.mem_get_info(dev)[0] + cached + total - n) // 4:
+                    return None
         try:
-            data = torch.empty(n, dtype=torch.uint8, device="cuda")
+            data = torch.empty(n, dtype=torch.uint8, device=dev)
         except torch.OutOfMemoryError:
             self._records_granted = 0
             return None
-        self._records_granted = max(n, self._records_granted)
+        if self.cfg.batch_records == 0:
+            self._records_granted = max(total, self._records_granted)
         return _Records(data, stamp)
 
     def autotune(self, scene: Scene, cache: Optional[str] = None) -> dict:
