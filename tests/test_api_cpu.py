@@ -42,6 +42,7 @@ def _fake_cuda(monkeypatch, tensors):
         return 0
 
     monkeypatch.setattr(torch.cuda, "device", device)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: current[-1].index)
     monkeypatch.setattr(api, "_stream", lambda: current[-1].index)
     monkeypatch.setattr(api.L, "load", lambda: types.SimpleNamespace(psdr_index_bounds=bounds))
     return calls

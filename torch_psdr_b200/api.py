@@ -8,6 +8,7 @@ calls psdr_render_bwd (the path-replay adjoint).
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import json
 import os
@@ -54,7 +55,8 @@ def _check_index_buffers(jobs) -> None:
         ptrs = (C.c_void_p * n)(*[t.data_ptr() for t, _, _ in own])
         counts = (C.c_int64 * n)(*[t.numel() for t, _, _ in own])
         out = (C.c_int32 * (2 * n))()
-        with torch.cuda.device(dev):
+        # (entering a device takes 10 us, as long as the kernel: left out for the current one)
+        with contextlib.nullcontext() if dev.index == torch.cuda.current_device() else torch.cuda.device(dev):
             L.check(L.load().psdr_index_bounds(ptrs, counts, n, out, _stream()), "psdr_index_bounds")
         for i, (_, bound, what) in enumerate(own):
             if out[2 * i] < 0 or out[2 * i + 1] >= bound:
