@@ -114,9 +114,74 @@ PSDR_D void acc_add(GradAcc* a, float v) {
   if (dh) atomicAdd(reinterpret_cast<unsigned long long*>(&a->hi), (unsigned long long)(neg ? -dh : dh));
   if (dl) atomicAdd(reinterpret_cast<unsigned long long*>(&a->lo), (unsigned long long)(neg ? -dl : dl));
 }
+// (the low limb's carry is moved up first, so equal sums give equal values however they were split)
 PSDR_HD double acc_value(long long hi, long long lo) {
+  hi += lo >> 32;
+  lo &= 0xffffffffll;
   return (double)hi * 9.5367431640625e-07 + (double)lo * 2.220446049250313e-16;  // 2^-20, 2^-52
 }
+
+// A thread's own sum of contributions to one accumulator, in the same two limbs. Contributions
+// below 512 go to lo as whole units of 2^-52, larger ones (whole units of 2^-20, as fp32
+// numbers) to hi, and lo's carry moves up before it overflows: the sum is exactly what
+// acc_add of each contribution would give, however the contributions are grouped over threads.
+constexpr float kOwnMax = 512.f;
+PSDR_D long long own_units(float v) {  // 0 for the contributions that own_carry takes (and NaN)
+  return fabsf(v) < kOwnMax ? __float2ll_rn(v * 4503599627370496.f) : 0;  // 2^52: exact
+}
+// |lo| >= 2^61: the top three bits differ.
+PSDR_D unsigned own_top(long long lo) { return ((unsigned)(lo >> 32) + 0x20000000u) & 0xC0000000u; }
+static __device__ __noinline__ void own_carry(long long& lo, long long& hi, float v) {
+  if (own_top(lo)) {
+    hi += lo >> 32;
+    lo &= 0xffffffffll;
+  }
+  if (fabsf(v) >= kOwnMax && isfinite(v)) hi += __float2ll_rn(fminf(fmaxf(v, -4398046511104.f), 4398046511104.f) * 1048576.f);
+}
+// lo and hi of three accumulators, one test for all.
+PSDR_D bool own_add3(long long* lo, float3 v) {
+  lo[0] += own_units(v.x);
+  lo[1] += own_units(v.y);
+  lo[2] += own_units(v.z);
+  const bool small = fabsf(v.x) < kOwnMax && fabsf(v.y) < kOwnMax && fabsf(v.z) < kOwnMax;
+  return small && !(own_top(lo[0]) | own_top(lo[1]) | own_top(lo[2]));  // false: own_carry
+}
+PSDR_D void acc_put(GradAcc* a, long long hi, long long lo) {
+  hi += lo >> 32;
+  lo &= 0xffffffffll;
+  if (hi) atomicAdd(reinterpret_cast<unsigned long long*>(&a->hi), (unsigned long long)hi);
+  if (lo) atomicAdd(reinterpret_cast<unsigned long long*>(&a->lo), (unsigned long long)lo);
+}
+// The sums of a warp's lanes, all for accumulator a, in one addition (all lanes call it).
+PSDR_D void acc_put_warp(GradAcc* a, long long hi, long long lo) {
+  if (!__any_sync(0xffffffffu, (hi | lo) != 0)) return;
+  hi += lo >> 32;
+  lo &= 0xffffffffll;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    hi += __shfl_xor_sync(0xffffffffu, hi, o);
+    lo += __shfl_xor_sync(0xffffffffu, lo, o);
+  }
+  if ((threadIdx.x & 31) == 0) acc_put(a, hi, lo);
+}
+// Sums for the three accumulators of a vector.
+struct Own3 {
+  long long lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
+  PSDR_D void add(float3 v) {
+    if (own_add3(lo, v)) return;
+    own_carry(lo[0], hi[0], v.x);
+    own_carry(lo[1], hi[1], v.y);
+    own_carry(lo[2], hi[2], v.z);
+  }
+  PSDR_D void put(GradAcc* a) const {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) acc_put(a + k, hi[k], lo[k]);
+  }
+  PSDR_D void put_warp(GradAcc* a) const {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) acc_put_warp(a + k, hi[k], lo[k]);
+  }
+};
 
 // ------------------------------------------------------------------ scene records
 struct DevTex {

@@ -625,36 +625,54 @@ PSDR_D SurfAdj zero_adj() {
   return a;
 }
 
-// A lane's sums of the gradients that most of its paths share: the vertices of the scene's only
-// light (DevScene::light_nv) and the emission of its first kHotLights lights. They belong to
-// one scene; a lane that goes on to another scene's paths adds them to the accumulators first.
-// (In jobs with several scenes the emission gradients used to go to the accumulators one by one,
-// every lane of the GPU adding to the same few words: a 9-view step over three scenes took
-// 67.2 ms, now 51.5.)
+// A lane's own sums (own_add3) of the gradients that most of its paths share: the vertices of
+// the scene's only light (DevScene::light_nv) and the emission of its first kHotLights lights.
+// They belong to one scene; a lane that goes on to another scene's paths adds them to the
+// accumulators first. (In jobs with several scenes the emission gradients used to go to the
+// accumulators one by one, every lane of the GPU adding to the same few words: a 9-view step
+// over three scenes took 67.2 ms, 51.5 with sums per lane.) Their exact integers cost about a
+// twentieth of the adjoint kernels' time against fp32 sums, which lose the small terms
+// and depend on how paths are dealt to lanes.
 constexpr int kHotLights = 4;
+constexpr int kHotEmit = 3 * kMaxLightVerts;  // first emission sum
+constexpr int kHotSums = kHotEmit + 3 * kHotLights;
 struct HotAcc {
   const DevScene* sc;
   int lv0, nlv;  // light vertex range; nlv = 0: none
   int nlt;       // lights whose emission gradient is summed here
-  float g[kMaxLightVerts * 3];
-  float e[kHotLights * 3];
+  bool high;     // hi is in use (large contributions, carries)
+  long long lo[kHotSums], hi[kHotSums];
 };
 PSDR_D void hot_init(HotAcc& hot) {
   hot.sc = nullptr;
   hot.lv0 = hot.nlv = hot.nlt = 0;
+  hot.high = false;
 #pragma unroll
-  for (int k = 0; k < kMaxLightVerts * 3; ++k) hot.g[k] = 0.f;
-#pragma unroll
-  for (int k = 0; k < kHotLights * 3; ++k) hot.e[k] = 0.f;
+  for (int k = 0; k < kHotSums; ++k) hot.lo[k] = 0;
+}
+static __device__ __noinline__ void hot_carry(HotAcc& hot, int k, float3 v) {
+  if (!hot.high) {
+    for (int q = 0; q < kHotSums; ++q) hot.hi[q] = 0;
+    hot.high = true;
+  }
+  own_carry(hot.lo[k], hot.hi[k], v.x);
+  own_carry(hot.lo[k + 1], hot.hi[k + 1], v.y);
+  own_carry(hot.lo[k + 2], hot.hi[k + 2], v.z);
+}
+// Adds v to sums k, k + 1, k + 2 (a dynamic index: the sums live in local memory, L1).
+PSDR_D void hot_add(HotAcc& hot, int k, float3 v) {
+  if (!own_add3(hot.lo + k, v)) hot_carry(hot, k, v);
+}
+PSDR_D GradAcc* hot_target(const HotAcc& hot, int k) {
+  return k < kHotEmit ? hot.sc->grad_verts + 3 * (size_t)hot.lv0 + k
+                      : hot.sc->lights[(k - kHotEmit) / 3].grad_emit + (k - kHotEmit) % 3;
 }
 static __device__ __noinline__ void hot_spill(HotAcc& hot) {
-  const DevScene* sc = hot.sc;
-  if (!sc) return;
-  if (hot.nlv > 0 && vert_wanted(*sc, hot.lv0))
-    for (int k = 0; k < hot.nlv * 3; ++k) acc_add(sc->grad_verts + 3 * (size_t)hot.lv0 + k, hot.g[k]);
-  for (int l = 0; l < hot.nlt; ++l)
-    if (sc->lights[l].grad_emit)
-      for (int k = 0; k < 3; ++k) acc_add(sc->lights[l].grad_emit + k, hot.e[3 * l + k]);
+  if (!hot.sc) return;
+  for (int k = 0; k < kHotSums; ++k) {
+    const long long hi = hot.high ? hot.hi[k] : 0;
+    if (hi | hot.lo[k]) acc_put(hot_target(hot, k), hi, hot.lo[k]);
+  }
   hot_init(hot);
 }
 PSDR_D void hot_bind(HotAcc& hot, const DevScene* sc) {
@@ -662,7 +680,7 @@ PSDR_D void hot_bind(HotAcc& hot, const DevScene* sc) {
   hot_spill(hot);
   hot.sc = sc;
   hot.lv0 = sc->light_v0;
-  hot.nlv = sc->light_nv;
+  hot.nlv = sc->light_nv > 0 && vert_wanted(*sc, sc->light_v0) ? sc->light_nv : 0;
   hot.nlt = min(sc->nlight, kHotLights);
 }
 // End of a kernel (all lanes together): one addition per warp when its lanes share the scene.
@@ -675,27 +693,10 @@ PSDR_D void hot_flush(HotAcc& hot) {
     hot_spill(hot);
     return;
   }
-  if (!own) {
-    hot.sc = reinterpret_cast<const DevScene*>(first);
-    hot.lv0 = hot.sc->light_v0;
-    hot.nlv = hot.sc->light_nv;
-    hot.nlt = min(hot.sc->nlight, kHotLights);
-  }
-#pragma unroll
-  for (int k = 0; k < kMaxLightVerts * 3; ++k) {
-    float v = hot.g[k];
-#pragma unroll
-    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    hot.g[k] = v;
-  }
-#pragma unroll
-  for (int k = 0; k < kHotLights * 3; ++k) {
-    float v = hot.e[k];
-#pragma unroll
-    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    hot.e[k] = v;
-  }
-  if ((threadIdx.x & 31) == 0) hot_spill(hot);
+  if (!own) hot_bind(hot, reinterpret_cast<const DevScene*>(first));
+  for (int k = 0; k < 3 * hot.nlv; ++k) acc_put_warp(hot_target(hot, k), hot.high ? hot.hi[k] : 0, hot.lo[k]);
+  for (int k = kHotEmit; k < kHotEmit + 3 * hot.nlt; ++k)
+    if (hot.sc->lights[(k - kHotEmit) / 3].grad_emit) acc_put_warp(hot_target(hot, k), hot.high ? hot.hi[k] : 0, hot.lo[k]);
 }
 
 // Adjoint ae of an environment light's radiance at box uv (u, v), incoming direction wi:
@@ -723,13 +724,10 @@ static __device__ __noinline__ float3 env_emit_adj(const DevLight* L, float u, f
 // accumulator, environment lights into their parameters, and the SH9 direction's share
 // into the point x (wi = -normalize(q - x)).
 PSDR_D void add_emit(const DevScene& sc, HotAcc& hot, int light, float3 a) {
-  if (light < hot.nlt) {
-    hot.e[3 * light] += a.x;
-    hot.e[3 * light + 1] += a.y;
-    hot.e[3 * light + 2] += a.z;
-  } else if (sc.lights[light].grad_emit) {
-    atomic_add3(sc.lights[light].grad_emit, a);
-  }
+  GradAcc* to = sc.lights[light].grad_emit;
+  if (!to) return;
+  if (light < hot.nlt) hot_add(hot, kHotEmit + 3 * light, a);
+  else atomic_add3(to, a);
 }
 
 template <bool EXT>
@@ -747,11 +745,7 @@ PSDR_D void add_vertex(const DevScene& sc, HotAcc& hot, int v, float3 a) {
   if (!sc.grad_verts) return;
   const int rel = v - hot.lv0;
   if (hot.nlv > 0 && rel >= 0 && rel < hot.nlv) {
-    // dynamic index: the accumulators live in local memory (L1), which keeps this code
-    // short at each of the adjoint's scatter sites
-    hot.g[3 * rel] += a.x;
-    hot.g[3 * rel + 1] += a.y;
-    hot.g[3 * rel + 2] += a.z;
+    hot_add(hot, 3 * rel, a);
     return;
   }
   vert_add(sc, v, a);
@@ -1159,35 +1153,28 @@ PSDR_D float3 suffix_radiance(const WF& w, int s, int from) {
   return S;
 }
 
-// Camera-origin adjoint kept in registers while consecutive samples share a view.
+// Camera-origin adjoint summed per lane while consecutive samples share a view.
 struct CamAcc {
   const DevView* v = nullptr;
-  float3 g;
+  Own3 g;
   PSDR_D void add(const DevView* view, float3 a) {
     if (view != v) {
       flush();
       v = view;
-      g = f3(0.f, 0.f, 0.f);
     }
-    g += a;
+    if (v->grad_pos) g.add(a);
   }
   PSDR_D void flush() {
-    if (v && v->grad_pos && (g.x != 0.f || g.y != 0.f || g.z != 0.f)) atomic_add3(v->grad_pos, g);
+    if (v && v->grad_pos) g.put(v->grad_pos);
     v = nullptr;
+    g = Own3();
   }
-  // End of a kernel: one atomic per warp when the warp shares the view.
+  // End of a kernel: one addition per warp when the warp shares the view.
   PSDR_D void flush_warp() {
     const unsigned long long key = (unsigned long long)v;
     const unsigned long long k0 = __shfl_sync(0xffffffffu, key, 0);
     if (!__all_sync(0xffffffffu, key == k0) || !v) { flush(); return; }
-    float3 s = g;
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
-      s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
-      s.z += __shfl_xor_sync(0xffffffffu, s.z, o);
-    }
-    if ((threadIdx.x & 31) == 0) { g = s; flush(); }
+    if (v->grad_pos) g.put_warp(v->grad_pos);
     v = nullptr;
   }
 };
@@ -1781,7 +1768,7 @@ __global__ void __launch_bounds__(256) k_edge_final_unb(WF w, const DevScene* __
   const DevScene& sc = scenes[V.scene];
   const float3 look = view_look(V);
   const float fxfy = view_fxfy(V);
-  float3 go = f3(0.f, 0.f, 0.f);
+  Own3 go;  // camera origin
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n32; s += stride) {
     if (s >= n || !V.dimage) continue;
     const float4 hg = eb.hb[s];
@@ -1816,17 +1803,9 @@ __global__ void __launch_bounds__(256) k_edge_final_unb(WF w, const DevScene* __
       vert_add(sc, tv.y, ag * hg.y);
       vert_add(sc, tv.z, ag * hg.z);
     }
-    go -= av * (1.f - ratio);
+    if (V.grad_pos) go.add(-(av * (1.f - ratio)));
   }
-  if (V.grad_pos) {
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      go.x += __shfl_xor_sync(0xffffffffu, go.x, o);
-      go.y += __shfl_xor_sync(0xffffffffu, go.y, o);
-      go.z += __shfl_xor_sync(0xffffffffu, go.z, o);
-    }
-    if ((threadIdx.x & 31) == 0 && (go.x != 0.f || go.y != 0.f || go.z != 0.f)) atomic_add3(V.grad_pos, go);
-  }
+  if (V.grad_pos) go.put_warp(V.grad_pos);
 }
 
 // Between the two trace2light calls: keep L_a, restart the slot at the +eps hit with
@@ -1863,7 +1842,7 @@ __global__ void __launch_bounds__(256) k_edge_final(WF w, const DevScene* __rest
   const int n32 = (n + 31) & ~31;
   const DevView& V = views[v];
   const DevScene& sc = scenes[V.scene];
-  float3 go = f3(0.f, 0.f, 0.f);
+  Own3 go;  // camera origin
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n32; s += stride) {
     if (s >= n) continue;
     const float4 hb = eb.hb[s];
@@ -1895,18 +1874,10 @@ __global__ void __launch_bounds__(256) k_edge_final(WF w, const DevScene* __rest
         vert_add(sc, ev.x, ax * (1.f - ss));
         vert_add(sc, ev.y, ax * ss);
       }
-      go += (nflip - jo) * K;
+      if (V.grad_pos) go.add((nflip - jo) * K);
     }
   }
-  if (!PRE && V.grad_pos) {
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      go.x += __shfl_xor_sync(0xffffffffu, go.x, o);
-      go.y += __shfl_xor_sync(0xffffffffu, go.y, o);
-      go.z += __shfl_xor_sync(0xffffffffu, go.z, o);
-    }
-    if ((threadIdx.x & 31) == 0 && (go.x != 0.f || go.y != 0.f || go.z != 0.f)) atomic_add3(V.grad_pos, go);
-  }
+  if (!PRE && V.grad_pos) go.put_warp(V.grad_pos);
 }
 
 // ------------------------------------------------------------------ pixel borders
@@ -2031,7 +2002,7 @@ __global__ void __launch_bounds__(256) k_border_final(WF w, const DevScene* __re
   const int n32 = (n + 31) & ~31;
   const DevView& V = views[v];
   const DevScene& sc = scenes[V.scene];
-  float3 go = f3(0.f, 0.f, 0.f);
+  Own3 go;  // camera origin
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n32; s += stride) {
     if (s >= n || !V.dimage) continue;
     const float4 h = eb.hb[s];
@@ -2067,17 +2038,9 @@ __global__ void __launch_bounds__(256) k_border_final(WF w, const DevScene* __re
       vert_add(sc, tv.y, ag * h.y);
       vert_add(sc, tv.z, ag * h.z);
     }
-    go -= ag;
+    if (V.grad_pos) go.add(-ag);
   }
-  if (V.grad_pos) {
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      go.x += __shfl_xor_sync(0xffffffffu, go.x, o);
-      go.y += __shfl_xor_sync(0xffffffffu, go.y, o);
-      go.z += __shfl_xor_sync(0xffffffffu, go.z, o);
-    }
-    if ((threadIdx.x & 31) == 0 && (go.x != 0.f || go.y != 0.f || go.z != 0.f)) atomic_add3(V.grad_pos, go);
-  }
+  if (V.grad_pos) go.put_warp(V.grad_pos);
 }
 
 // ------------------------------------------------------------------ camera lens
@@ -2095,36 +2058,24 @@ __global__ void __launch_bounds__(256) k_border_final(WF w, const DevScene* __re
 // pixel's dPhi/dI), grad_lens[3..11] = dPhi/dG of the border part (row-major 3x3).
 struct LensAcc {
   const DevView* v = nullptr;
-  float s0 = 0.f, sx = 0.f, sy = 0.f;
+  Own3 s;
   PSDR_D void add(const DevView* view, float gl, float ux, float uy) {
     if (view != v) {
       flush();
       v = view;
-      s0 = sx = sy = 0.f;
     }
-    s0 += gl;
-    sx += gl * ux;
-    sy += gl * uy;
+    s.add(f3(gl, gl * ux, gl * uy));  // (views without grad_lens are skipped)
   }
   PSDR_D void flush() {
-    if (v && v->grad_lens && (s0 != 0.f || sx != 0.f || sy != 0.f)) {
-      acc_add(v->grad_lens, s0);
-      acc_add(v->grad_lens + 1, sx);
-      acc_add(v->grad_lens + 2, sy);
-    }
+    if (v) s.put(v->grad_lens);
     v = nullptr;
+    s = Own3();
   }
   PSDR_D void flush_warp() {
     const unsigned long long key = (unsigned long long)v;
     const unsigned long long k0 = __shfl_sync(0xffffffffu, key, 0);
     if (!__all_sync(0xffffffffu, key == k0) || !v) { flush(); return; }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-      sx += __shfl_xor_sync(0xffffffffu, sx, o);
-      sy += __shfl_xor_sync(0xffffffffu, sy, o);
-    }
-    if ((threadIdx.x & 31) == 0) flush();
+    s.put_warp(v->grad_lens);
     v = nullptr;
   }
 };
@@ -2172,7 +2123,7 @@ __global__ void __launch_bounds__(256) k_lens_border(WF w, const DevView* __rest
   const int stride = gridDim.x * blockDim.x;
   const int n32 = (n + 31) & ~31;
   const DevView& V = views[v];
-  float b0 = 0.f, b1 = 0.f, b2 = 0.f, b3 = 0.f, b4 = 0.f, b5 = 0.f, b6 = 0.f, b7 = 0.f, b8 = 0.f;
+  Own3 bv, bh, bc;  // rows of dPhi/dG
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n32; s += stride) {
     if (s >= n || !V.dimage || !V.grad_lens) continue;
     if (__float_as_int(eb.hb[s].x) < 0) continue;  // the border ray left the scene: no radiance
@@ -2188,22 +2139,14 @@ __global__ void __launch_bounds__(256) k_lens_border(WF w, const DevView* __rest
     const float ux = (vert ? (float)k : a.y + (float)k) - 0.5f * (float)V.W;
     const float uy = (vert ? a.y + (float)j : (float)j) - 0.5f * (float)V.H;
     const float wc = wgt * (vert ? ux : uy);
-    if (vert) { b0 -= wgt * ux; b1 -= wgt * uy; b2 -= wgt; }
-    else { b3 -= wgt * ux; b4 -= wgt * uy; b5 -= wgt; }
-    b6 += wc * ux;
-    b7 += wc * uy;
-    b8 += wc;
+    if (vert) bv.add(f3(-wgt * ux, -wgt * uy, -wgt));
+    else bh.add(f3(-wgt * ux, -wgt * uy, -wgt));
+    bc.add(f3(wc * ux, wc * uy, wc));
   }
-  float b[9] = {b0, b1, b2, b3, b4, b5, b6, b7, b8};
-#pragma unroll
-  for (int o = 16; o; o >>= 1)
-#pragma unroll
-    for (int m = 0; m < 9; ++m) b[m] += __shfl_xor_sync(0xffffffffu, b[m], o);
-  if ((threadIdx.x & 31) == 0 && V.grad_lens) {
-#pragma unroll
-    for (int m = 0; m < 9; ++m)
-      if (b[m] != 0.f) acc_add(V.grad_lens + 3 + m, b[m]);
-  }
+  if (!V.grad_lens) return;
+  bv.put_warp(V.grad_lens + 3);
+  bh.put_warp(V.grad_lens + 6);
+  bc.put_warp(V.grad_lens + 9);
 }
 
 // dPhi/dtheta_j = <Gamma, P_j>, Gamma = B + the interior part of dPhi/dG.
@@ -2614,7 +2557,7 @@ __global__ void __launch_bounds__(256) k_crease_final(WF w, const DevScene* __re
   const int n32 = (n + 31) & ~31;
   const DevView& V = views[v];
   const DevScene& sc = scenes[V.scene];
-  float3 go = f3(0.f, 0.f, 0.f);
+  Own3 go;  // camera origin
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n32; s += stride) {
     if (s >= n || !V.dimage) continue;
     const int flag = __float_as_int(eb.hb[s].w);
@@ -2651,17 +2594,9 @@ __global__ void __launch_bounds__(256) k_crease_final(WF w, const DevScene* __re
       vert_add(sc, v2.y, a2 * b2.y);
       vert_add(sc, v2.z, a2 * b2.z);
     }
-    go -= a1 + a2;  // moving the camera by d is moving both surfaces by -d
+    if (V.grad_pos) go.add(-(a1 + a2));  // moving the camera by d is moving both surfaces by -d
   }
-  if (V.grad_pos) {
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      go.x += __shfl_xor_sync(0xffffffffu, go.x, o);
-      go.y += __shfl_xor_sync(0xffffffffu, go.y, o);
-      go.z += __shfl_xor_sync(0xffffffffu, go.z, o);
-    }
-    if ((threadIdx.x & 31) == 0 && (go.x != 0.f || go.y != 0.f || go.z != 0.f)) atomic_add3(V.grad_pos, go);
-  }
+  if (V.grad_pos) go.put_warp(V.grad_pos);
 }
 
 // ------------------------------------------------------------------ BSDF jumps
@@ -2777,9 +2712,7 @@ __global__ void __launch_bounds__(256) k_jump_final(WF w, const DevScene* __rest
   const int n32 = (n + 31) & ~31;
   const DevView& V = views[v];
   const DevScene& sc = scenes[V.scene];
-  HotAcc hot;
-  hot_init(hot);  // never bound to a scene: everything goes to the accumulators
-  float3 go = f3(0.f, 0.f, 0.f);
+  Own3 go;  // camera origin
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n32; s += stride) {
     if (s >= n || !V.dimage) continue;
     const float4 hk = eb.n[s];
@@ -2823,25 +2756,17 @@ __global__ void __launch_bounds__(256) k_jump_final(WF w, const DevScene* __rest
     aa.p = du;
     ax.p = -du;
     const float3 ao = mat_finalize(ob, x, mp, ma, ax);
-    scatter_surf(sc, hot, tk, hk.y, hk.z, x.front, ax);
-    scatter_surf(sc, hot, ta, hn.y, hn.z, xa.front, aa);
+    scatter_mesh(sc, tk, hk.y, hk.z, x.front, ax);
+    scatter_mesh(sc, ta, hn.y, hn.z, xa.front, aa);
     if (tp >= 0) {
       SurfAdj ap = zero_adj();
       ap.p = ao;
-      scatter_surf(sc, hot, tp, hp.y, hp.z, true, ap);
-    } else if (!fixed_v) {
-      go += ao;
+      scatter_mesh(sc, tp, hp.y, hp.z, true, ap);
+    } else if (!fixed_v && V.grad_pos) {
+      go.add(ao);
     }
   }
-  if (V.grad_pos) {
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      go.x += __shfl_xor_sync(0xffffffffu, go.x, o);
-      go.y += __shfl_xor_sync(0xffffffffu, go.y, o);
-      go.z += __shfl_xor_sync(0xffffffffu, go.z, o);
-    }
-    if ((threadIdx.x & 31) == 0 && (go.x != 0.f || go.y != 0.f || go.z != 0.f)) atomic_add3(V.grad_pos, go);
-  }
+  if (V.grad_pos) go.put_warp(V.grad_pos);
 }
 
 // ------------------------------------------------------------------ direct edges
