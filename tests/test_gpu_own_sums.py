@@ -53,10 +53,10 @@ def _grads(spec, scale=1.0, lens=False, **kw):
 @pytest.mark.parametrize("estimator", ["reference", "unbiased"])
 @pytest.mark.parametrize("case", [dict(), dict(lights=6), dict(fan=12), dict(rough=True, lights=2)])
 def test_tiles_give_bitwise_equal_gradients(cuda, estimator, case):
-    spec = _spec(**case)
+    spec = _spec(size=256, **case)  # 2^20 paths: some fourteen to a thread in one tile
     want = _grads(spec, estimator=estimator)
     assert len(want) >= 5
-    for records, tile in ((0, 1 << 12), (-1, 1 << 14)):
+    for records, tile in ((0, 1 << 14), (-1, 1 << 18)):
         got = _grads(spec, estimator=estimator, tile_paths=tile, batch_records=records)
         for k in want:
             assert want[k].any(), k
@@ -64,7 +64,7 @@ def test_tiles_give_bitwise_equal_gradients(cuda, estimator, case):
 
 
 def test_tiles_give_bitwise_equal_lens_gradients(cuda):
-    want, got = (_grads(_spec(), lens=True, estimator="unbiased", tile_paths=t) for t in (0, 1 << 12))
+    want, got = (_grads(_spec(size=256), lens=True, estimator="unbiased", tile_paths=t) for t in (0, 1 << 14))
     for k in want:
         assert want[k].any() and np.array_equal(want[k], got[k]), k
 
@@ -73,7 +73,7 @@ def test_tiles_give_bitwise_equal_lens_gradients(cuda):
 def test_scenes_of_a_batch_give_the_plain_gradients(cuda, estimator):
     """Three scenes of one, six and one lights; every view holds whole groups of 32 paths, so
     the batch sums the same terms as three plain steps."""
-    specs = [_spec(size=32), _spec(lights=6, size=40), _spec(fan=12, size=48)]
+    specs = [_spec(size=128), _spec(lights=6, size=160), _spec(fan=12, size=192)]
     plain, Ts, scenes = [_grads(s, estimator=estimator) for s in specs], [], []
     for s in specs:
         scene, T = to_torch_scene(s, requires_grad=KINDS)

@@ -3501,8 +3501,23 @@ void lens_out(const GradAcc* acc, const LensChain& ch, float* out, int accumulat
   PSDR_CUDA(cudaGetLastError());
 }
 
+// Pixels that hold whole groups of 32 paths: the adjoint kernels reduce the camera vertices of 32
+// consecutive paths of a tile over the warp, in fp32.
+static int group_pixels(int spp) {
+  int g = 32;
+  while (spp % g) g >>= 1;
+  return 32 / g;
+}
+
+// Tiles of whole pixels, and of whole groups of 32 paths of the job where a tile holds one: those
+// groups, and with them the gradients, are then the same for any such tile size.
 std::vector<Tile> plan_tiles(const std::vector<DevView>& views, int cap) {
   std::vector<Tile> tiles;
+  if (!views.empty()) {  // (the views of a job share their spp)
+    const int spp = views[0].spp, unit = group_pixels(spp);
+    const int pixels = cap / spp;
+    if (pixels > unit) cap = spp * (pixels / unit * unit);
+  }
   Tile cur{0, 0, 0, 0};
   for (const DevView& v : views) {
     long long rem = (long long)v.H * v.W;
@@ -3674,11 +3689,13 @@ static size_t path_bytes(const psdr_config& cfg, bool records) {
 // 120 node visits for the longest against 14 on average), about 60 us in which the lanes
 // empty out; larger tiles pay for it less often. 1.31 M triangles, 1024^2 x 16 spp, depth 5:
 // traversal 18.2 ms with 2^20-path tiles, 14.7 with 2^21, 13.0 with 2^22.
-// A workspace that already holds such a tile keeps it without asking for the free memory.
+// A workspace that already holds such a tile keeps it without asking for the free memory. The
+// choice changes no image and no gradient (plan_tiles): samples per pixel for which the smallest
+// tile could cut a group of 32 paths get that tile always.
 constexpr long long kTileMax = 1 << 22, kTileBatch = 1 << 21, kTileMin = 1 << 20;
 constexpr size_t kTileBytes = size_t(4) << 30;
 static long long auto_tile(const psdr_config& cfg, long long need, bool records, const psdr_workspace* ws) {
-  if (need <= kTileMin) return kTileMin;
+  if (need <= kTileMin || (long long)group_pixels(cfg.spp_interior) * cfg.spp_interior > kTileMin) return kTileMin;
   const size_t pb = path_bytes(cfg, records);
   long long t = kTileMax;
   while (t > kTileMin && (size_t)t * pb > kTileBytes) t >>= 1;
@@ -3714,6 +3731,7 @@ int choose_cap(const psdr_config& cfg, const std::vector<DevView>& views, bool b
   long long cap = cfg.tile_paths > 0 ? cfg.tile_paths : auto_tile(cfg, need, backward && records, ws);
   if (backward) {
     if (cfg.tile_paths == 0) {
+      // (as few tiles as one per lane, but no smaller than 2^20)
       if (lanes > 1) cap = std::min({cap, kTileBatch, std::max(kTileMin, (total + lanes - 1) / lanes)});
       cap = std::min(cap, need);
     }
