@@ -65,6 +65,16 @@ struct Rng {
     uint32_t rot = (uint32_t)(old >> 59);
     return (xs >> rot) | (xs << ((32u - rot) & 31u));
   }
+  // n draws at once: n steps of s -> a s + c are again such a step, found by squaring
+  // (Brown 1994, random number generation with arbitrary stride).
+  PSDR_HD void skip(uint64_t n) {
+    uint64_t a = kPcgMult, c = inc;
+    for (; n; n >>= 1) {
+      if (n & 1u) state = state * a + c;
+      c *= a + 1;
+      a *= a;
+    }
+  }
   PSDR_HD float next_float(bool advance = true) {
     uint32_t bits = (next(advance) >> 9) | 0x3f800000u;
 #ifdef __CUDA_ARCH__

@@ -2797,7 +2797,7 @@ PSDR_D bool direct_draw(const WF& w, const DevScene& sc, const HCube& hc, int ro
   o.hpdf = 1.f;
   if (PRE) {
     o.rng = make_rng((unsigned long long)i);
-    for (int k = 0; k < 3 * round; ++k) o.rng.next(true);
+    o.rng.skip(3ull * (unsigned)round);
     const int r12 = hc.res[1] * hc.res[2];
     const int c0 = (int)(i / r12);
     const int rem = (int)(i - (long long)c0 * r12);
