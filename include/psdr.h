@@ -279,8 +279,9 @@ PSDR_API psdr_status psdr_render_fwd_noalloc(psdr_scene* scene, const psdr_camer
 PSDR_API psdr_status psdr_render_samples(psdr_scene* scene, psdr_workspace* ws, const psdr_camera_desc* cam,
                                 const psdr_config* cfg, float* samples, void* stream);
 /* Autotuner (extension; the reference has no tuner): times forward renders of the
- * given cameras for every wavefront tile size in {2^18, 2^19, 2^20, 2^21} paths, BVH
- * leaf size in {1, 2, 4} triangles (the scene's BVH is rebuilt for each) and traversal
+ * given cameras for every wavefront tile size in {2^18, 2^19, 2^20, 2^21} paths, and the
+ * automatic one where the job's is larger (written as 0 when it is the fastest), BVH leaf
+ * size in {1, 2, 4} triangles (the scene's BVH is rebuilt for each) and traversal
  * queue depth in {4, 6, 8} x 128 rays per SM, keeps the fastest leaf size in the scene
  * (later psdr_scene_update calls use it), writes the fastest tile size and queue depth to
  * cfg->tile_paths / cfg->trace_queue and, when non-null, the leaf size and the fastest

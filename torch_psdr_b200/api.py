@@ -702,7 +702,8 @@ class PathIntegrator:
     def autotune(self, scene: Scene, cache: Optional[str] = None) -> dict:
         """Pick the wavefront tile size and the scene's BVH leaf size by timing forward
         renders of the scene's cameras (psdr_autotune); the integrator keeps the tile
-        size, the scene keeps the leaf size. Extension: the reference has no tuner.
+        size (0: the automatic one was fastest, and stays), the scene keeps the leaf size.
+        Extension: the reference has no tuner.
 
         cache: path of a JSON file of earlier results, keyed by the GPU (name, SM count)
         and the job's shape (triangles, view sizes, spp, depth, light and BSDF samples,

@@ -661,15 +661,22 @@ psdr_status psdr_autotune(psdr_scene* scene, psdr_workspace* ws, const psdr_came
   PSDR_CUDA(cudaEventCreate(&ev1.e));
   cudaEvent_t e0 = ev0.e, e1 = ev1.e;
   const int leaves[3] = {1, 2, 4};
-  const int tiles[4] = {1 << 18, 1 << 19, 1 << 20, 1 << 21};
+  std::vector<int> tiles = {1 << 18, 1 << 19, 1 << 20, 1 << 21};
+  {
+    // the automatic tile, where it is larger (it then stays automatic: a batch and a backward
+    // choose theirs by lanes and memory)
+    psdr_config c = *cfg;
+    c.tile_paths = 0;
+    if (choose_cap(c, views, false, 1, ws) > tiles.back()) tiles.push_back(0);
+  }
   const int queues[3] = {4, 6, 8};
   float best = INFINITY;
   int bl = scene->leaf_size, bt = cfg->tile_paths, bq = cfg->trace_queue;
   for (int leaf : leaves) {
     scene->leaf_size = leaf;
     scene_build_geometry(scene, st);
-    for (int trial = 0; trial < 12; ++trial) {
-      const int tile = tiles[trial % 4], queue = queues[trial / 4];
+    for (int trial = 0; trial < 3 * (int)tiles.size(); ++trial) {
+      const int tile = tiles[trial % tiles.size()], queue = queues[trial / tiles.size()];
       psdr_config c = *cfg;
       c.tile_paths = tile;
       c.trace_queue = queue;
