@@ -3699,7 +3699,11 @@ static long long auto_tile(const psdr_config& cfg, long long need, bool records,
   const size_t pb = path_bytes(cfg, records);
   long long t = kTileMax;
   while (t > kTileMin && (size_t)t * pb > kTileBytes) t >>= 1;
-  if (t == kTileMin || (ws && ws->cap >= std::min(t, need) && (!records || ws->rec.p))) return t;
+  if (t == kTileMin) return t;
+  const size_t held = (size_t)std::min(t, need);
+  if (ws && (size_t)ws->cap >= held && ws->R >= cfg.mis_light_samples + std::max(cfg.mis_bsdf_samples, records ? 1 : 0) + 1 &&
+      ws->D >= cfg.max_bounce && (!records || ws->rec.bytes >= held * (pb - path_bytes(cfg, false))))
+    return t;
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
     cudaGetLastError();
@@ -3774,7 +3778,8 @@ void psdr_workspace::ensure(int c, int r, int d, int nv, int rec_needed, cudaStr
     cnt.alloc(sizeof(int) * 2 * (kMaxDepth + 2), st);
     ro.alloc(16 * n * R, st); rd.alloc(16 * n * R, st); ra.alloc(16 * n * R, st); hit.alloc(16 * n * R, st);
   }
-  if (rec_needed) rec.alloc(16 * (size_t)cap * (1 + (size_t)D * R + 2 * (size_t)D), st);
+  // the records of the job's tile, which may be smaller than what an earlier job left
+  if (rec_needed) rec.alloc(16 * (size_t)c * (1 + (size_t)d * r + 2 * (size_t)d), st);
   if (nv > nviews_cap) {
     nviews_cap = nv;
     views.alloc(sizeof(DevView) * nv, st);
@@ -3786,7 +3791,7 @@ void psdr_workspace::ensure(int c, int r, int d, int nv, int rec_needed, cudaStr
   wf.q0 = q0.as<int>(); wf.q1 = q1.as<int>(); wf.qs = qs.as<int>(); wf.cnt = cnt.as<int>();
   wf.ro = ro.as<float4>(); wf.rd = rd.as<float4>(); wf.ra = ra.as<float4>(); wf.hit = hit.as<float4>();
   wf.rec = rec.as<float4>();
-  wf.rec_plane = cap;
+  wf.rec_plane = c;
 }
 
 namespace psdr {
