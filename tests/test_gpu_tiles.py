@@ -1,11 +1,14 @@
 """Jobs of several automatic tiles (2^20 to 2^22 paths, by lanes, records, memory and what the
 workspace holds): the images and every gradient are bitwise the same for all of them, and for
 tiles that the caller sets."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
 
 import torch_psdr_b200 as dr
+from torch_psdr_b200 import _lib as L
 from torch_psdr_b200 import synth
 from helpers import to_torch_scene
 
@@ -61,3 +64,32 @@ def test_workspace_history_changes_nothing(cuda):
         out.append([img.detach()] + [t.grad for t in T.values() if t is not None and t.grad is not None])
     for a, b in zip(*out):
         assert torch.equal(a, b)
+
+
+def _trace_launches(run):
+    lib = L.load()
+    out, ms = (C.c_int64 * 3)(), C.c_double()
+    L.check(lib.psdr_profile_enable(1), "enable")
+    L.check(lib.psdr_profile_reset(), "reset")
+    try:
+        run()
+        torch.cuda.synchronize()
+        L.check(lib.psdr_profile_read(out, C.byref(ms)), "read")
+    finally:
+        lib.psdr_profile_enable(0)
+    return out[1]
+
+
+@pytest.mark.parametrize("spp", [32, 37])
+def test_whole_groups_cut_no_extra_tile(cuda, spp):
+    """One tile for a job that fits it, and one per lane for a batch, at any samples per pixel."""
+    spec = synth.sphere_scene(level=1, tex_hw=9, height=170, width=171)
+    scene, _ = to_torch_scene(spec)
+    kw = dict(spp_interior=spp, max_bounce=2)
+    assert _trace_launches(lambda: dr.PathIntegrator(**kw).renderC(scene)) == 2
+    spec.cameras[0].height, spec.cameras[0].width = 499, 491
+    scene, _ = to_torch_scene(spec)
+    for lanes in (2, 4, 7):
+        batch = dr.BatchRender(dr.PathIntegrator(batch_lanes=lanes, **kw), [scene], differentiable=False)
+        tiles = max(lanes, -(-499 * 491 * spp // (1 << 21)))
+        assert _trace_launches(batch.forward) == 2 * tiles, lanes

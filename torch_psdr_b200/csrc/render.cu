@@ -3513,7 +3513,9 @@ static int group_pixels(int spp) {
 // groups, and with them the gradients, are then the same for any such tile size.
 std::vector<Tile> plan_tiles(const std::vector<DevView>& views, int cap) {
   std::vector<Tile> tiles;
-  if (!views.empty()) {  // (the views of a job share their spp)
+  long long total = 0;
+  for (const DevView& v : views) total += (long long)v.H * v.W * v.spp;
+  if (total > cap) {  // (the views of a job share their spp)
     const int spp = views[0].spp, unit = group_pixels(spp);
     const int pixels = cap / spp;
     if (pixels > unit) cap = spp * (pixels / unit * unit);
@@ -3735,8 +3737,10 @@ int choose_cap(const psdr_config& cfg, const std::vector<DevView>& views, bool b
   long long cap = cfg.tile_paths > 0 ? cfg.tile_paths : auto_tile(cfg, need, backward && records, ws);
   if (backward) {
     if (cfg.tile_paths == 0) {
-      // (as few tiles as one per lane, but no smaller than 2^20)
-      if (lanes > 1) cap = std::min({cap, kTileBatch, std::max(kTileMin, (total + lanes - 1) / lanes)});
+      // (as few tiles as one per lane, of whole groups of paths, but no smaller than 2^20)
+      const long long group = (long long)group_pixels(cfg.spp_interior) * cfg.spp_interior;
+      const long long share = ((total + lanes - 1) / lanes + group - 1) / group * group;
+      if (lanes > 1) cap = std::min({cap, kTileBatch, std::max(kTileMin, share)});
       cap = std::min(cap, need);
     }
     long long cells = std::max<long long>(cfg.primary_edge_hypercube_resolution,
