@@ -3761,32 +3761,36 @@ int choose_cap(const psdr_config& cfg, const std::vector<DevView>& views, bool b
 // Mass / prefix-sum buffers of the hypercube cells and pixel-border segments.
 void psdr_workspace::ensure_mass(long long n, cudaStream_t st) {
   if (n <= mass_cap) return;
-  mass_cap = n;
+  mass_cap = 0;  // (until all of them are there: an allocation may fail)
   mass.alloc(4 * (size_t)n, st);
   mass_d.alloc(8 * (size_t)n, st);
   mass_pre.alloc(8 * (size_t)n, st);
   scan_tmp.alloc(8 * (psdr::scan_tmp_doubles((int)n) + 64), st);
+  mass_cap = n;
 }
 
 void psdr_workspace::ensure(int c, int r, int d, int nv, int rec_needed, cudaStream_t st) {
   using namespace psdr;
   stream = st;
   if (c > cap || r > R || d > D) {
-    cap = std::max(c, cap);
-    R = std::max(r, R);
-    D = std::max(d, D);
-    const size_t n = (size_t)cap;
+    const int cap1 = std::max(c, cap), R1 = std::max(r, R), D1 = std::max(d, D);
+    cap = 0;  // until all of the buffers are there: an allocation may fail
+    const size_t n = (size_t)cap1;
     rs.alloc(8 * n, st); ri.alloc(8 * n, st); view.alloc(4 * n, st); pix.alloc(4 * n, st);
     T.alloc(16 * n, st); L.alloc(16 * n, st); cur.alloc(16 * n, st); org.alloc(16 * n, st);
     q0.alloc(4 * n, st); q1.alloc(4 * n, st); qs.alloc(4 * n, st);
     cnt.alloc(sizeof(int) * 2 * (kMaxDepth + 2), st);
-    ro.alloc(16 * n * R, st); rd.alloc(16 * n * R, st); ra.alloc(16 * n * R, st); hit.alloc(16 * n * R, st);
+    ro.alloc(16 * n * R1, st); rd.alloc(16 * n * R1, st); ra.alloc(16 * n * R1, st); hit.alloc(16 * n * R1, st);
+    cap = cap1;
+    R = R1;
+    D = D1;
   }
   // the records of the job's tile, which may be smaller than what an earlier job left
   if (rec_needed) rec.alloc(16 * (size_t)c * (1 + (size_t)d * r + 2 * (size_t)d), st);
   if (nv > nviews_cap) {
-    nviews_cap = nv;
+    nviews_cap = 0;
     views.alloc(sizeof(DevView) * nv, st);
+    nviews_cap = nv;
   }
   wf.cap = cap;
   wf.rs = rs.as<unsigned long long>(); wf.ri = ri.as<unsigned long long>();
@@ -3989,12 +3993,13 @@ void ensure_border(psdr_workspace* ws, const psdr_config& cfg, const std::vector
   for (const BwdUnit& u : backward_units(views, cfg, cap, gi)) samples = std::max(samples, u.samples);
   for (const DevView& v : views)
     if (unb) mass = std::max({mass, border_segments(v), (long long)kCreaseCap, (long long)v.scene_ntri});
-  ws->eb_cap = std::max(ws->eb_cap, std::min<long long>(samples, cap));
-  const size_t n = (size_t)ws->eb_cap;
+  const size_t n = (size_t)std::max(ws->eb_cap, std::min<long long>(samples, cap));
+  ws->eb_cap = 0;
   ws->eb_a.alloc(16 * n, st);
   ws->eb_n.alloc(16 * n, st);
   ws->eb_hb.alloc(16 * n, st);
   ws->eb_La.alloc(16 * n, st);
+  ws->eb_cap = (long long)n;
   ws->hc_pmf.alloc(4 * (size_t)std::max(cells1, cells2), st);
   ws->hc_cmf.alloc(4 * (size_t)std::max(cells1, cells2), st);
   ws->ensure_mass(mass, st);
