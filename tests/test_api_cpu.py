@@ -144,6 +144,58 @@ def test_records_of_all_graphs_share_one_limit(monkeypatch, size):
     for _ in range(5):
         assert first._new_records(None, [None]) is not None
     assert mem.free == free and mem.queries == 0
-    # memory that went elsewhere since is asked for, not assumed
-    mem.free, mem.reserved = size // 2, 0
-    assert first._new_records(None, [None]) is None or size <= 64 << 20
+
+
+def _graph(monkeypatch, limit):
+    """renderD over fakes: forwards and backwards run out of memory while records are held and
+    `limit` (the calls that may fail) is not used up. Returns the integrator and its calls."""
+    calls = []
+
+    class Integ:
+        def _new_records(self, scene, cams):
+            return api._Records(_OnGpu([], 0), "stamp")
+
+        def _render(self, scene, cams=None, records=None):
+            calls.append(("fwd", records is not None))
+            if records is not None and "fwd" in limit:
+                raise api.L.PsdrOutOfMemory("fwd")
+            return [torch.ones(2)]
+
+        def _backward(self, scene, grads, torch_vars, records=None):
+            calls.append(("bwd", records is not None))
+            if records is not None and "bwd" in limit:
+                raise api.L.PsdrOutOfMemory("bwd")
+            return [torch.full((2,), 3.0) for _ in torch_vars]
+
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: "stream")
+    scene = types.SimpleNamespace(_camera_descs=lambda: "cams")
+    return Integ(), scene, calls
+
+
+@pytest.mark.parametrize("limit,want", [
+    ((), [("fwd", True), ("bwd", True)]),
+    (("fwd",), [("fwd", True), ("fwd", False), ("bwd", False)]),
+    (("bwd",), [("fwd", True), ("bwd", True), ("bwd", False)])])
+def test_records_are_dropped_when_the_library_runs_out_of_memory(monkeypatch, limit, want):
+    integ, scene, calls = _graph(monkeypatch, limit)
+    before = len(api._Records._alive)
+    x = torch.zeros(2, requires_grad=True)
+    (img,) = api._RenderD.apply(integ, scene, True, x)
+    assert len(api._Records._alive) == before + (limit != ("fwd",))
+    img.sum().backward()
+    assert calls == want and torch.equal(x.grad, torch.full((2,), 3.0))
+    assert len(api._Records._alive) == before
+
+
+def test_native_calls_get_torchs_cache_back(monkeypatch):
+    """An out-of-memory status empties torch's cache and repeats the call once."""
+    empties = []
+    monkeypatch.setattr(torch.cuda, "empty_cache", lambda: empties.append(1))
+    status = [api.L.PSDR_ERR_OOM, 0]
+    api._native(lambda: status.pop(0), "call")
+    assert empties == [1] and not status
+    with pytest.raises(api.L.PsdrOutOfMemory):
+        api._native(lambda: api.L.PSDR_ERR_OOM, "call")
+    with pytest.raises(ValueError):
+        api._native(lambda: api.L.PSDR_ERR_INVALID_ARG, "call")
+    assert empties == [1, 1]

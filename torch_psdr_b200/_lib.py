@@ -14,6 +14,7 @@ LIB_PATH = os.environ.get("PSDR_B200_LIB", os.path.join(HERE, "_lib", "libpsdr_b
 
 PSDR_OK = 0
 PSDR_ERR_INVALID_ARG = 1
+PSDR_ERR_OOM = 2
 PSDR_ERR_UNSUPPORTED = 6
 STATUS_NAMES = {0: "OK", 1: "INVALID_ARG", 2: "OOM", 3: "CUDA_ERROR", 4: "TIMEOUT", 5: "NUMERIC", 6: "UNSUPPORTED"}
 
@@ -138,6 +139,10 @@ class PsdrError(RuntimeError):
     pass
 
 
+class PsdrOutOfMemory(PsdrError):
+    pass
+
+
 def check(status: int, what: str = ""):
     if status == PSDR_OK:
         return
@@ -145,4 +150,4 @@ def check(status: int, what: str = ""):
     text = f"{what}: {STATUS_NAMES.get(status, status)}: {msg}"
     if status == PSDR_ERR_INVALID_ARG:
         raise ValueError(text)
-    raise PsdrError(text)
+    raise (PsdrOutOfMemory if status == PSDR_ERR_OOM else PsdrError)(text)

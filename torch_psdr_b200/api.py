@@ -63,6 +63,18 @@ def _check_index_buffers(jobs) -> None:
                 raise ValueError(f"{what} must lie in [0, {bound}): found values in [{out[2 * i]}, {out[2 * i + 1]}]")
 
 
+def _native(call, what: str) -> None:
+    """A native call that may allocate. Memory that torch keeps from freed tensors is out of the
+    library's reach: when the library runs out, torch gives its cache back and the call is
+    made once more (a call that failed has changed nothing)."""
+    try:
+        return L.check(call(), what)
+    except L.PsdrOutOfMemory:
+        pass
+    torch.cuda.empty_cache()
+    L.check(call(), what)
+
+
 def _stream():
     return C.c_void_p(torch.cuda.current_stream().cuda_stream)
 
@@ -405,7 +417,7 @@ class Scene(VarContex):
             lt._desc(next(values), box) if isinstance(lt, SH9Light) else lt._desc(next(values)) for lt in self.lights])
         desc = L.SceneDesc(md, len(self.meshes), ld, len(self.lights))
         handle = C.c_void_p()
-        L.check(lib.psdr_scene_create(C.byref(desc), _stream(), C.byref(handle)), "psdr_scene_create")
+        _native(lambda: lib.psdr_scene_create(C.byref(desc), _stream(), C.byref(handle)), "psdr_scene_create")
         self._handle = handle
         self._lib = lib
         self._builds = 0  # rebuilds since creation
@@ -469,7 +481,15 @@ class _RenderD(torch.autograd.Function):
     def forward(ctx, integrator, scene, keep, *torch_vars):
         cams = scene._camera_descs()
         ctx.records = integrator._new_records(scene, cams) if keep else None
-        imgs = integrator._render(scene, cams, ctx.records)
+        imgs = None
+        try:
+            imgs = integrator._render(scene, cams, ctx.records)
+        except L.PsdrOutOfMemory:
+            if ctx.records is None:
+                raise
+            ctx.records = None
+        if imgs is None:  # the records took the memory that the render needs
+            imgs = integrator._render(scene, cams)
         ctx.integrator = integrator
         ctx.scene = scene
         ctx.n_vars = len(torch_vars)
@@ -481,7 +501,15 @@ class _RenderD(torch.autograd.Function):
     def backward(ctx, *grads):
         grads = [g if g is not None else None for g in grads]
         records, ctx.records = ctx.records, None  # a second backward re-traces the paths
-        out = ctx.integrator._backward(ctx.scene, grads, ctx.vars, records)
+        out = None
+        try:
+            out = ctx.integrator._backward(ctx.scene, grads, ctx.vars, records)
+        except L.PsdrOutOfMemory:
+            if records is None:
+                raise
+            records = None
+        if out is None:
+            out = ctx.integrator._backward(ctx.scene, grads, ctx.vars)
         return (None, None, None) + tuple(out)
 
 
@@ -503,6 +531,8 @@ class _Records:
     @staticmethod
     def held(device) -> int:
         """Bytes of the records on a GPU that autograd graphs hold now."""
+        if not _Records._alive:
+            return 0
         with _Records._lock:
             return sum(r.data.numel() for r in _Records._alive if r.data.device == device)
 
@@ -658,9 +688,9 @@ class PathIntegrator:
         imgs = [torch.empty((c.height, c.width, 3), dtype=torch.float32, device="cuda") for c in scene.cameras]
         ptrs = (C.c_void_p * len(imgs))(*[i.data_ptr() for i in imgs])
         cams = scene._camera_descs() if cams is None else cams
-        L.check(self._lib.psdr_render_fwd_records(scene.handle, self._workspace(), cams, len(imgs), C.byref(self.cfg),
-                                                  ptrs, None if records is None else records.data.data_ptr(),
-                                                  _stream()), "psdr_render_fwd")
+        rec = None if records is None else records.data.data_ptr()
+        _native(lambda: self._lib.psdr_render_fwd_records(scene.handle, self._workspace(), cams, len(imgs),
+                                                          C.byref(self.cfg), ptrs, rec, _stream()), "psdr_render_fwd")
         return imgs
 
     def _stamp(self, scene: Scene, cams):
@@ -680,16 +710,15 @@ class PathIntegrator:
         L.check(self._lib.psdr_records_bytes(cams, len(cams), C.byref(self.cfg), C.byref(n)), "psdr_records_bytes")
         n = int(n.value)
         # All graphs' records together may take a quarter of the memory there would be without
-        # them. The query takes a third of a millisecond: it is left out up to 64 MB in all, and
-        # for what was granted before as long as torch's cache still holds the memory.
+        # them. The query takes 0.1 to 0.3 ms: it is left out up to 64 MB in all and for totals
+        # granted before (should the memory have gone elsewhere since, _RenderD drops the records).
         dev = torch.device("cuda", torch.cuda.current_device())
         total = _Records.held(dev) + n
-        if self.cfg.batch_records == 0 and total > 64 << 20:
+        if self.cfg.batch_records == 0 and total > max(64 << 20, self._records_granted):
             stats = torch.cuda.memory_stats_as_nested_dict(dev)
             cached = stats["reserved_bytes"]["all"]["current"] - stats["allocated_bytes"]["all"]["current"]
-            if total > self._records_granted or n > cached:
-                if total > (torch.cuda.mem_get_info(dev)[0] + cached + total - n) // 4:
-                    return None
+            if total > (torch.cuda.mem_get_info(dev)[0] + cached + total - n) // 4:
+                return None
         try:
             data = torch.empty(n, dtype=torch.uint8, device=dev)
         except torch.OutOfMemoryError:
@@ -800,8 +829,9 @@ class PathIntegrator:
         dp = (P * len(dimgs))(*[d.data_ptr() for d in dimgs])
         cams = scene._camera_descs()
         rec = None if records is None else records.pointer(self._stamp(scene, cams))
-        L.check(self._lib.psdr_render_bwd_records(scene.handle, self._workspace(), cams, len(dimgs), C.byref(self.cfg),
-                                                  dp, C.byref(tg), rec, _stream()), "psdr_render_bwd")
+        _native(lambda: self._lib.psdr_render_bwd_records(scene.handle, self._workspace(), cams, len(dimgs),
+                                                          C.byref(self.cfg), dp, C.byref(tg), rec, _stream()),
+                "psdr_render_bwd")
         # map the accumulators onto the input tensors (a tensor may play several roles)
         acc = {}
 
@@ -915,8 +945,8 @@ class BatchRender:
         self._keep += [tgt, sh, cd, csc, ip, dp]
         h = C.c_void_p()
         torch.cuda.synchronize()
-        L.check(self.lib.psdr_batch_create(sh, len(self.scenes), cd, csc, len(cams), C.byref(integrator.cfg), ip, dp,
-                                           tgt, C.byref(h)), "psdr_batch_create")
+        _native(lambda: self.lib.psdr_batch_create(sh, len(self.scenes), cd, csc, len(cams), C.byref(integrator.cfg), ip,
+                                                   dp, tgt, C.byref(h)), "psdr_batch_create")
         self._handle = h
 
     def forward(self) -> List[Tensor]:
