@@ -104,9 +104,9 @@ typedef struct {
 } psdr_camera_desc;
 
 /* PathIntegrator::Config (path_integrator.h:8-21; torch_psdr.py:478-536) plus the
- * B200 extensions: estimator, tile_paths (wavefront tile, 0 = 2^20 to 2^22 paths by job and
- * free memory; see
- * psdr_autotune), leaf_size
+ * B200 extensions: estimator, tile_paths (wavefront tile, 0 = 2^20 to 2^22 paths by job,
+ * lanes and free memory, see psdr_autotune; images do not depend on it, gradients only where
+ * a tile holds less than a whole group of 32 paths in whole pixels), leaf_size
  * (BVH leaf collapse, 0 = default), terms, spp_pixel_boundary and seed (0 = the
  * reference's sample streams; seed s offsets every stream index by s * 2654435761
  * modulo 2^32).
@@ -152,8 +152,9 @@ typedef struct {
                             max_bounce, R = light + BSDF samples + 1) and the backward runs the
                             adjoint from them instead of re-tracing the paths. 0 = when they
                             fit in a quarter of the free device memory (a batch asks at
-                            psdr_batch_create), 1 = always, -1 = never (re-trace, memory O(tile)). Gradients are
-                            bitwise the same either way. */
+                            psdr_batch_create; renderD counts the records of every live graph
+                            together), 1 = always, -1 = never (re-trace, memory O(tile)).
+                            Gradients are bitwise the same either way. */
 } psdr_config;
 
 /* Gradient outputs of psdr_render_bwd (caller-owned device buffers, fp32).

@@ -623,8 +623,10 @@ class PathIntegrator:
         and its backward's interior tiles and per-view boundary terms; 1..8, 0 = 4; the
         gradients do not depend on it), batch_records (renderD and BatchRender: the forward keeps
         every interior path's replay record and the backward runs the adjoint from them
-        instead of re-tracing; 0 = when they fit in a quarter of the free device memory,
-        1 = always, -1 = never; the gradients do not depend on it).
+        instead of re-tracing; 0 = when they fit in a quarter of the free device memory
+        (renderD: together with those of every other image whose graph is still alive; an
+        image kept without a backward holds its records), 1 = always, -1 = never; the
+        gradients do not depend on it).
         """
         assert n_pass > 0
         assert spp_interior > 0

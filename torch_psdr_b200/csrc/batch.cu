@@ -23,8 +23,8 @@ struct psdr_batch {
   psdr_config cfg{};
   psdr_workspace ws;
   psdr::DBuf scenes_dev;  // DevScene array, one entry per scene
-  psdr::DBuf campos;      // fp64 camera-origin accumulators, 3 per view
-  psdr::DBuf lens;        // fp64 camera-lens accumulators, kLensAcc per view
+  psdr::DBuf campos;      // camera-origin accumulators (GradAcc), 3 per view
+  psdr::DBuf lens;        // camera-lens accumulators (GradAcc), kLensAcc per view
   int cap = 0;
   bool backward = false;
   bool rebuild = true;
@@ -322,8 +322,8 @@ PSDR_API psdr_status psdr_batch_forward(psdr_batch* b, void* stream) {
   return PSDR_OK;
 }
 
-// Backward of every view (interior replay + adjoint, both edge terms), fp64
-// accumulation, then the fp32 gradient outputs bound at creation.
+// Backward of every view (interior adjoint, from kept records or a replay, and the boundary
+// terms), fixed-point accumulation, then the fp32 gradient outputs bound at creation.
 PSDR_API psdr_status psdr_batch_backward(psdr_batch* b, void* stream) {
   try {
     PSDR_CHECK(b != nullptr, "null batch");

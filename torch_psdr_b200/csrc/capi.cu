@@ -462,7 +462,7 @@ psdr_status psdr_scene_create(const psdr_scene_desc* desc, void* stream, psdr_sc
     check_index_ranges(desc, stream);
     s->grad_texels = texoff;
     psdr_scene_alloc(s);
-    // fp64 gradient accumulators live with the scene
+    // the gradient accumulators live with the scene
     cudaStream_t st = s->stream;
     s->dev.grad_verts = s->g_verts.as<GradAcc>();
     PSDR_CUDA(cudaMemsetAsync(s->vmask.p, 1, std::max<size_t>(1, s->nvert), st));

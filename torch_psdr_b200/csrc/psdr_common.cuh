@@ -220,8 +220,8 @@ struct DevLight {
 // Per-triangle shading record, 6 x float4 (96 B) in original triangle order:
 //  [0] p0.xyz, area   [1] p1.xyz, obj(bits)   [2] p2.xyz, uv0.x
 //  [3] n.xyz, uv0.y   [4] t.xyz, uv1.x        [5] uv1.y, uv2.x, uv2.y, 0
-// BVH node (4-wide, child boxes stored in the parent), 8 x float4 (128 B, 128-byte aligned):
-//  [0] lo.x of children 0..3 [1] hi.x [2] lo.y [3] hi.y [4] lo.z [5] hi.z [6] links (int) [7] -
+// BVH node (4-wide, child boxes stored in the parent), 7 x float4 (kNodeF4; 112 B, 16-byte aligned):
+//  [0] lo.x of children 0..3 [1] hi.x [2] lo.y [3] hi.y [4] lo.z [5] hi.z [6] links (int)
 // link >= 0: internal node; link < 0: leaf ~((first << 3) | (count-1)); 0x7fffffff: empty.
 // Leaf triangles, 3 x float4 (48 B) in BVH order: p0.xyz + id(bits), p1.xyz, p2.xyz.
 constexpr int kMaxLightVerts = 8;  // light vertices whose gradients the adjoint sums per lane

@@ -136,7 +136,7 @@ struct psdr_scene {
   // build scratch
   psdr::DBuf keys, vals, aux_i, aux_i2, aux_d, aux_d2, aabb, box_levels, flags, cbox;
   psdr::SortTmp sort_tmp;
-  // fp64 gradient accumulators (allocated on first backward)
+  // fixed-point gradient accumulators (GradAcc), parts of the slab
   psdr::DBuf g_verts, g_tex, g_emit;
   psdr::DBuf vmask;  // per-vertex gradient mask (set from the gradient targets of a backward)
   std::vector<size_t> tex_grad_off;  // per object offset into g_tex (doubles), SIZE_MAX if none

@@ -224,7 +224,9 @@ PSDR_D float mis_light_bound(const DevScene& sc, float3 o, float3 d) {
 // the ray, while the other rays of the warp wait. The test adds 6 us to a small launch of this
 // kernel, which is what k_trace saves on 2^18 paths (plain 128^2 x 16 spp render); 2^20 paths
 // of 256^2 x 16 spp: k_trace 595 -> 566 us for 11 us more here; 2^22 of 256^2 x 64 spp: 1.18 ->
-// 1.05 ms for 0.02.
+// 1.05 ms for 0.02. The form holds for every depth of a loop, since it pays at the late ones too:
+// with the list at the first depth only, the first two, the first three and all, the large
+// render (depth 5) takes 17.78, 17.72, 17.68 and 17.67 ms, its batched step 87.5, 87.3, 87.2, 87.1.
 constexpr int kListMin = 1 << 19;
 template <int MODE, bool BSDF, bool LIST>
 __global__ void __launch_bounds__(256) k_shade(WF w, const DevScene* __restrict__ scenes,
@@ -332,9 +334,9 @@ __global__ void __launch_bounds__(256) k_shade(WF w, const DevScene* __restrict_
 // at least half a warp. The fetch counter is w.cnt[2D+2], reset by k_shade.
 //
 // Bound by instruction issue and divergence, not by memory: on 256^2 x 32 spp rays of the
-// icosphere scene the SMs issue on 79 % of the cycles with 18.8 of 32 lanes active at the first
+// icosphere scene the SMs issue on 79 % of the cycles with 18.7 of 32 lanes active at the first
 // depth, 68 % and 16 at the third (11 before lanes waited for one another at leaves,
-// trav_step); L1 64-82 %, L2 12-18 %, DRAM 2-3 % of their peaks. Traversal
+// trav_step); L1 64-82 %, L2 12-19 %, DRAM 2-3 % of their peaks. Traversal
 // of the 512^2 x 32 spp icosphere step: 14.0 ms before, 12.2 ms now (2^20-path tiles).
 constexpr int kRefill = 16;
 // Per-lane memory of k_trace: the first kShort stack entries, the ray as the triangle test
@@ -1140,13 +1142,13 @@ PSDR_D void scatter_tex_warp(const DevTex* tx, int off, float3 a, bool active) {
   if ((threadIdx.x & 31) == 0) scatter_tex(*tx, off, f3(v0, v1, v2), false);
 }
 
-// ------------------------------------------------------------------ adjoint kernel
-// One thread per path of the tile: the replay stored each depth's contribution C_d
-// and throughput factor beta_d, so the suffix radiances S_d = C_d + beta_d S_{d+1}
-// come straight from the records; the path is then walked forward once, replaying
-// its sampler stream, and every depth's reverse-mode adjoint is applied
-// (PSDR_EST_REFERENCE: pdfs and MIS weights are constants, jacobi = area/detach(area),
-// barycentrics are not differentiated), scattering into fp64 accumulators.
+// ------------------------------------------------------------------ adjoint kernels
+// The records hold each depth's contribution C_d and throughput factor beta_d, so the suffix
+// radiances S_d = C_d + beta_d S_{d+1} come straight from them; every path's vertices are then
+// visited from the camera on, replaying its sampler stream, and every depth's reverse-mode
+// adjoint is applied (PSDR_EST_REFERENCE: pdfs and MIS weights are constants, jacobi =
+// area/detach(area), barycentrics are not differentiated), scattering into the fixed-point
+// accumulators: k_adjoint, from per-warp lists, and k_adjoint_ext, one thread per path.
 PSDR_D float3 suffix_radiance(const WF& w, int s, int from) {
   float3 S = f3(0.f, 0.f, 0.f);
   for (int k = w.D - 1; k >= from; --k) S = xyz(rec_c(w, s, k)) + mul(xyz(rec_beta(w, s, k)), S);
@@ -1251,9 +1253,10 @@ __host__ __device__ constexpr int adj_warp_words(int nB) { return kVertFields * 
 // each path to its end instead (one thread per path over all depths) ran every depth's code
 // for the few paths still alive, and the BSDF-sample code for two lanes of a warp on average:
 // 5.8 ms per 512^2 x 32 spp x depth 3 step against 2.9 ms with lists; 2.3 ms with the warps of a
-// block starting together. Bound by the latency of its record loads (6.4 cycles per issued
-// instruction at 24 % occupancy, 128 registers; DRAM 8 % busy); instruction fetch is down from
-// 7.2 cycles to 1.0, for 3.3 at the block's barrier.
+// block starting together (2.8 ms in tiles of 2^22 paths whose records lie in HBM: 2.76 with fp32
+// sums per thread, 2.83 with exact ones). Bound by the latency of its record loads (6.2 cycles
+// per issued instruction at 24 % occupancy, 128 registers; DRAM 8 % busy); instruction fetch is
+// down from 7.2 cycles to 1.3, for 3.1 at the block's barrier.
 // Without vertex gradients (VERTS false: texture and emission optimisation) the lists carry no
 // surface adjoint and the vertex scatters go; 256^2 x 64 spp: 0.83 -> 0.55 ms (three blocks per
 // SM spill: 0.63 ms).
@@ -3690,7 +3693,10 @@ static size_t path_bytes(const psdr_config& cfg, bool records) {
 // smallest). Every launch over a tile ends with its warps draining their last rays (50 to
 // 120 node visits for the longest against 14 on average), about 60 us in which the lanes
 // empty out; larger tiles pay for it less often. 1.31 M triangles, 1024^2 x 16 spp, depth 5:
-// traversal 18.2 ms with 2^20-path tiles, 14.7 with 2^21, 13.0 with 2^22.
+// traversal 18.2 ms with 2^20-path tiles, 14.7 with 2^21, 13.0 with 2^22. A workspace's first job
+// maps its memory, 0.3 KB per path of the tile: at 2^22 about 5 ms more than at 2^20, once (first
+// pass of a new integrator against its later ones: 256^2 x 64 spp step 11.1 and 3.3 ms,
+// 1024^2 x 16 spp render 20.5 and 17.7 ms).
 // A workspace that already holds such a tile keeps it without asking for the free memory. The
 // choice changes no image and no gradient (plan_tiles): samples per pixel for which the smallest
 // tile could cut a group of 32 paths get that tile always.
@@ -3717,7 +3723,8 @@ static long long auto_tile(const psdr_config& cfg, long long need, bool records,
 
 // lanes: concurrent tiles of a batch; its automatic tile is small enough for each lane to
 // get one, and at most 2^21 (the lanes' tiles fill one another's tails: 2^22 is no faster), but no
-// smaller than 2^20.
+// smaller than 2^20. 512^2 x 32 spp step in four lanes: 15.6 ms at 2^20, 14.9 at 2^21, for 1.4 GB
+// more memory and 34 ms to create the batch against 29; 1024^2 x 32 spp: 91.5 and 87.3 ms.
 int choose_cap(const psdr_config& cfg, const std::vector<DevView>& views, bool backward, int lanes,
                const psdr_workspace* ws, bool records) {
   int maxspp = 1;
