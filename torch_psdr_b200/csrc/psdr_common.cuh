@@ -141,12 +141,14 @@ PSDR_D long long own_units(float v) {  // 0 for the contributions that own_carry
 }
 // |lo| >= 2^61: the top three bits differ.
 PSDR_D unsigned own_top(long long lo) { return ((unsigned)(lo >> 32) + 0x20000000u) & 0xC0000000u; }
-static __device__ __noinline__ void own_carry(long long& lo, long long& hi, float v) {
+// Returns lo without its carry (by value: only hi need lie in memory).
+static __device__ __noinline__ long long own_carry(long long lo, long long* hi, float v) {
   if (own_top(lo)) {
-    hi += lo >> 32;
+    *hi += lo >> 32;
     lo &= 0xffffffffll;
   }
-  if (fabsf(v) >= kOwnMax && isfinite(v)) hi += __float2ll_rn(fminf(fmaxf(v, -4398046511104.f), 4398046511104.f) * 1048576.f);
+  if (fabsf(v) >= kOwnMax && isfinite(v)) *hi += __float2ll_rn(fminf(fmaxf(v, -4398046511104.f), 4398046511104.f) * 1048576.f);
+  return lo;
 }
 // lo and hi of three accumulators, one test for all.
 PSDR_D bool own_add3(long long* lo, float3 v) {
@@ -179,9 +181,9 @@ struct Own3 {
   long long lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
   PSDR_D void add(float3 v) {
     if (own_add3(lo, v)) return;
-    own_carry(lo[0], hi[0], v.x);
-    own_carry(lo[1], hi[1], v.y);
-    own_carry(lo[2], hi[2], v.z);
+    lo[0] = own_carry(lo[0], hi, v.x);
+    lo[1] = own_carry(lo[1], hi + 1, v.y);
+    lo[2] = own_carry(lo[2], hi + 2, v.z);
   }
   PSDR_D void put(GradAcc* a) const {
 #pragma unroll

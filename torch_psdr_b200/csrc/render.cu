@@ -632,9 +632,11 @@ PSDR_D SurfAdj zero_adj() {
 // They belong to one scene; a lane that goes on to another scene's paths adds them to the
 // accumulators first. (In jobs with several scenes the emission gradients used to go to the
 // accumulators one by one, every lane of the GPU adding to the same few words: a 9-view step
-// over three scenes took 67.2 ms, 51.5 with sums per lane.) Their exact integers cost about a
-// twentieth of the adjoint kernels' time against fp32 sums, which lose the small terms
-// and depend on how paths are dealt to lanes.
+// over three scenes took 67.2 ms, 51.5 with sums per lane.) Against fp32 sums, which lose small
+// terms and depend on how paths are dealt to lanes, the exact ones cost k_adjoint up to 5 % (489
+// and 510 us, 250^2 x 16 spp with every gradient; 2.78 and 2.75 ms, 512^2 x 32 spp with vertices)
+// and k_adjoint_ext 1 to 7 % (2.85 and 3.04 ms, 377 x 97 x 96 spp). Only the sums in use are cleared
+// and flushed: all 36 of a lane, at each change of scene too, took 1 to 3 % more.
 constexpr int kHotLights = 4;
 constexpr int kHotEmit = 3 * kMaxLightVerts;  // first emission sum
 constexpr int kHotSums = kHotEmit + 3 * kHotLights;
@@ -649,41 +651,49 @@ PSDR_D void hot_init(HotAcc& hot) {
   hot.sc = nullptr;
   hot.lv0 = hot.nlv = hot.nlt = 0;
   hot.high = false;
-#pragma unroll
-  for (int k = 0; k < kHotSums; ++k) hot.lo[k] = 0;
 }
 static __device__ __noinline__ void hot_carry(HotAcc& hot, int k, float3 v) {
   if (!hot.high) {
     for (int q = 0; q < kHotSums; ++q) hot.hi[q] = 0;
     hot.high = true;
   }
-  own_carry(hot.lo[k], hot.hi[k], v.x);
-  own_carry(hot.lo[k + 1], hot.hi[k + 1], v.y);
-  own_carry(hot.lo[k + 2], hot.hi[k + 2], v.z);
+  hot.lo[k] = own_carry(hot.lo[k], hot.hi + k, v.x);
+  hot.lo[k + 1] = own_carry(hot.lo[k + 1], hot.hi + k + 1, v.y);
+  hot.lo[k + 2] = own_carry(hot.lo[k + 2], hot.hi + k + 2, v.z);
 }
 // Adds v to sums k, k + 1, k + 2 (a dynamic index: the sums live in local memory, L1).
 PSDR_D void hot_add(HotAcc& hot, int k, float3 v) {
   if (!own_add3(hot.lo + k, v)) hot_carry(hot, k, v);
 }
 PSDR_D GradAcc* hot_target(const HotAcc& hot, int k) {
-  return k < kHotEmit ? hot.sc->grad_verts + 3 * (size_t)hot.lv0 + k
-                      : hot.sc->lights[(k - kHotEmit) / 3].grad_emit + (k - kHotEmit) % 3;
+  if (k < kHotEmit) return hot.sc->grad_verts + 3 * (size_t)hot.lv0 + k;
+  GradAcc* e = hot.sc->lights[(k - kHotEmit) / 3].grad_emit;
+  return e ? e + (k - kHotEmit) % 3 : nullptr;
+}
+// Calls f(sum) for the sums in use.
+template <class F>
+PSDR_D void hot_each(const HotAcc& hot, F f) {
+  for (int k = 0; k < 3 * hot.nlv; ++k) f(k);
+  for (int k = kHotEmit; k < kHotEmit + 3 * hot.nlt; ++k) f(k);
 }
 static __device__ __noinline__ void hot_spill(HotAcc& hot) {
   if (!hot.sc) return;
-  for (int k = 0; k < kHotSums; ++k) {
+  hot_each(hot, [&](int k) {
     const long long hi = hot.high ? hot.hi[k] : 0;
     if (hi | hot.lo[k]) acc_put(hot_target(hot, k), hi, hot.lo[k]);
-  }
+  });
   hot_init(hot);
 }
-PSDR_D void hot_bind(HotAcc& hot, const DevScene* sc) {
-  if (hot.sc == sc) return;
+static __device__ __noinline__ void hot_rebind(HotAcc& hot, const DevScene* sc) {
   hot_spill(hot);
   hot.sc = sc;
   hot.lv0 = sc->light_v0;
   hot.nlv = sc->light_nv > 0 && vert_wanted(*sc, sc->light_v0) ? sc->light_nv : 0;
   hot.nlt = min(sc->nlight, kHotLights);
+  hot_each(hot, [&](int k) { hot.lo[k] = 0; });
+}
+PSDR_D void hot_bind(HotAcc& hot, const DevScene* sc) {
+  if (hot.sc != sc) hot_rebind(hot, sc);
 }
 // End of a kernel (all lanes together): one addition per warp when its lanes share the scene.
 PSDR_D void hot_flush(HotAcc& hot) {
@@ -696,9 +706,9 @@ PSDR_D void hot_flush(HotAcc& hot) {
     return;
   }
   if (!own) hot_bind(hot, reinterpret_cast<const DevScene*>(first));
-  for (int k = 0; k < 3 * hot.nlv; ++k) acc_put_warp(hot_target(hot, k), hot.high ? hot.hi[k] : 0, hot.lo[k]);
-  for (int k = kHotEmit; k < kHotEmit + 3 * hot.nlt; ++k)
-    if (hot.sc->lights[(k - kHotEmit) / 3].grad_emit) acc_put_warp(hot_target(hot, k), hot.high ? hot.hi[k] : 0, hot.lo[k]);
+  hot_each(hot, [&](int k) {
+    if (GradAcc* to = hot_target(hot, k)) acc_put_warp(to, hot.high ? hot.hi[k] : 0, hot.lo[k]);
+  });
 }
 
 // Adjoint ae of an environment light's radiance at box uv (u, v), incoming direction wi:
@@ -799,8 +809,7 @@ PSDR_D void scatter_surf(const DevScene& sc, HotAcc& hot, int tri, float b1, flo
 // scatter_surf for a triangle that is not a light's: path vertices past the camera hit
 // (paths end at lights), whose vertices never fall in the light-vertex register range.
 // Out of line: the adjoint scatters from several depths' call sites.
-static __device__ __noinline__ void scatter_mesh(const DevScene& sc, int tri, float b1, float b2, bool front,
-                                                 SurfAdj a) {
+PSDR_D void scatter_verts(const DevScene& sc, int tri, float b1, float b2, bool front, const SurfAdj& a) {
   if (!sc.grad_verts) return;
   const int4 tv = __ldg(sc.tri_v + tri);
   if (!vert_wanted(sc, tv.x) && !vert_wanted(sc, tv.y) && !vert_wanted(sc, tv.z)) return;
@@ -809,6 +818,9 @@ static __device__ __noinline__ void scatter_mesh(const DevScene& sc, int tri, fl
   vert_add(sc, tv.x, g0);
   vert_add(sc, tv.y, g1);
   vert_add(sc, tv.z, g2);
+}
+static __device__ __noinline__ void scatter_mesh(const DevScene& sc, int tri, float b1, float b2, bool front, SurfAdj a) {
+  scatter_verts(sc, tri, b1, b2, front, a);
 }
 
 PSDR_D void scatter_tex(const DevTex& tx, int off, float3 a, bool /*unused*/) {
@@ -1158,26 +1170,30 @@ PSDR_D float3 suffix_radiance(const WF& w, int s, int from) {
 // Camera-origin adjoint summed per lane while consecutive samples share a view.
 struct CamAcc {
   const DevView* v = nullptr;
+  GradAcc* to = nullptr;  // its accumulators or null
   Own3 g;
   PSDR_D void add(const DevView* view, float3 a) {
     if (view != v) {
       flush();
       v = view;
+      to = view->grad_pos;
     }
-    if (v->grad_pos) g.add(a);
+    if (to) g.add(a);
   }
   PSDR_D void flush() {
-    if (v && v->grad_pos) g.put(v->grad_pos);
+    if (to) {
+      g.put(to);
+      g = Own3();
+    }
     v = nullptr;
-    g = Own3();
+    to = nullptr;
   }
   // End of a kernel: one addition per warp when the warp shares the view.
   PSDR_D void flush_warp() {
-    const unsigned long long key = (unsigned long long)v;
+    const unsigned long long key = (unsigned long long)to;
     const unsigned long long k0 = __shfl_sync(0xffffffffu, key, 0);
-    if (!__all_sync(0xffffffffu, key == k0) || !v) { flush(); return; }
-    if (v->grad_pos) g.put_warp(v->grad_pos);
-    v = nullptr;
+    if (!__all_sync(0xffffffffu, key == k0)) { flush(); return; }
+    if (to) g.put_warp(to);
   }
 };
 
@@ -1192,13 +1208,13 @@ PSDR_D float view_fxfy(const DevView& V) {
 }
 
 // Unbiased estimator, primary vertex: adjoint of the camera Jacobian ratio J/detach(J),
-// J = |n.(x-o)| / z^3, z = (x-o).look, scaled by phi = dot(dI, L).
-PSDR_D void cam_jacobian_adj(const DevView& V, const Surf& x, float phi, SurfAdj& ax, CamAcc& cam) {
+// J = |n.(x-o)| / z^3, z = (x-o).look, scaled by phi = dot(dI, L). Returns the camera origin's share.
+PSDR_D float3 cam_jacobian_adj(const DevView& V, const Surf& x, float phi, SurfAdj& ax) {
   if (V.ortho) {
     // J = |n.look|: only the normal moves it
     const float3 look = view_look(V);
     ax.n += look * (phi / dot(x.n, look));
-    return;
+    return f3(0.f, 0.f, 0.f);
   }
   const float3 rel = x.p - V.pos;
   const float nr = dot(x.n, rel);
@@ -1207,7 +1223,7 @@ PSDR_D void cam_jacobian_adj(const DevView& V, const Surf& x, float phi, SurfAdj
   ax.n += rel * (phi / nr);
   const float3 ap = x.n * (phi / nr) - look * (3.f * phi / z);
   ax.p += ap;
-  cam.add(&V, -ap);
+  return -ap;
 }
 
 // The camera end of a path (depth 0): its view, primary surface and pixel gradient.
@@ -1253,8 +1269,8 @@ __host__ __device__ constexpr int adj_warp_words(int nB) { return kVertFields * 
 // each path to its end instead (one thread per path over all depths) ran every depth's code
 // for the few paths still alive, and the BSDF-sample code for two lanes of a warp on average:
 // 5.8 ms per 512^2 x 32 spp x depth 3 step against 2.9 ms with lists; 2.3 ms with the warps of a
-// block starting together (2.8 ms in tiles of 2^22 paths whose records lie in HBM: 2.76 with fp32
-// sums per thread, 2.83 with exact ones). Bound by the latency of its record loads (6.2 cycles
+// block starting together (2.8 ms in tiles of 2^22 paths whose records lie in HBM, with fp32
+// or with exact sums per thread). Bound by the latency of its record loads (6.2 cycles
 // per issued instruction at 24 % occupancy, 128 registers; DRAM 8 % busy); instruction fetch is
 // down from 7.2 cycles to 1.3, for 3.1 at the block's barrier.
 // Without vertex gradients (VERTS false: texture and emission optimisation) the lists carry no
@@ -1337,7 +1353,7 @@ __global__ void __launch_bounds__(32 * kAdjWarps, 2) k_adjoint(WF w, const DevSc
             const float3 L = light_emit<false>(Lt, x);
             has0 = true;
             ax.area = dot(g, L) / x.area;
-            if (UNB) cam_jacobian_adj(V, x, dot(g, L), ax, cam);
+            if (UNB) cam.add(&V, cam_jacobian_adj(V, x, dot(g, L), ax));
             add_emit(*scp, hot, x.light, g);
           }
         } else {
@@ -1348,7 +1364,7 @@ __global__ void __launch_bounds__(32 * kAdjWarps, 2) k_adjoint(WF w, const DevSc
             rng.next_float();
             rng.next_float();
             ax.area = dot(g, L) / x.area;  // jacobi of the primary hit
-            if (UNB) cam_jacobian_adj(V, x, dot(g, L), ax, cam);
+            if (UNB) cam.add(&V, cam_jacobian_adj(V, x, dot(g, L), ax));
           }
         }
       }
@@ -1484,6 +1500,7 @@ __global__ void __launch_bounds__(128, 2) k_adjoint_ext(WF w, const DevScene* __
       const DevView& V = *Vp;
       const DevScene& sc = *scp;
       hot_bind(hot, scp);
+      float3 co = f3(0.f, 0.f, 0.f);  // the path's share of the camera origin's adjoint
       if (x0.is_light) {
         // camera ray on a light: L = emit at depth 0 when lights are visible
         if (w.light_vis) {
@@ -1491,14 +1508,14 @@ __global__ void __launch_bounds__(128, 2) k_adjoint_ext(WF w, const DevScene* __
           const float3 L = light_emit<true>(Lt, x0);
           has0 = true;
           ax0.area = dot(g, L) / x0.area;
-          if (UNB) cam_jacobian_adj(V, x0, dot(g, L), ax0, cam);
+          if (UNB) co = cam_jacobian_adj(V, x0, dot(g, L), ax0);
           if (Lt.kind == kLightArea) {
             add_emit(sc, hot, x0.light, g);
           } else {
             // an SH9 light's radiance depends on wi = -normalize(x0 - o): its share goes
             // to the ray origin, which moves with the camera
             const float3 aw = env_emit_adj(&Lt, x0.u, x0.v, x0.wi, g);
-            if (Lt.kind == kLightSh9) cam.add(&V, (aw - x0.wi * dot(x0.wi, aw)) / sqrtf(x0.sqd));
+            if (Lt.kind == kLightSh9) co += (aw - x0.wi * dot(x0.wi, aw)) / sqrtf(x0.sqd);
           }
         }
       } else {
@@ -1510,7 +1527,7 @@ __global__ void __launch_bounds__(128, 2) k_adjoint_ext(WF w, const DevScene* __
           rng.next_float();
           SurfAdj ax = zero_adj();
           ax.area = dot(g, L) / x0.area;  // jacobi of the primary hit
-          if (UNB) cam_jacobian_adj(V, x0, dot(g, L), ax, cam);
+          if (UNB) co = cam_jacobian_adj(V, x0, dot(g, L), ax);
           Surf xc = x0;
           int tric = __float_as_int(h0.x);
           float4 hc = h0;
@@ -1543,7 +1560,7 @@ __global__ void __launch_bounds__(128, 2) k_adjoint_ext(WF w, const DevScene* __
             const bool next = d < w.D - 1 && continuation_adj<UNB, true, true>(sc, xc, mp.color * kInvPi, rx, ry,
                                                                          rec_hit(w, s, d, w.nL + w.nB), adjB, ax, nextc, nx, none, &mp, &ma);
             const float3 aorg = mat_finalize(ob, xc, mp, ma, ax);
-            if (d == 0) cam.add(&V, aorg);
+            if (d == 0) co += aorg;
             else if (d == 1) ax0.p += aorg;
             else axq.p += aorg;
             if (triq >= 0) scatter_mesh(sc, triq, hq.y, hq.z, frontq, axq);
@@ -1572,6 +1589,7 @@ __global__ void __launch_bounds__(128, 2) k_adjoint_ext(WF w, const DevScene* __
           if (triq >= 0) scatter_mesh(sc, triq, hq.y, hq.z, frontq, axq);
         }
       }
+      if (has0) cam.add(&V, co);
     }
     scatter_surf_warp(scp, hot, __float_as_int(h0.x), h0.y, h0.z, x0.front, ax0, has0);
     scatter_tex_warp(tx0, toff0, atex0, has0);
@@ -1771,6 +1789,7 @@ __global__ void __launch_bounds__(256) k_edge_final_unb(WF w, const DevScene* __
   const DevScene& sc = scenes[V.scene];
   const float3 look = view_look(V);
   const float fxfy = view_fxfy(V);
+  GradAcc* const gpos = V.grad_pos;
   Own3 go;  // camera origin
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n32; s += stride) {
     if (s >= n || !V.dimage) continue;
@@ -1806,9 +1825,9 @@ __global__ void __launch_bounds__(256) k_edge_final_unb(WF w, const DevScene* __
       vert_add(sc, tv.y, ag * hg.y);
       vert_add(sc, tv.z, ag * hg.z);
     }
-    if (V.grad_pos) go.add(-(av * (1.f - ratio)));
+    if (gpos) go.add(-(av * (1.f - ratio)));
   }
-  if (V.grad_pos) go.put_warp(V.grad_pos);
+  if (gpos) go.put_warp(gpos);
 }
 
 // Between the two trace2light calls: keep L_a, restart the slot at the +eps hit with
@@ -1845,6 +1864,7 @@ __global__ void __launch_bounds__(256) k_edge_final(WF w, const DevScene* __rest
   const int n32 = (n + 31) & ~31;
   const DevView& V = views[v];
   const DevScene& sc = scenes[V.scene];
+  GradAcc* const gpos = V.grad_pos;
   Own3 go;  // camera origin
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n32; s += stride) {
     if (s >= n) continue;
@@ -1877,10 +1897,10 @@ __global__ void __launch_bounds__(256) k_edge_final(WF w, const DevScene* __rest
         vert_add(sc, ev.x, ax * (1.f - ss));
         vert_add(sc, ev.y, ax * ss);
       }
-      if (V.grad_pos) go.add((nflip - jo) * K);
+      if (gpos) go.add((nflip - jo) * K);
     }
   }
-  if (!PRE && V.grad_pos) go.put_warp(V.grad_pos);
+  if (!PRE && gpos) go.put_warp(gpos);
 }
 
 // ------------------------------------------------------------------ pixel borders
@@ -2005,6 +2025,7 @@ __global__ void __launch_bounds__(256) k_border_final(WF w, const DevScene* __re
   const int n32 = (n + 31) & ~31;
   const DevView& V = views[v];
   const DevScene& sc = scenes[V.scene];
+  GradAcc* const gpos = V.grad_pos;
   Own3 go;  // camera origin
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n32; s += stride) {
     if (s >= n || !V.dimage) continue;
@@ -2041,9 +2062,9 @@ __global__ void __launch_bounds__(256) k_border_final(WF w, const DevScene* __re
       vert_add(sc, tv.y, ag * h.y);
       vert_add(sc, tv.z, ag * h.z);
     }
-    if (V.grad_pos) go.add(-ag);
+    if (gpos) go.add(-ag);
   }
-  if (V.grad_pos) go.put_warp(V.grad_pos);
+  if (gpos) go.put_warp(gpos);
 }
 
 // ------------------------------------------------------------------ camera lens
@@ -2560,6 +2581,7 @@ __global__ void __launch_bounds__(256) k_crease_final(WF w, const DevScene* __re
   const int n32 = (n + 31) & ~31;
   const DevView& V = views[v];
   const DevScene& sc = scenes[V.scene];
+  GradAcc* const gpos = V.grad_pos;
   Own3 go;  // camera origin
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n32; s += stride) {
     if (s >= n || !V.dimage) continue;
@@ -2597,9 +2619,9 @@ __global__ void __launch_bounds__(256) k_crease_final(WF w, const DevScene* __re
       vert_add(sc, v2.y, a2 * b2.y);
       vert_add(sc, v2.z, a2 * b2.z);
     }
-    if (V.grad_pos) go.add(-(a1 + a2));  // moving the camera by d is moving both surfaces by -d
+    if (gpos) go.add(-(a1 + a2));  // moving the camera by d is moving both surfaces by -d
   }
-  if (V.grad_pos) go.put_warp(V.grad_pos);
+  if (gpos) go.put_warp(gpos);
 }
 
 // ------------------------------------------------------------------ BSDF jumps
@@ -2715,6 +2737,7 @@ __global__ void __launch_bounds__(256) k_jump_final(WF w, const DevScene* __rest
   const int n32 = (n + 31) & ~31;
   const DevView& V = views[v];
   const DevScene& sc = scenes[V.scene];
+  GradAcc* const gpos = V.grad_pos;
   Own3 go;  // camera origin
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n32; s += stride) {
     if (s >= n || !V.dimage) continue;
@@ -2759,17 +2782,17 @@ __global__ void __launch_bounds__(256) k_jump_final(WF w, const DevScene* __rest
     aa.p = du;
     ax.p = -du;
     const float3 ao = mat_finalize(ob, x, mp, ma, ax);
-    scatter_mesh(sc, tk, hk.y, hk.z, x.front, ax);
-    scatter_mesh(sc, ta, hn.y, hn.z, xa.front, aa);
+    scatter_verts(sc, tk, hk.y, hk.z, x.front, ax);
+    scatter_verts(sc, ta, hn.y, hn.z, xa.front, aa);
     if (tp >= 0) {
       SurfAdj ap = zero_adj();
       ap.p = ao;
-      scatter_mesh(sc, tp, hp.y, hp.z, true, ap);
-    } else if (!fixed_v && V.grad_pos) {
+      scatter_verts(sc, tp, hp.y, hp.z, true, ap);
+    } else if (!fixed_v && gpos) {
       go.add(ao);
     }
   }
-  if (V.grad_pos) go.put_warp(V.grad_pos);
+  if (gpos) go.put_warp(gpos);
 }
 
 // ------------------------------------------------------------------ direct edges
