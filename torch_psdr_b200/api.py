@@ -8,7 +8,6 @@ calls psdr_render_bwd (the path-replay adjoint).
 """
 from __future__ import annotations
 
-import contextlib
 import ctypes as C
 import json
 import os
@@ -49,18 +48,25 @@ def _check_index_buffers(jobs) -> None:
     kernel and one host read for all of them, on the GPU that holds them (which need not be
     the current one)."""
     jobs = [j for j in jobs if j[0].numel()]
-    for dev in dict.fromkeys(t.device for t, _, _ in jobs):
-        own = [j for j in jobs if j[0].device == dev]
-        n = len(own)
-        ptrs = (C.c_void_p * n)(*[t.data_ptr() for t, _, _ in own])
-        counts = (C.c_int64 * n)(*[t.numel() for t, _, _ in own])
-        out = (C.c_int32 * (2 * n))()
-        # (entering a device takes 10 us, as long as the kernel: left out for the current one)
-        with contextlib.nullcontext() if dev.index == torch.cuda.current_device() else torch.cuda.device(dev):
-            L.check(L.load().psdr_index_bounds(ptrs, counts, n, out, _stream()), "psdr_index_bounds")
-        for i, (_, bound, what) in enumerate(own):
-            if out[2 * i] < 0 or out[2 * i + 1] >= bound:
-                raise ValueError(f"{what} must lie in [0, {bound}): found values in [{out[2 * i]}, {out[2 * i + 1]}]")
+    n = len(jobs)
+    if n == 0:
+        return
+    dev = jobs[0][0].device
+    if n > 1 and any(j[0].device != dev for j in jobs):
+        for d in dict.fromkeys(j[0].device for j in jobs):
+            _check_index_buffers([j for j in jobs if j[0].device == d])
+        return
+    if dev.index != torch.cuda.current_device():  # (entering a device takes 10 us, as long as the kernel)
+        with torch.cuda.device(dev):
+            _check_index_buffers(jobs)
+        return
+    ptrs = (C.c_void_p * n)(*[t.data_ptr() for t, _, _ in jobs])
+    counts = (C.c_int64 * n)(*[t.numel() for t, _, _ in jobs])
+    out = (C.c_int32 * (2 * n))()
+    L.check(L.load().psdr_index_bounds(ptrs, counts, n, out, _stream()), "psdr_index_bounds")
+    for i, (_, bound, what) in enumerate(jobs):
+        if out[2 * i] < 0 or out[2 * i + 1] >= bound:
+            raise ValueError(f"{what} must lie in [0, {bound}): found values in [{out[2 * i]}, {out[2 * i + 1]}]")
 
 
 def _native(call, what: str) -> None:
