@@ -283,8 +283,9 @@ PSDR_D int discrete_sample(const float* __restrict__ pmf, const float* __restric
 //
 // The test works in coordinates permuted so that the ray's largest direction component comes
 // last. The published test also swaps the other two for a negative component, to keep the
-// winding; that only negates U, V, W and det together, exactly, so it is left out: t and the
-// barycentrics are the same bits.
+// winding; that only negates U, V, W and det together, exactly but for zeros (whose sign a
+// difference does not take), so it is left out up to the barycentrics of an accepted hit: t and
+// they are the same bits.
 struct RayPre {
   float3 o;
   int kz;            // the axis that comes last; the order is (kz + 1, kz + 2, kz) mod 3
@@ -325,6 +326,11 @@ PSDR_D bool tri_test(const RayPre& r, float3 p0, float3 p1, float3 p2, float tmi
   float tt = __fdiv_rn(T, det);
   if (!(tt > tmin && tt <= tmax)) return false;
   t = tt;
+  if (r.Sz < 0.0f) {  // as with the swap, down to the signs of zeros (hits on edges)
+    V = __fsub_rn(__fmul_rn(Ay, Cx), __fmul_rn(Ax, Cy));
+    W = __fsub_rn(__fmul_rn(By, Ax), __fmul_rn(Bx, Ay));
+    det = -det;
+  }
   b1 = __fdiv_rn(V, det);
   b2 = __fdiv_rn(W, det);
   return true;
