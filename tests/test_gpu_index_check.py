@@ -44,7 +44,7 @@ def test_threads_get_their_own_bounds(cuda):
     assert not wrong, wrong[:3]
 
 
-@pytest.mark.parametrize("n,bad", [(31, None), (32, 31), (33, 32), (70, 64), (70, None)])
+@pytest.mark.parametrize("n,bad", [(31, None), (32, 31), (33, 32), (70, 64), (256, 255), (257, 255), (300, None)])
 def test_scene_of_many_meshes(cuda, n, bad):
     """More index buffers than one launch checks; an index out of range in the last of them."""
     V, F = synth.quad((0.0, 0.0), 1.0, 0.0, facing_down=False)

@@ -178,7 +178,8 @@ using namespace psdr;
 // give it back (0.5 to 2 ms per mesh, against 55 us with the kept words). Checks that run at
 // the same time take different slots.
 constexpr int kBoundsSlots = 16, kBoundsDevices = 64;
-__device__ unsigned g_bounds[kBoundsSlots][2 * kIndexJobs];
+constexpr int kBoundsJobs = 8 * kIndexJobs;  // buffers per slot and host read
+__device__ unsigned g_bounds[kBoundsSlots][2 * kBoundsJobs];
 class BoundsSlot {
  public:
   BoundsSlot() {
@@ -200,7 +201,7 @@ class BoundsSlot {
   }
   BoundsSlot(const BoundsSlot&) = delete;
   BoundsSlot& operator=(const BoundsSlot&) = delete;
-  unsigned* words() const { return slot_ < 0 ? nullptr : base_[dev_] + slot_ * 2 * kIndexJobs; }  // null: all taken
+  unsigned* words() const { return slot_ < 0 ? nullptr : base_[dev_] + slot_ * 2 * kBoundsJobs; }  // null: all taken
 
  private:
   static std::mutex mutex_;
@@ -212,36 +213,37 @@ std::mutex BoundsSlot::mutex_;
 unsigned* BoundsSlot::base_[kBoundsDevices] = {nullptr};
 unsigned BoundsSlot::used_[kBoundsDevices] = {0};
 
-// Smallest and largest entry of each of n device buffers: one kernel and one host read per 32
-// buffers.
+// Smallest and largest entry of each of n device buffers: a kernel per 32 buffers and a host read
+// per 256.
 static void index_bounds(const int* const* ptr, const long long* cnt, int n, int* out, cudaStream_t st) {
   if (n == 0) return;
-  constexpr size_t kBytes = sizeof(unsigned) * 2 * kIndexJobs;
   BoundsSlot slot;
   DBuf own;
-  if (!slot.words()) own.alloc(kBytes, st);
+  if (!slot.words()) own.alloc(sizeof(unsigned) * 2 * kBoundsJobs, st);
   unsigned* words = slot.words() ? slot.words() : own.as<unsigned>();
-  for (int j0 = 0; j0 < n; j0 += kIndexJobs) {
-    IndexJobs jobs{};
-    const int m = std::min(kIndexJobs, n - j0);
-    long long most = 0;
-    for (int j = 0; j < m; ++j) {
-      jobs.p[j] = ptr[j0 + j];
-      jobs.n[j] = cnt[j0 + j];
-      most = std::max(most, cnt[j0 + j]);
-    }
-    PSDR_CUDA(cudaMemsetAsync(words, 0, kBytes, st));
-    if (most > 0) {
+  unsigned h[2 * kBoundsJobs];
+  for (int i0 = 0; i0 < n; i0 += kBoundsJobs) {
+    const int part = std::min(kBoundsJobs, n - i0);
+    PSDR_CUDA(cudaMemsetAsync(words, 0, sizeof(unsigned) * 2 * part, st));
+    for (int j0 = 0; j0 < part; j0 += kIndexJobs) {
+      IndexJobs jobs{};
+      const int m = std::min(kIndexJobs, part - j0);
+      long long most = 0;
+      for (int j = 0; j < m; ++j) {
+        jobs.p[j] = ptr[i0 + j0 + j];
+        jobs.n[j] = cnt[i0 + j0 + j];
+        most = std::max(most, cnt[i0 + j0 + j]);
+      }
+      if (most == 0) continue;
       const dim3 grid((unsigned)std::min<long long>((most + 255) / 256, 148LL * 8), m);
-      k_index_bounds<<<grid, 256, 0, st>>>(jobs, words);
+      k_index_bounds<<<grid, 256, 0, st>>>(jobs, words + 2 * j0);
       PSDR_CUDA(cudaGetLastError());
     }
-    unsigned h[2 * kIndexJobs];
-    PSDR_CUDA(cudaMemcpyAsync(h, words, kBytes, cudaMemcpyDeviceToHost, st));
+    PSDR_CUDA(cudaMemcpyAsync(h, words, sizeof(unsigned) * 2 * part, cudaMemcpyDeviceToHost, st));
     PSDR_CUDA(cudaStreamSynchronize(st));
-    for (int j = 0; j < m; ++j) {
-      out[2 * (j0 + j)] = (int)(~h[2 * j] ^ 0x80000000u);
-      out[2 * (j0 + j) + 1] = (int)(h[2 * j + 1] ^ 0x80000000u);
+    for (int j = 0; j < part; ++j) {
+      out[2 * (i0 + j)] = (int)(~h[2 * j] ^ 0x80000000u);
+      out[2 * (i0 + j) + 1] = (int)(h[2 * j + 1] ^ 0x80000000u);
     }
   }
 }
