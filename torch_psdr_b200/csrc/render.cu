@@ -1508,14 +1508,14 @@ __global__ void __launch_bounds__(128, 2) k_adjoint_ext(WF w, const DevScene* __
           const float3 L = light_emit<true>(Lt, x0);
           has0 = true;
           ax0.area = dot(g, L) / x0.area;
-          if (UNB) co = cam_jacobian_adj(V, x0, dot(g, L), ax0);
+          if (UNB) cam.add(&V, cam_jacobian_adj(V, x0, dot(g, L), ax0));
           if (Lt.kind == kLightArea) {
             add_emit(sc, hot, x0.light, g);
           } else {
             // an SH9 light's radiance depends on wi = -normalize(x0 - o): its share goes
             // to the ray origin, which moves with the camera
             const float3 aw = env_emit_adj(&Lt, x0.u, x0.v, x0.wi, g);
-            if (Lt.kind == kLightSh9) co += (aw - x0.wi * dot(x0.wi, aw)) / sqrtf(x0.sqd);
+            if (Lt.kind == kLightSh9) cam.add(&V, (aw - x0.wi * dot(x0.wi, aw)) / sqrtf(x0.sqd));
           }
         }
       } else {
@@ -1560,7 +1560,7 @@ __global__ void __launch_bounds__(128, 2) k_adjoint_ext(WF w, const DevScene* __
             const bool next = d < w.D - 1 && continuation_adj<UNB, true, true>(sc, xc, mp.color * kInvPi, rx, ry,
                                                                          rec_hit(w, s, d, w.nL + w.nB), adjB, ax, nextc, nx, none, &mp, &ma);
             const float3 aorg = mat_finalize(ob, xc, mp, ma, ax);
-            if (d == 0) co += aorg;
+            if (d == 0) cam.add(&V, co + aorg);
             else if (d == 1) ax0.p += aorg;
             else axq.p += aorg;
             if (triq >= 0) scatter_mesh(sc, triq, hq.y, hq.z, frontq, axq);
@@ -1589,7 +1589,6 @@ __global__ void __launch_bounds__(128, 2) k_adjoint_ext(WF w, const DevScene* __
           if (triq >= 0) scatter_mesh(sc, triq, hq.y, hq.z, frontq, axq);
         }
       }
-      if (has0) cam.add(&V, co);
     }
     scatter_surf_warp(scp, hot, __float_as_int(h0.x), h0.y, h0.z, x0.front, ax0, has0);
     scatter_tex_warp(tx0, toff0, atex0, has0);
