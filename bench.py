@@ -57,8 +57,8 @@ TRACE_BYTES_PER_RAY = 40  # ray read 24 B + hit write 16 B (per-ray share of the
 # launch, so the BVH is read from DRAM each time), from one capture of
 #   ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum,gpu__time_duration.sum -k regex:k_trace -s 12 -c 32
 #   python bench.py --mode plain --tile-paths 2097152 --no-autotune --steps 1 --warmup 1 ...
-TRACE_DRAM_BYTES_PER_LAUNCH = 27.36e6
-TRACE_L2_THROUGHPUT_PCT = (11.8, 18.5)  # ncu lts__throughput, % of peak, 256^2 case
+TRACE_DRAM_BYTES_PER_LAUNCH = 27.34e6
+TRACE_L2_THROUGHPUT_PCT = (11.4, 17.9)  # ncu lts__throughput, % of peak, 256^2 case
 STEP_BYTES_PER_SAMPLE = 2628  # fwd+bwd algorithmic bytes per path sample at depth 3
 
 

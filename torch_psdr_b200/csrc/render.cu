@@ -334,9 +334,9 @@ __global__ void __launch_bounds__(256) k_shade(WF w, const DevScene* __restrict_
 // at least half a warp. The fetch counter is w.cnt[2D+2], reset by k_shade.
 //
 // Bound by instruction issue and divergence, not by memory: on 256^2 x 32 spp rays of the
-// icosphere scene the SMs issue on 79 % of the cycles with 18.7 of 32 lanes active at the first
+// icosphere scene the SMs issue on 79 % of the cycles with 18.6 of 32 lanes active at the first
 // depth, 68 % and 16 at the third (11 before lanes waited for one another at leaves,
-// trav_step); L1 64-82 %, L2 12-19 %, DRAM 2-3 % of their peaks. Traversal
+// trav_step); L1 64-82 %, L2 11-18 %, DRAM 2-3 % of their peaks. Traversal
 // of the 512^2 x 32 spp icosphere step: 14.0 ms before, 12.2 ms now (2^20-path tiles).
 constexpr int kRefill = 16;
 // Per-lane memory of k_trace: the first kShort stack entries, the ray as the triangle test
@@ -1270,9 +1270,9 @@ __host__ __device__ constexpr int adj_warp_words(int nB) { return kVertFields * 
 // for the few paths still alive, and the BSDF-sample code for two lanes of a warp on average:
 // 5.8 ms per 512^2 x 32 spp x depth 3 step against 2.9 ms with lists; 2.3 ms with the warps of a
 // block starting together (2.8 ms in tiles of 2^22 paths whose records lie in HBM, with fp32
-// or with exact sums per thread). Bound by the latency of its record loads (6.2 cycles
+// or with exact sums per thread). Bound by the latency of its record loads (5.9 cycles
 // per issued instruction at 24 % occupancy, 128 registers; DRAM 8 % busy); instruction fetch is
-// down from 7.2 cycles to 1.3, for 3.1 at the block's barrier.
+// down from 7.2 cycles to 1.3, for 3.0 at the block's barrier.
 // Without vertex gradients (VERTS false: texture and emission optimisation) the lists carry no
 // surface adjoint and the vertex scatters go; 256^2 x 64 spp: 0.83 -> 0.55 ms (three blocks per
 // SM spill: 0.63 ms).
